@@ -15,6 +15,7 @@ from mcnla_b200 import isvd
 
 # Work of the largest drawn case against the largest listed one (FP64 operations of a solve).
 MAX_FLOPS = 1.0e13
+WY_STEPS = 12
 
 
 # ----------------------------------------------------------------------------------------------
@@ -52,8 +53,9 @@ def listed():
         # the Gramian integrator with the headline's sketches on fewer rows
         _stage("integrate_kn", "integrate", 20000, 2000, 50, 14, 64, stage="rb_gramian_kn", tol=1e-6,
                spectrum="noise"),
-        # the drivers' default integrator (Wen-Yin) and tolerance on a mid-size problem's sketches.  Its line search
-        # carries rounding of the sketch into its step sizes, so it is timed on given bases and not in whole solves
+        # the drivers' default integrator (Wen-Yin) on a mid-size problem's sketches.  Its line search carries
+        # rounding into its step sizes, more with every step, so it is timed on given bases for a given number of
+        # steps (WY_STEPS, the drivers' maximum-iteration argument) and not in whole solves
         _stage("integrate_wy", "integrate", 16384, 2000, 50, 14, 16, stage="rb_wy", tol=1e-3, spectrum="noise"),
         # the SVD former of a wide request
         _stage("form_svd", "form", 16384, 4096, 64, 32, 8, stage="svd"),
@@ -212,7 +214,7 @@ def prepare(case, seed):
         stage = {"kn": isvd.KolmogorovNagumoIntegrator, "rb_kn": isvd.RowBlockKolmogorovNagumoIntegrator,
                  "rb_gramian_kn": isvd.RowBlockGramianKolmogorovNagumoIntegrator,
                  "rb_wy": isvd.RowBlockWenYinIntegrator, "rb_gramian_wy": isvd.RowBlockGramianWenYinIntegrator}
-        state["stage"] = stage[case["stage"]](prm, 256, case["tol"])
+        state["stage"] = stage[case["stage"]](prm, WY_STEPS if case["stage"].endswith("wy") else 256, case["tol"])
         state["qbar"] = prm.createMatrixQbar()
     else:
         state["a"] = _matrix(g, m, n, case["spectrum"], case["layout"])
@@ -227,6 +229,13 @@ def prepare(case, seed):
 # ----------------------------------------------------------------------------------------------
 # one pass
 # ----------------------------------------------------------------------------------------------
+def _signed(u, *others):
+    """Columns with the sign that makes the first row of u positive: singular vectors and bases are defined up to
+    it, and a program that compares or stores them picks one."""
+    sign = torch.copysign(torch.ones_like(u[0]), u[0])
+    return [x * sign for x in (u, *others)]
+
+
 def run(state):
     kind = state["kind"]
     if kind == "serve":
@@ -238,7 +247,7 @@ def run(state):
         # at most 64 outputs: all sigmas and iteration counts side by side, every U and V whole
         return {"s": torch.cat([r.s for r in state["requests"]]),
                 "iterations": torch.tensor([int(r.result.iteration) for r in state["requests"]]),
-                "u": [r.u for r in state["requests"]], "v": [r.v for r in state["requests"]]}
+                "uv": [_signed(r.u, r.v) for r in state["requests"]]}
     c = state["case"]
     if kind == "solve":
         if c["mixed"]:
@@ -248,6 +257,7 @@ def run(state):
         else:
             s, u, v, it = isvd.solve(state["a"], c["k"], c["p"], c["N"], omega=state.get("omega"), seed=state["seed"],
                                      integrator=c["integrator"], former=c["former"], tol=c["tol"])
+        u, v = _signed(u, v)
         return {"s": s, "u": u, "v": v, "iterations": it}
     stage = state["stage"]
     if kind == "sketch":
@@ -256,12 +266,13 @@ def run(state):
     if kind == "orthogonalize":
         q = state["y"].clone()          # the stage works in place, and the sketch is wanted again
         stage(q)
-        return {"q": q}
+        return {"q": _signed(q)[0]}
     if kind == "integrate":
         stage(state["q"], state["qbar"])
         return {"qbar": state["qbar"], "iterations": stage.iteration()}
     stage(state["a"], state["qbar"])
-    return {"s": stage.vectorS(), "u": stage.matrixU(), "v": stage.matrixV()}
+    u, v = _signed(stage.matrixU(), stage.matrixV())
+    return {"s": stage.vectorS(), "u": u, "v": v}
 
 
 # ----------------------------------------------------------------------------------------------
@@ -340,7 +351,7 @@ def exact(case, seed):
     if kind == "integrate" and case["stage"].endswith("wy"):
         return None
     if kind == "orthogonalize":
-        return None                     # the columns' signs are free
+        return None                     # the order and the mixing of equal eigenvalues are free
     state = prepare(case, seed)
     if kind == "sketch":
         a, om = state["a"], state["omega"]
