@@ -14,8 +14,7 @@ constexpr int kSmallThreads = 512;
 constexpr int kSyevThreads = 1024;   // the Jacobi rounds are latency-bound: more warps hide more of it
 constexpr int kMaxSweeps = 40;
 constexpr int kKnNsMaxDim = 80;   // the matrix-function KN step keeps four padded l x l matrices on chip
-constexpr int kGjThreads = 1024;   // the Gauss-Jordan steps are latency-bound: fewer rows per thread per step
-static_assert(2 * MCNLA_B200_MAX_DIM_SKETCH_WENYIN <= kGjThreads, "cta_gj_inverse needs n <= blockDim.x");
+static_assert(2 * MCNLA_B200_MAX_DIM_SKETCH_WENYIN <= 160, "gj_inverse_regs is instantiated for n <= 160");
 
 // Shared-memory carve-up shared by the one-CTA solvers.
 struct SmemCarve {
@@ -48,21 +47,6 @@ __device__ small::JacobiScratch carve_jacobi(SmemCarve& sc, int n) {
   js.count = sc.take<int>(1);
   js.red = sc.take<double>(32);
   return js;
-}
-
-__host__ __device__ inline size_t gj_scratch_bytes(int n) {   // piv, col, prow, cand_v, cand_i
-  return (size_t(n) * 4 + 16) + (size_t(n) * 16 + 16) + (size_t(n) * 8 + 16) + (small::kGjMaxGroups * 8 + 16) +
-         (small::kGjMaxGroups * 4 + 16);
-}
-
-__device__ small::GjScratch carve_gj(SmemCarve& sc, int n) {
-  small::GjScratch g;
-  g.piv = sc.take<int>(n);
-  g.col = sc.take<double>(2 * size_t(n));
-  g.prow = sc.take<double>(n);
-  g.cand_v = sc.take<double>(small::kGjMaxGroups);
-  g.cand_i = sc.take<int>(small::kGjMaxGroups);
-  return g;
 }
 
 // rank[j] = position of eigenvalue j in the requested order (ties by index).
@@ -496,48 +480,81 @@ __global__ void __launch_bounds__(GMEM ? kSyevThreads : kSmallThreads)
 // ---------------------------------------------------------------------------
 // Wen-Yin trial
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kGjThreads) k_wy_trial(int l, const double* dd, double tau, double inv_n,
-                                                            double* F, double* FN, DevScalars* scal) {
-  extern __shared__ __align__(16) char smem_raw[];
-  SmemCarve sc(smem_raw);
-  const int n = 2 * l, ld = n + 1, ldd = 2 * l;
-  double* cm = sc.take<double>(size_t(n) * ld);
-  const small::GjScratch gs = carve_gj(sc, n);
-  const int tid = threadIdx.x, nt = blockDim.x;
+// RA: rows of the 2l x 2l matrix per lane (2l <= 32 RA).
+template <int RA>
+__global__ void __launch_bounds__(small::kGjThreads) k_wy_trial(int l, const double* dd, double tau, double inv_n,
+                                                                double* F, double* FN, DevScalars* scal) {
+  extern __shared__ __align__(16) double inv_s[];   // inv(C), 2l x 2l
+  __shared__ small::GjShared<RA> sh;
+  const int n = 2 * l, ldd = 2 * l;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double it = 1.0 / tau;
   // C := [ Dc/2 - I/tau , I/2 ; -Dgc/2 , -Dc/2 - I/tau ]
   // (row_block_wen_yin_integrator.hpp:176-183)
-  for (int e = tid; e < n * n; e += nt) {
-    const int i = e / n, j = e % n;
-    const int bi = i / l, bj = j / l, ii = i % l, jj = j % l;
-    double x;
-    if (bi == 0 && bj == 0) x = 0.5 * dd[ii * ldd + jj] - (ii == jj ? it : 0.0);
-    else if (bi == 0) x = (ii == jj) ? 0.5 : 0.0;
-    else if (bj == 0) x = -0.5 * dd[ii * ldd + l + jj];
-    else x = -0.5 * dd[ii * ldd + jj] - (ii == jj ? it : 0.0);
-    cm[i * ld + j] = x;
+  double x[RA][2 * RA];
+  int pos[RA];
+#pragma unroll
+  for (int a = 0; a < RA; ++a) {
+    const int i = lane + 32 * a;
+    const int bi = i >= l, ii = i - (bi ? l : 0);
+#pragma unroll
+    for (int b = 0; b < 2 * RA; ++b) {
+      const int j = wid + small::kGjWarps * b;
+      const int bj = j >= l, jj = j - (bj ? l : 0);
+      double v = 0.0;
+      if (i < n && j < n) {
+        if (!bi && !bj) v = 0.5 * dd[ii * ldd + jj] - (ii == jj ? it : 0.0);
+        else if (!bi) v = (ii == jj) ? 0.5 : 0.0;
+        else if (!bj) v = -0.5 * dd[ii * ldd + l + jj];
+        else v = -0.5 * dd[ii * ldd + jj] - (ii == jj ? it : 0.0);
+      }
+      x[a][b] = v;
+    }
   }
-  __syncthreads();
-  const int sing = small::cta_gj_inverse(cm, ld, n, gs);
+  const int sing = small::gj_inverse_regs<RA>(x, pos, n, sh);
   if (sing) {
-    if (tid == 0) scal->status = MCNLA_B200_ERR_SINGULAR;
+    if (threadIdx.x == 0) scal->status = MCNLA_B200_ERR_SINGULAR;
     return;
   }
+#pragma unroll
+  for (int b = 0; b < 2 * RA; ++b) {
+    const int j = wid + small::kGjWarps * b;
+    if (j >= n) continue;
+    const int jo = sh.at[j];
+#pragma unroll
+    for (int a = 0; a < RA; ++a)
+      if (pos[a] >= 0) inv_s[pos[a] * n + jo] = x[a][b];
+  }
+  __syncthreads();
   // T := inv(C)(:, l:2l) * Dc - inv(C)(:, 0:l); Fgc = T(0:l, :), Fc = T(l:2l, :) + I
-  // F = [Fc; Fgc]   (row_block_wen_yin_integrator.hpp:189-193)
-  for (int e = tid; e < n * l; e += nt) {
-    const int i = e / l, j = e % l;
-    double s = 0.0;
-    for (int k = 0; k < l; ++k) s = fma(cm[i * ld + l + k], dd[k * ldd + j], s);
-    s -= cm[i * ld + j];
-    if (i >= l) {   // Fc row
-      const int r = i - l;
-      const double fc = s + (r == j ? 1.0 : 0.0);
-      F[r * l + j] = fc;
-      if (FN) FN[r * l + j] = fc;
-    } else {        // Fgc row
-      F[size_t(l) * l + i * l + j] = s;
-      if (FN) FN[size_t(l) * l + i * l + j] = s * inv_n;
+  // F = [Fc; Fgc]   (row_block_wen_yin_integrator.hpp:189-193).  A warp takes kTR rows (one address
+  // per load of inv(C)), a lane one column of Dc, which the rows share.
+  constexpr int kTR = 4;
+  for (int r0 = wid * kTR; r0 < n; r0 += small::kGjWarps * kTR) {
+    for (int j = lane; j < l; j += 32) {
+      double s[kTR];
+#pragma unroll
+      for (int r = 0; r < kTR; ++r) s[r] = 0.0;
+#pragma unroll 4
+      for (int k = 0; k < l; ++k) {
+        const double d = dd[k * ldd + j];
+#pragma unroll
+        for (int r = 0; r < kTR; ++r) s[r] = fma(r0 + r < n ? inv_s[(r0 + r) * n + l + k] : 0.0, d, s[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < kTR; ++r) {
+        const int i = r0 + r;
+        if (i >= n) continue;
+        const double t = s[r] - inv_s[i * n + j];
+        if (i >= l) {   // Fc row
+          const double fc = t + (i - l == j ? 1.0 : 0.0);
+          F[(i - l) * l + j] = fc;
+          if (FN) FN[(i - l) * l + j] = fc;
+        } else {        // Fgc row
+          F[size_t(l) * l + i * l + j] = t;
+          if (FN) FN[size_t(l) * l + i * l + j] = t * inv_n;
+        }
+      }
     }
   }
 }
@@ -679,21 +696,36 @@ __global__ void k_sqrt_vec(int n, const double* w, double* out) {
   for (int i = threadIdx.x + blockIdx.x * blockDim.x; i < n; i += blockDim.x * gridDim.x) out[i] = sqrt(w[i]);
 }
 
-__global__ void __launch_bounds__(kGjThreads) k_inverse(int n, double* A, DevScalars* scal) {
-  extern __shared__ __align__(16) char smem_raw[];
-  SmemCarve sc(smem_raw);
-  const int ld = n + 1;
-  double* a = sc.take<double>(size_t(n) * ld);
-  const small::GjScratch gs = carve_gj(sc, n);
+template <int RA>
+__global__ void __launch_bounds__(small::kGjThreads) k_inverse(int n, double* A, DevScalars* scal) {
+  __shared__ small::GjShared<RA> sh;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double* Ab = A + size_t(blockIdx.x) * n * n;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) a[(e / n) * ld + (e % n)] = Ab[e];
-  __syncthreads();
-  const int sing = small::cta_gj_inverse(a, ld, n, gs);
+  double x[RA][2 * RA];
+  int pos[RA];
+#pragma unroll
+  for (int a = 0; a < RA; ++a) {
+    const int i = lane + 32 * a;
+#pragma unroll
+    for (int b = 0; b < 2 * RA; ++b) {
+      const int j = wid + small::kGjWarps * b;
+      x[a][b] = (i < n && j < n) ? Ab[i * n + j] : 0.0;
+    }
+  }
+  const int sing = small::gj_inverse_regs<RA>(x, pos, n, sh);
   if (sing) {
     if (threadIdx.x == 0) scal->status = MCNLA_B200_ERR_SINGULAR;
     return;
   }
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) Ab[e] = a[(e / n) * ld + (e % n)];
+#pragma unroll
+  for (int b = 0; b < 2 * RA; ++b) {
+    const int j = wid + small::kGjWarps * b;
+    if (j >= n) continue;
+    const int jo = sh.at[j];
+#pragma unroll
+    for (int a = 0; a < RA; ++a)
+      if (pos[a] >= 0) Ab[pos[a] * n + jo] = x[a][b];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -957,10 +989,18 @@ int launch_kn_step(Context* c, int l, const double* z, const double* dd, double 
 int launch_wy_trial(Context* c, int l, const double* dd, double tau, double inv_n, double* F, double* FN) {
   if (l < 1 || l > MCNLA_B200_MAX_DIM_SKETCH_WENYIN) return MCNLA_B200_ERR_UNSUPPORTED;
   const int n = 2 * l;
-  const size_t smem = size_t(n) * (n + 1) * 8 + 16 + gj_scratch_bytes(n) + 64;
-  if (smem > c->smem_optin) return MCNLA_B200_ERR_UNSUPPORTED;
-  MB_CHECK(set_smem(c, reinterpret_cast<const void*>(k_wy_trial), smem));
-  k_wy_trial<<<1, kGjThreads, smem, c->stream>>>(l, dd, tau, inv_n, F, FN, c->scal);
+  const size_t smem = size_t(n) * n * sizeof(double);
+  auto go = [&](auto kern) -> int {
+    MB_CHECK(set_smem(c, reinterpret_cast<const void*>(kern), smem));
+    kern<<<1, small::kGjThreads, smem, c->stream>>>(l, dd, tau, inv_n, F, FN, c->scal);
+    return MCNLA_B200_OK;
+  };
+  // the fewest registers that hold the matrix: 2l <= 32 RA
+  if (n <= 32) MB_CHECK(go(k_wy_trial<1>));
+  else if (n <= 64) MB_CHECK(go(k_wy_trial<2>));
+  else if (n <= 96) MB_CHECK(go(k_wy_trial<3>));
+  else if (n <= 128) MB_CHECK(go(k_wy_trial<4>));
+  else MB_CHECK(go(k_wy_trial<5>));
   c->kernels_launched++;
   MB_CHECK_CUDA(cudaGetLastError());
   return MCNLA_B200_OK;
@@ -1091,10 +1131,11 @@ int launch_gwy_small_dots(Context* c, int l, const double* phi1, const double* p
 
 int launch_inverse(Context* c, int n, int batch, double* A) {
   if (n < 1 || n > 2 * MCNLA_B200_MAX_DIM_SKETCH_WENYIN || batch < 1) return MCNLA_B200_ERR_UNSUPPORTED;
-  const size_t smem = size_t(n) * (n + 1) * 8 + 16 + gj_scratch_bytes(n) + 64;
-  if (smem > c->smem_optin) return MCNLA_B200_ERR_UNSUPPORTED;
-  MB_CHECK(set_smem(c, reinterpret_cast<const void*>(k_inverse), smem));
-  k_inverse<<<batch, kGjThreads, smem, c->stream>>>(n, A, c->scal);
+  if (n <= 32) k_inverse<1><<<batch, small::kGjThreads, 0, c->stream>>>(n, A, c->scal);
+  else if (n <= 64) k_inverse<2><<<batch, small::kGjThreads, 0, c->stream>>>(n, A, c->scal);
+  else if (n <= 96) k_inverse<3><<<batch, small::kGjThreads, 0, c->stream>>>(n, A, c->scal);
+  else if (n <= 128) k_inverse<4><<<batch, small::kGjThreads, 0, c->stream>>>(n, A, c->scal);
+  else k_inverse<5><<<batch, small::kGjThreads, 0, c->stream>>>(n, A, c->scal);
   c->kernels_launched++;
   MB_CHECK_CUDA(cudaGetLastError());
   return MCNLA_B200_OK;

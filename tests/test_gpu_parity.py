@@ -101,6 +101,23 @@ def test_inverse_batched(cuda, n):
         assert np.abs(inv[b] - np.linalg.inv(a[b])).max() <= 1e-12 * np.linalg.cond(a[b])
 
 
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 63, 64, 65, 95, 97, 127, 129, 159])
+def test_inverse_batched_tile_edges(cuda, n):
+    """Sizes around the register tiles of the inverse, on matrices whose pivots move (no dominant diagonal;
+    the second one has tied pivots and needs an interchange in its first column)."""
+    from mcnla_b200 import isvd, _lib
+    import ctypes
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((2, n, n))
+    a[1] = np.eye(n)[rng.permutation(n)] + np.triu(rng.integers(-1, 2, (n, n)), 1) / (4.0 * n)
+    at = dev(a, cuda)
+    ctx = isvd.context()
+    _lib.check(ctx.lib.mcnla_b200_inverse_batched(ctx.bind(), n, 2, ctypes.c_void_p(at.data_ptr())), "inverse")
+    inv = host(at)
+    for b in range(2):
+        assert np.abs(inv[b] - np.linalg.inv(a[b])).max() <= 1e-12 * np.linalg.cond(a[b])
+
+
 def test_inverse_singular_reports_status(cuda):
     from mcnla_b200 import isvd, _lib
     import ctypes
