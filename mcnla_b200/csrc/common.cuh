@@ -57,6 +57,7 @@ struct DevScalars {
   unsigned bar_spare;
   int resume_it;      // persistent integrator: iteration it handed back to the host (-1: none)
   int kn_ns_failed;   // 1: the Newton-Schulz KN step with its matrices in global memory failed
+  int wait_status;    // a bounded wait of the int8 GEMM ran out: kept (ctx_reset_scalars) until it is reported
 };
 
 // Per-device context: one stream, a growable workspace arena, timing events.
@@ -149,6 +150,7 @@ int ctx_toc(Context* c);
 int ctx_collect_times(Context* c);
 
 int ctx_sync_scalars(Context* c);   // copies DevScalars to the pinned mirror and waits
+int ctx_reset_scalars(Context* c);  // zeroes DevScalars (stream-ordered), except a wait_status not yet reported
 
 // Sums `count` doubles at the device pointer buf over the ranks of the context's
 // row-block decomposition, in place, ordered on the context's stream (comm.cu).  A

@@ -107,6 +107,15 @@ int ctx_collect_times(Context* c) {
 int ctx_sync_scalars(Context* c) {
   MB_CHECK_CUDA(cudaMemcpyAsync(c->scal_host, c->scal, sizeof(DevScalars), cudaMemcpyDeviceToHost, c->stream));
   MB_CHECK_CUDA(cudaStreamSynchronize(c->stream));
+  if (c->scal_host->wait_status) {
+    if (!c->scal_host->status) c->scal_host->status = c->scal_host->wait_status;
+    MB_CHECK_CUDA(cudaMemsetAsync(&c->scal->wait_status, 0, sizeof(int), c->stream));
+  }
+  return MCNLA_B200_OK;
+}
+
+int ctx_reset_scalars(Context* c) {
+  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, offsetof(DevScalars, wait_status), c->stream));
   return MCNLA_B200_OK;
 }
 

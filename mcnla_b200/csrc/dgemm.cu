@@ -33,7 +33,19 @@ struct KArgs {
   const int* guard_stop;   // skip the launch when *guard_stop < guard_it
   int guard_it;
   int lower;               // 1: only tiles touching the lower triangle (row >= column) are computed
+  GemmFlags fl;            // the FLAGGED kernels: only elements with a flagged row or column (batch 1)
 };
+
+// Whether a tile holds a flagged row or column (block-uniform).
+__device__ __forceinline__ bool tile_flagged(const GemmFlags& fl, int64_t m0, int bm, int64_t M, int64_t n0, int bn,
+                                             int64_t N) {
+  int any = 0;
+  for (int i = threadIdx.x; i < bm + bn; i += blockDim.x) {
+    if (i < bm) any |= m0 + i < M && fl.row[m0 + i];
+    else any |= n0 + i - bm < N && fl.col[n0 + i - bm];
+  }
+  return __syncthreads_or(any) != 0;
+}
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
   unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -131,7 +143,9 @@ struct TileLoader {
   }
 };
 
-template <class C>
+// FLAGGED: a product restricted by g.fl.  A kernel of its own: the two tests in the epilogue cost the ordinary
+// one 8-15 %.
+template <class C, bool FLAGGED>
 __global__ void __launch_bounds__(C::THREADS) dgemm_kernel(KArgs g) {
   extern __shared__ __align__(16) double smem[];
   if (g.guard_stop && *g.guard_stop < g.guard_it) return;
@@ -143,6 +157,7 @@ __global__ void __launch_bounds__(C::THREADS) dgemm_kernel(KArgs g) {
   const int64_t n0 = int64_t(blockIdx.x) * C::BN;
   const int64_t m0 = int64_t(blockIdx.y) * C::BM;
   if (g.lower && n0 >= m0 + C::BM) return;        // every element of the tile has column > row
+  if (FLAGGED && (*g.fl.any == 0 || !tile_flagged(g.fl, m0, C::BM, g.M, n0, C::BN, g.N))) return;
   const int bz = blockIdx.z / g.splits;
   const int split = blockIdx.z % g.splits;
   const double* A = g.A + bz * g.a_bs;
@@ -224,6 +239,7 @@ __global__ void __launch_bounds__(C::THREADS) dgemm_kernel(KArgs g) {
       for (int h = 0; h < 2; ++h) {
         const int64_t col = n0 + wn * C::WN + j * 8 + 2 * t4 + h;
         if (col >= g.N) continue;
+        if (FLAGGED && !g.fl.row[row] && !g.fl.col[col]) continue;
         if (g.splits == 1) {
           double* cp = Cb + row * g.c_rs + col * g.c_cs;
           double v = g.alpha * acc[i][j][h];
@@ -239,8 +255,9 @@ __global__ void __launch_bounds__(C::THREADS) dgemm_kernel(KArgs g) {
 
 __global__ void splitk_reduce_kernel(const double* ws, int splits, int batch, int64_t M, int64_t N, double alpha,
                                      double beta, double* C, int64_t c_rs, int64_t c_cs, int64_t c_bs,
-                                     const int* guard_stop, int guard_it, int lower) {
+                                     const int* guard_stop, int guard_it, int lower, GemmFlags fl) {
   if (guard_stop && *guard_stop < guard_it) return;
+  if (fl.any && *fl.any == 0) return;
   const int64_t MN = M * N;
   const int64_t total = MN * batch;
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
@@ -248,6 +265,7 @@ __global__ void splitk_reduce_kernel(const double* ws, int splits, int batch, in
     const int64_t b = idx / MN, e = idx % MN;
     const int64_t r = e / N, c = e % N;
     if (lower && c > r) continue;
+    if (fl.any && !fl.row[r] && !fl.col[c]) continue;
     const double* w = ws + b * splits * MN + e;
     double s = 0.0;
     for (int k = 0; k < splits; ++k) s += w[k * MN];
@@ -258,11 +276,11 @@ __global__ void splitk_reduce_kernel(const double* ws, int splits, int batch, in
   }
 }
 
-template <class C>
+template <class C, bool FLAGGED = false>
 int launch(Context* ctx, const KArgs& g, int batch) {
   // the shared-memory opt-in is a per-device property of the function: one bit per device
   static std::atomic<uint64_t> attr_set{0};
-  auto kern = dgemm_kernel<C>;
+  auto kern = dgemm_kernel<C, FLAGGED>;
   const uint64_t bit = uint64_t(1) << (ctx->device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & bit)) {
     MB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(C::SMEM)));
@@ -281,6 +299,8 @@ enum Shape { S128x128 = 0, S128x64 = 1, S64x64 = 2, S128x32 = 3, S64x32 = 4, S12
 
 template <bool AK, bool BKM, int VEC>
 int dispatch_shape(Context* ctx, const KArgs& g, int batch, Shape s) {
+  // restricted products are parts of large ones: one tile shape, whose k-tile every plan's split is a multiple of
+  if (g.fl.any) return launch<Cfg<64, 128, 32, 64, AK, BKM, VEC, 4>, true>(ctx, g, batch);
   switch (s) {
     case S128x128: return launch<Cfg<128, 128, 64, 32, AK, BKM, VEC, 4>>(ctx, g, batch);
     case S128x128w16: return launch<Cfg<128, 128, 32, 32, AK, BKM, VEC, 4>>(ctx, g, batch);
@@ -390,7 +410,7 @@ int run_plan(Context* ctx, KArgs g, int batch, const Plan& p, bool AK, bool BKM,
     const int blocks = int(std::min<int64_t>(cdiv(total, threads), int64_t(ctx->num_sms) * 8));
     splitk_reduce_kernel<<<blocks, threads, 0, ctx->stream>>>(g.ws, p.splits, batch, g.M, g.N, g.alpha, g.beta, g.C,
                                                              g.c_rs, g.c_cs, g.c_bs, g.guard_stop, g.guard_it,
-                                                             g.lower);
+                                                             g.lower, g.fl);
     ctx->kernels_launched++;
     MB_CHECK_CUDA(cudaGetLastError());
   }
@@ -472,7 +492,7 @@ int tune(Context* ctx, const KArgs& g0, int batch, const Plan& heuristic, int ma
 }  // namespace
 
 int dgemm(Context* ctx, int64_t M, int64_t N, int64_t K, double alpha, CMat A, CMat B, double beta, DMat Cm,
-          GemmBatch batch, double* ws, int force_splits, bool lower_only) {
+          GemmBatch batch, double* ws, int force_splits, bool lower_only, const GemmFlags* flags) {
   if (M < 0 || N < 0 || K < 0 || batch.count < 1) return MCNLA_B200_ERR_SHAPE;
   if (M == 0 || N == 0) return MCNLA_B200_OK;
   bool AK, BKM;
@@ -494,6 +514,10 @@ int dgemm(Context* ctx, int64_t M, int64_t N, int64_t K, double alpha, CMat A, C
   g.guard_stop = ctx->guard_stop;
   g.guard_it = ctx->guard_it;
   g.lower = lower_only ? 1 : 0;
+  if (flags) {
+    if (batch.count != 1) return MCNLA_B200_ERR_ARG;
+    g.fl = *flags;
+  }
   // split-K workspace available to this call (the planned need, or the stage's buffer)
   const bool have_ws = ws && ws == ctx->gws;
   const size_t ws_bytes = have_ws ? ctx->gws_bytes : 0;

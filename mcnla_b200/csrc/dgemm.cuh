@@ -21,6 +21,14 @@ struct GemmBatch {
   int64_t a = 0, b = 0, c = 0;   // element strides between batch members
 };
 
+// Restricts a product to the elements whose row or whose column is flagged (device arrays, one byte each);
+// *any == 0: none is.  Element values are those of the unrestricted product.
+struct GemmFlags {
+  const uint8_t* row = nullptr;
+  const uint8_t* col = nullptr;
+  const int* any = nullptr;
+};
+
 // Bytes of workspace dgemm() needs for this shape (0 when no split-K is used).
 size_t dgemm_workspace_bytes(const Context* c, int64_t M, int64_t N, int64_t K, int batch);
 // The split-K count the shape heuristic picks for this product (1: none).  Every
@@ -32,9 +40,11 @@ int dgemm_heuristic_splits(const Context* c, int64_t M, int64_t N, int64_t K, in
 // dgemm_workspace_bytes() is 0.  force_splits > 0 overrides the split choice
 // (tests use it to cover the split-K path at small sizes).  lower_only: C is
 // square and only its lower triangle is needed (SYRK-like: tiles strictly
-// above the diagonal are skipped and the elements above it are unspecified).
+// above the diagonal are skipped and the elements above it are unspecified).  flags: only
+// the flagged elements are computed and written.
 int dgemm(Context* ctx, int64_t M, int64_t N, int64_t K, double alpha, CMat A, CMat B, double beta, DMat C,
-          GemmBatch batch = GemmBatch(), double* ws = nullptr, int force_splits = 0, bool lower_only = false);
+          GemmBatch batch = GemmBatch(), double* ws = nullptr, int force_splits = 0, bool lower_only = false,
+          const GemmFlags* flags = nullptr);
 
 // C := A B where C holds the same rows as A (an in-place update of A's row
 // panels, e.g. Q_i := Q_i T_i): run only when one CTA covers all N output

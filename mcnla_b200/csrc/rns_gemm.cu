@@ -1,0 +1,638 @@
+// FP64 products through int8 tensor-core residue products (see rns.cuh).
+//
+// Four kernels: the residues of A's rows and of B's columns (K-contiguous int8 planes, one per
+// modulus), the int8 GEMMs of all moduli in one persistent launch (tcgen05 kind::i8),
+// and the CRT back to FP64; then the DMMA GEMM on what was flagged.
+#include "rns.cuh"
+#include "rns_math.cuh"
+#include "tma.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+
+namespace mb {
+namespace {
+
+static_assert(rns::kNum == kRnsModuli, "one plane per modulus");
+__constant__ rns::Tables kT = rns::make_tables();
+
+constexpr int kKTile = 128;                 // K of a shared-memory tile: one 128-byte swizzle row
+constexpr int64_t kMaxChunk = 131071;       // 32-bit sums of products of two signed bytes
+constexpr int kTileM = 128, kTileN = 256;    // output tile of a CTA
+constexpr double kMaxScale = 0x1p800, kMinScale = 0x1p-800;   // squares: entries within 2^+-400
+
+__device__ __forceinline__ double pow2(int e) {   // |e| < 1023
+  return __longlong_as_double((long long)(e + 1023) << 52);
+}
+
+// The scale of a row or column from its squared 2-norm and largest |entry|: exponent s such that the 2-norm
+// times 2^s is at most 2^target.  bad: the DMMA path takes it.
+__device__ __forceinline__ int scale_of(double norm2, double mx, int64_t K, int target, bool* bad) {
+  if (mx == 0.0 && norm2 == 0.0) { *bad = false; return 0; }
+  *bad = !(norm2 <= kMaxScale) || !(norm2 >= kMinScale) || norm2 * 256.0 < double(K) * mx * mx;
+  if (*bad) return 0;
+  const int e = int((__double_as_longlong(norm2) >> 52) & 0x7ff) - 1022;   // norm2 < 2^e
+  return target - ((e + 1) >> 1);
+}
+
+// Four consecutive residue bytes of plane i; u: the elements times their scale, rounded, plus the offset.
+__device__ __forceinline__ uint32_t pack4(const uint64_t (&u)[4], const rns::Bytes& w, int i) {
+  const uint32_t r0 = rns::residue(u[0], w, kT, i), r1 = rns::residue(u[1], w, kT, i);
+  const uint32_t r2 = rns::residue(u[2], w, kT, i), r3 = rns::residue(u[3], w, kT, i);
+  return __byte_perm(__byte_perm(r0, r1, 0x0040), __byte_perm(r2, r3, 0x0040), 0x5410);
+}
+
+__device__ __forceinline__ uint64_t to_int(double x, double s1, double s2) {
+  return uint64_t(__double2ll_rn(x * s1 * s2) + (long long)rns::kOffset);
+}
+
+// s = s1 s2: a scale of up to 2^+-460 as two factors, so that no intermediate product leaves the range
+__device__ __forceinline__ void split_scale(int s, double* s1, double* s2) {
+  const int h = s / 2;
+  *s1 = pow2(h);
+  *s2 = pow2(s - h);
+}
+
+struct Out {
+  uint8_t* planes;        // [modulus][row][kp]
+  int64_t rows_pad;       // rows per plane
+  int64_t kp;             // bytes per row: K rounded up to kKTile, zero past K
+  double* unscale;        // per row: 2^-s
+  uint8_t* flag;          // per row: 1 when the DMMA path takes it (never cleared here)
+  int* any;
+};
+
+// Residues of the rows of a K-contiguous matrix, one CTA per row: the norm, then the row again (from
+// L2) into the planes.  Bound by the integer pipe: ~100 instructions an element (15 residues of a 64-bit
+// integer, two dp4a and a division by rounding each) against 8 bytes read and 15 written.
+constexpr int kRowThreads = 256;
+template <bool VEC, bool IS_B>
+__global__ void __launch_bounds__(kRowThreads) k_rns_rows(const double* __restrict__ A, int64_t lda, int64_t K,
+                                                          int target, Out o) {
+  __shared__ double red_s[kRowThreads / 32], red_m[kRowThreads / 32];
+  __shared__ int scale_s;
+  const int64_t row = blockIdx.x;
+  const double* a = A + row * lda;
+  const int tid = threadIdx.x;
+  double s = 0.0, mx = 0.0;
+  const int64_t quads = (K + 3) / 4;
+  auto load = [&](int64_t q, double (&x)[4]) {
+    const int64_t k = 4 * q;
+    if (VEC && k + 4 <= K) {
+      const double2 p0 = *reinterpret_cast<const double2*>(a + k), p1 = *reinterpret_cast<const double2*>(a + k + 2);
+      x[0] = p0.x; x[1] = p0.y; x[2] = p1.x; x[3] = p1.y;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = k + j < K ? a[k + j] : 0.0;
+    }
+  };
+  for (int64_t q = tid; q < quads; q += kRowThreads) {
+    double x[4];
+    load(q, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s = fma(x[j], x[j], s);      // NaN and infinities reach the sum
+      mx = fmax(mx, fabs(x[j]));
+    }
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, d);
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+  }
+  if ((tid & 31) == 0) { red_s[tid >> 5] = s; red_m[tid >> 5] = mx; }
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < kRowThreads / 32; ++w) { s += red_s[w]; mx = fmax(mx, red_m[w]); }
+    bool bad;
+    const int e = scale_of(s, mx, K, target, &bad);
+    scale_s = bad ? INT32_MIN : e;
+    o.unscale[row] = pow2(-e);
+    if (bad) { o.flag[row] = 1; *o.any = 1; }
+  }
+  __syncthreads();
+  const int e = scale_s;
+  if (e == INT32_MIN) return;      // its planes' bytes are not used
+  double s1, s2;
+  split_scale(e, &s1, &s2);
+  const int64_t plane = o.rows_pad * o.kp;
+  for (int64_t q = tid; q < o.kp / 4; q += kRowThreads) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(o.planes + row * o.kp) + q;
+    if (q >= quads) {
+#pragma unroll
+      for (int i = 0; i < kRnsModuli; ++i) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(w) + i * plane) = 0u;
+      continue;
+    }
+    double x[4];
+    load(q, x);
+    uint64_t u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = to_int(x[j], s1, s2);   // past K: zero, whose residues are zero
+#pragma unroll
+    for (int i = 0; i < kRnsModuli; ++i)
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(w) + i * plane) = pack4(u, IS_B ? kT.b : kT.a, i);
+  }
+}
+
+// The same for a matrix whose rows run along the other dimension (element (row r, k) at p[k ld + r]): squared
+// norms and maxima per chunk of kStatK rows of k, combined in order; then tiles through shared memory.
+constexpr int kStatK = 256;
+__global__ void __launch_bounds__(256) k_rns_colstats(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
+                                                      double* part) {
+  __shared__ double ss[8][33], sm[8][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t r = int64_t(blockIdx.x) * 32 + lane;
+  const int64_t k0 = int64_t(blockIdx.y) * kStatK, k1 = min(K, k0 + kStatK);
+  double s = 0.0, mx = 0.0;
+  if (r < R) {
+#pragma unroll 4
+    for (int64_t k = k0 + w; k < k1; k += 8) {
+      const double x = B[k * ld + r];
+      s = fma(x, x, s);
+      mx = fmax(mx, fabs(x));
+    }
+  }
+  ss[w][lane] = s;
+  sm[w][lane] = mx;
+  __syncthreads();
+  if (w == 0 && r < R) {
+    for (int i = 1; i < 8; ++i) { s += ss[i][lane]; mx = fmax(mx, sm[i][lane]); }
+    part[(2 * int64_t(blockIdx.y)) * R + r] = s;
+    part[(2 * int64_t(blockIdx.y) + 1) * R + r] = mx;
+  }
+}
+
+__global__ void k_rns_colscale(const double* part, int64_t R, int64_t K, int chunks, int target, int* scale, Out o) {
+  const int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (r >= R) return;
+  double s = 0.0, mx = 0.0;
+  for (int c = 0; c < chunks; ++c) {
+    s += part[2 * int64_t(c) * R + r];
+    mx = fmax(mx, part[(2 * int64_t(c) + 1) * R + r]);
+  }
+  bool bad;
+  const int e = scale_of(s, mx, K, target, &bad);
+  scale[r] = bad ? INT32_MIN : e;
+  o.unscale[r] = pow2(-e);
+  if (bad) { o.flag[r] = 1; *o.any = 1; }
+}
+
+constexpr int kColTile = 32;
+template <bool IS_B>
+__global__ void __launch_bounds__(256) k_rns_cols(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
+                                                  const int* scale, Out o) {
+  __shared__ double tile[kColTile][kKTile + 2];   // [row][k]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t r0 = int64_t(blockIdx.y) * kColTile, k0 = int64_t(blockIdx.x) * kKTile;
+  const int64_t r = r0 + lane;
+  for (int k = w; k < kKTile; k += 8) tile[lane][k] = (r < R && k0 + k < K) ? B[(k0 + k) * ld + r] : 0.0;
+  __syncthreads();
+  const int64_t plane = o.rows_pad * o.kp;
+  for (int i = w; i < kColTile; i += 8) {          // a warp writes one row's 128 bytes of a plane
+    const int64_t row = r0 + i;
+    if (row >= R) break;
+    const int e = scale[row];
+    if (e == INT32_MIN) continue;
+    double s1, s2;
+    split_scale(e, &s1, &s2);
+    uint64_t u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = to_int(tile[i][4 * lane + j], s1, s2);
+    uint8_t* dst = o.planes + row * o.kp + k0 + 4 * lane;
+#pragma unroll
+    for (int m = 0; m < kRnsModuli; ++m) *reinterpret_cast<uint32_t*>(dst + m * plane) = pack4(u, IS_B ? kT.b : kT.a, m);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// int8 GEMM of every modulus: D_p = A_p B_p' modulo m_p, as CRT digits
+// ---------------------------------------------------------------------------
+struct GemmArgs {
+  int64_t a_rows_pad, b_rows_pad;   // rows per plane of the operand maps
+  int a_row0;                       // first row of A's planes (a block of a Gramian)
+  int mt, nt;                       // tiles
+  int kt;                           // k-tiles
+  int lower;                        // 1: only tiles with a_row0 + m0 + kTileM > n0
+  int64_t jobs;
+  uint8_t* y;                       // [modulus][y_rows][ldy] digits
+  int64_t y_rows, ldy;
+  const uint8_t* row_flag;          // rows of A / columns of B that the DMMA path takes
+  const uint8_t* col_flag;
+  const int* any;
+  int M, N;                         // valid rows and columns
+  int* status;
+};
+
+constexpr int kStages = 4;
+constexpr int kABytes = kTileM * kKTile, kBBytes = kTileN * kKTile, kStageBytes = kABytes + kBBytes;
+constexpr size_t kGemmSmem = size_t(kStages) * kStageBytes + 1024;
+// instruction descriptor, kind::i8: D s32, A and B signed 8-bit, K-major, M = 128, N = 256
+constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(kTileN >> 3) << 17) |
+                            (uint32_t(kTileM >> 4) << 24);
+constexpr uint32_t kTmemCols = 512;         // two 256-column accumulators
+constexpr int kEpiWarps = 8;                // two per TMEM lane quarter, 128 columns each
+constexpr int kGemmThreads = 128 + 32 * kEpiWarps;
+
+// Job -> modulus and tile (false: a tile above the diagonal).  Rows of tiles run fastest, so concurrent CTAs share
+// B's tiles.
+struct Job { int p, m, n; };
+__device__ __forceinline__ bool job_of(const GemmArgs& g, int64_t j, Job* out) {
+  const int64_t per = int64_t(g.mt) * g.nt;
+  out->p = int(j / per);
+  const int64_t t = j % per;
+  out->n = int(t / g.mt);
+  out->m = int(t % g.mt);
+  return !(g.lower && int64_t(out->n) * kTileN >= g.a_row0 + int64_t(out->m + 1) * kTileM);
+}
+
+// Whether every row or every column of a tile goes to the DMMA path (all threads of a warp call it).
+__device__ __forceinline__ bool tile_unused(const GemmArgs& g, const Job& jb) {
+  if (*g.any == 0) return false;
+  const int lane = threadIdx.x & 31;
+  bool rows = true, cols = true;
+  for (int i = lane; i < kTileN; i += 32) {
+    const int r = jb.m * kTileM + i, c = jb.n * kTileN + i;
+    if (i < kTileM && r < g.M && !g.row_flag[r]) rows = false;
+    if (c < g.N && !g.col_flag[c]) cols = false;
+  }
+  return __all_sync(0xffffffffu, rows) || __all_sync(0xffffffffu, cols);
+}
+
+// A CTA computes 128 x 256 tiles of every modulus' product.  Warp 0: TMA into the ring of 48 KB stages; warp 1: MMA
+// issue (M = 128, N = 256, K = 32); warps 4-11: the finished accumulator to CRT digits while the next tile
+// accumulates in the other TMEM half.  Every wait is bounded.  What bounds it on long K is power: 2.6 POP/s at the
+// 1000 W limit on 2048 x 4096 x 20000 blocks (CTA pairs with cta_group::2, which read a third less from L2, ran
+// at the same rate; and pairs launched from several streams at once did not get past their start).
+__global__ void __launch_bounds__(kGemmThreads, 1)
+    rns_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, GemmArgs g) {
+  extern __shared__ uint8_t smem_dyn[];
+  __shared__ __align__(8) uint64_t full_bar[kStages];    // the stage's copies have landed
+  __shared__ __align__(8) uint64_t empty_bar[kStages];   // the MMAs have read the stage
+  __shared__ __align__(8) uint64_t acc_full[2];          // accumulator b is complete
+  __shared__ __align__(8) uint64_t acc_empty[2];         // accumulator b has been read
+  __shared__ uint32_t tmem_base_s;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                 "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], kEpiWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = tmem_base_s;
+
+  if (warp == 0) {
+    // ---- producer (the whole warp walks the jobs; one lane copies)
+    int64_t it = 0;
+    bool ok = true;
+    for (int64_t j = blockIdx.x; j < g.jobs && ok; j += gridDim.x) {
+      Job jb;
+      if (!job_of(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (lane == 0) {
+        const int ya = int(int64_t(jb.p) * g.a_rows_pad) + g.a_row0 + jb.m * kTileM;
+        const int yb = int(int64_t(jb.p) * g.b_rows_pad) + jb.n * kTileN;
+        for (int kt = 0; kt < g.kt; ++kt) {
+          const int64_t i = it + kt;
+          const int s = int(i % kStages);
+          if (i >= kStages && !mbar_wait(&empty_bar[s], uint32_t(((i / kStages) & 1) ^ 1))) {
+            // let the copies in flight land before the CTA's shared memory goes away
+            for (int64_t f = i - kStages; f < i; ++f) mbar_wait(&full_bar[f % kStages], uint32_t((f / kStages) & 1));
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&full_bar[s], kStageBytes);
+          uint8_t* sa = smem + s * kStageBytes;
+          tma_load_2d(sa, &tm_a, &full_bar[s], kt * kKTile, ya);
+          tma_load_2d(sa + kABytes, &tm_b, &full_bar[s], kt * kKTile, yb);
+        }
+      }
+      it += g.kt;
+      ok = __all_sync(0xffffffffu, ok);
+    }
+    if (!ok && lane == 0) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
+  } else if (warp == 1) {
+    // ---- MMA issuer
+    int64_t it = 0, done = 0;
+    bool ok = true;
+    for (int64_t j = blockIdx.x; j < g.jobs && ok; j += gridDim.x) {
+      Job jb;
+      if (!job_of(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (lane == 0) {
+        const int b = int(done & 1);
+        if (done >= 2 && !mbar_wait(&acc_empty[b], uint32_t(((done >> 1) - 1) & 1))) ok = false;
+        fence_after();
+        for (int kt = 0; kt < g.kt && ok; ++kt) {
+          const int64_t i = it + kt;
+          const int s = int(i % kStages);
+          if (!mbar_wait(&full_bar[s], uint32_t((i / kStages) & 1))) { ok = false; break; }
+          fence_after();
+          const uint32_t sa = smem_u32(smem + s * kStageBytes);
+          const uint32_t sb = sa + kABytes;
+#pragma unroll
+          for (int k = 0; k < kKTile / 32; ++k)
+            umma_i8(tmem + uint32_t(b * kTileN), sw128_desc(sa + k * 32), sw128_desc(sb + k * 32), kIdesc,
+                    (kt | k) ? 1u : 0u);
+          umma_commit(&empty_bar[s]);
+        }
+        if (ok) umma_commit(&acc_full[b]);
+        else atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
+      }
+      it += g.kt;
+      ++done;
+      ok = __all_sync(0xffffffffu, ok);
+    }
+  } else if (warp >= 4) {
+    // ---- epilogue: residue sums -> digits
+    const int q = warp & 3;
+    const int c0 = ((warp - 4) >> 2) * (kTileN / 2);
+    const bool with_inverse = g.lower != 0;       // a Gramian's one set of residues has no factor
+    int64_t done = 0;
+    for (int64_t j = blockIdx.x; j < g.jobs; j += gridDim.x) {
+      Job jb;
+      if (!job_of(g, j, &jb) || tile_unused(g, jb)) continue;
+      const int b = int(done & 1);
+      // warp-uniform outcome: the TMEM loads below are .sync.aligned
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], uint32_t((done >> 1) & 1)));
+      fence_after();
+      if (!ok) {
+        if (lane == 0) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
+        break;
+      }
+      uint8_t* dst = g.y + (int64_t(jb.p) * g.y_rows + int64_t(jb.m) * kTileM + q * 32 + lane) * g.ldy +
+                     int64_t(jb.n) * kTileN + c0;
+#pragma unroll 1
+      for (int c = 0; c < kTileN / 64; ++c) {
+        uint32_t r[32];
+        tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(b * kTileN + c0 + c * 32), r);
+        uint32_t w[8];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) r[e] = rns::digit(int32_t(r[e]), kT, jb.p, with_inverse);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          w[e] = __byte_perm(__byte_perm(r[4 * e], r[4 * e + 1], 0x0040), __byte_perm(r[4 * e + 2], r[4 * e + 3], 0x0040),
+                             0x5410);
+        uint4* d = reinterpret_cast<uint4*>(dst + c * 32);
+        d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        d[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+      fence_before();
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+      ++done;
+    }
+  }
+  __syncwarp();
+  fence_before();
+  __syncthreads();
+  if (warp == 2) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+  }
+}
+
+// CRT: the digits of every modulus to FP64 (adding to C when add).  A thread takes four columns, a warp reads
+// 128 bytes of each plane.
+__global__ void __launch_bounds__(256) k_rns_crt(const uint8_t* __restrict__ y, int64_t y_rows, int64_t ldy, int64_t M,
+                                                 int64_t N, const double* __restrict__ ua,
+                                                 const double* __restrict__ ub, double* C, int64_t ldc, int add,
+                                                 int64_t lower_row0, const uint8_t* __restrict__ row_flag) {
+  const int64_t row = blockIdx.y;
+  if (row_flag[row]) return;
+  const int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int64_t col = 4 * q;
+  if (col >= N || (lower_row0 >= 0 && col > lower_row0 + row)) return;
+  const uint8_t* src = y + row * ldy + col;
+  const int64_t plane = y_rows * ldy;
+  rns::Crt acc[4];
+#pragma unroll
+  for (int i = 0; i < rns::kGroups; ++i) {
+    uint32_t w[3];
+#pragma unroll
+    for (int h = 0; h < 3; ++h) w[h] = *reinterpret_cast<const uint32_t*>(src + (3 * i + h) * plane);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      acc[j].add((w[0] >> (8 * j)) & 255u, (w[1] >> (8 * j)) & 255u, (w[2] >> (8 * j)) & 255u, kT, i);
+  }
+  const double sa = ua[row];
+  double* dst = C + row * ldc + col;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (col + j >= N) break;
+    const double v = acc[j].value(kT) * sa * ub[col + j];
+    dst[j] = add ? dst[j] + v : v;
+  }
+}
+
+// ---- host
+struct Work {   // workspace layout
+  uint8_t *pa, *pb, *y, *row_flag, *col_flag;
+  double *ua, *ub, *part;
+  int *scale, *any;
+  int64_t a_pad, b_pad, kp, y_rows, ldy;
+  size_t bytes;
+};
+
+size_t up(size_t b) { return (b + 1023) & ~size_t(1023); }
+
+Work layout(const RnsPlan& p, void* ws) {
+  Work w;
+  w.kp = cdiv(p.kc, kKTile) * kKTile;
+  w.a_pad = cdiv(p.mb, kTileM) * kTileM;
+  w.b_pad = cdiv(p.N, kTileN) * kTileN;
+  w.y_rows = w.a_pad;
+  w.ldy = w.b_pad;
+  char* base = static_cast<char*>(ws);
+  size_t off = 0;
+  auto take = [&](size_t b) { char* q = base + off; off += up(b); return q; };
+  w.pb = reinterpret_cast<uint8_t*>(take(size_t(kRnsModuli) * w.b_pad * w.kp));
+  w.pa = p.same ? w.pb : reinterpret_cast<uint8_t*>(take(size_t(kRnsModuli) * w.a_pad * w.kp));
+  w.y = reinterpret_cast<uint8_t*>(take(size_t(kRnsModuli) * w.y_rows * w.ldy));
+  const int64_t most = std::max(p.M, p.N);
+  w.part = reinterpret_cast<double*>(take(size_t(2 * cdiv(p.kc, kStatK)) * most * 8));   // of strided operands
+  w.scale = reinterpret_cast<int*>(take(size_t(most) * 4));
+  w.ub = reinterpret_cast<double*>(take(size_t(p.N) * 8));
+  w.ua = p.same ? w.ub : reinterpret_cast<double*>(take(size_t(p.M) * 8));
+  // one memset clears these
+  w.any = reinterpret_cast<int*>(take(up(sizeof(int)) + up(size_t(w.b_pad)) + (p.same ? 0 : up(size_t(p.M)))));
+  w.col_flag = reinterpret_cast<uint8_t*>(w.any) + up(sizeof(int));
+  w.row_flag = p.same ? w.col_flag : w.col_flag + up(size_t(w.b_pad));
+  w.bytes = off;
+  return w;
+}
+
+// Scales of R rows whose k runs along the other dimension (element (r, k) at x.p[r + k x.cs]).
+int strided_scales(Context* c, CMat x, int64_t R, int64_t K, bool is_b, const Work& w, const Out& o) {
+  const int chunks = int(cdiv(K, kStatK));
+  k_rns_colstats<<<dim3(unsigned(cdiv(R, 32)), unsigned(chunks)), 256, 0, c->stream>>>(x.p, x.cs, R, K, w.part);
+  k_rns_colscale<<<unsigned(cdiv(R, 256)), 256, 0, c->stream>>>(w.part, R, K, chunks, is_b ? rns::kTB : rns::kTA,
+                                                                w.scale, o);
+  c->kernels_launched += 2;
+  MB_CHECK_CUDA(cudaGetLastError());
+  return MCNLA_B200_OK;
+}
+
+// Residues of R rows (element (r, k) at x.p[r x.rs + k x.cs]); strided ones have their scales already, in `scale`.
+// is_b: B's, which carry the CRT's factors.
+int residues(Context* c, CMat x, int64_t R, int64_t K, bool is_b, const int* scale, const Out& o) {
+  if (x.cs == 1) {
+    const bool vec = (reinterpret_cast<uintptr_t>(x.p) & 15) == 0 && x.rs % 2 == 0;
+    auto kern = vec ? (is_b ? k_rns_rows<true, true> : k_rns_rows<true, false>)
+                    : (is_b ? k_rns_rows<false, true> : k_rns_rows<false, false>);
+    kern<<<unsigned(R), kRowThreads, 0, c->stream>>>(x.p, x.rs, K, is_b ? rns::kTB : rns::kTA, o);
+  } else {
+    auto kern = is_b ? k_rns_cols<true> : k_rns_cols<false>;
+    kern<<<dim3(unsigned(o.kp / kKTile), unsigned(cdiv(R, kColTile))), 256, 0, c->stream>>>(x.p, x.cs, R, K, scale, o);
+  }
+  c->kernels_launched++;
+  MB_CHECK_CUDA(cudaGetLastError());
+  return MCNLA_B200_OK;
+}
+
+}  // namespace
+
+// Where the line lies: estimated microseconds of both paths.  The DMMA GEMM runs at ~31 TFLOP/s on tiles
+// of 128 columns; the int8 path costs 8.5 ps an element of A (two passes, 15 residues), 10 ps of B, 12 ps an
+// element of C (digits and CRT), 15 int8 products on 128 x 256 tiles at ~2.6 POP/s (below K = 1024 the
+// epilogue bounds a tile) and ~40 us of launches.  Measured, DMMA and int8 in us for M x K by N columns:
+//   2048 x 1024:  512: 152, 144   768: 191, 157   1536: 321, 194
+//   4096 x 4096:  128: 240, 273   192: 417, 277    768: 994, 375   1536: 1844, 544
+//   16384 x 1024: 128: 236, 337   192: 399, 351    512: 662, 408   1536: 1739, 760
+//   16384 x 256: 1536: 516, 586   700 x 8192: 384: 208, 220   512: 251, 229
+//   100000 x 20000: 4096: 490800, 122000
+// A Gramian's triangle halves the products of both.
+RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, int64_t max_rows) {
+  RnsPlan p;
+  p.M = M; p.N = N; p.K = K; p.same = same;
+  if (M < 1 || N < 1 || K < 1) return p;
+  const double m = double(M), n = double(N), k = double(K), half = same ? 0.5 : 1.0;
+  const double n128 = double(cdiv(N, 128)) * 128.0;
+  const double tiles = double(cdiv(M, kTileM)) * double(cdiv(N, kTileN));
+  const double computed = same ? 0.5 * (tiles + 2.0 * double(cdiv(N, kTileM))) : tiles;   // a triangle's diagonal tiles are whole
+  const double dmma = half * 2.0 * m * n128 * k / 31e6;
+  const double int8 = 40.0 + (same ? 0.0 : 8.5e-6 * m * k) + 10e-6 * n * k + half * 12e-6 * m * n +
+                      computed * double(kTileM) * kTileN * 2.0 * kRnsModuli * std::max(k, 1024.0) / 2.6e9;
+  if (int8 >= dmma) return p;
+  if (c && c->smem_optin < kGemmSmem) return p;
+  // B's planes within ~1.3 GB (a Gramian's, beside the integrator's state, 0.5 GB): K in chunks of equal size
+  const int64_t b_pad = cdiv(N, kTileN) * kTileN;
+  const int64_t b_most = int64_t(same ? 512 : 1300) << 20;
+  const int64_t most = std::min<int64_t>(kMaxChunk, std::max<int64_t>(4096, b_most / (kRnsModuli * b_pad)));
+  p.chunks = int(cdiv(K, most));
+  p.kc = p.chunks == 1 ? K : cdiv(cdiv(K, p.chunks), kKTile) * kKTile;
+  p.chunks = int(cdiv(K, p.kc));
+  // A's planes and the digits of a block of rows within twice C's size, 320 MB at least and 0.7 GB at most; among
+  // those, the block whose tiles fill the SMs' waves best (a k-tile takes ~0.48 us, a block's launches ~10 us)
+  const int64_t kp = cdiv(p.kc, kKTile) * kKTile;
+  const int64_t rows = max_rows > 0 ? std::min(max_rows, M) : M;
+  const int64_t cap = std::min<int64_t>(int64_t(700) << 20, std::max<int64_t>(int64_t(320) << 20, 16 * M * N));
+  const int64_t row_bytes = kRnsModuli * ((same ? 0 : kp) + b_pad);
+  const int64_t panels = cdiv(rows, kTileM), most_panels = std::max<int64_t>(1, cap / row_bytes / kTileM);
+  const int64_t sms = c ? c->num_sms : 148, per_panel = kRnsModuli * cdiv(N, kTileN);
+  double best = 0.0;
+  for (int64_t q = 1; q <= std::min(panels, most_panels); ++q) {
+    const double us = double(cdiv(panels, q)) * (double(cdiv(q * per_panel, sms)) * 0.48 * double(kp / kKTile) + 10.0);
+    if (p.mb == 0 || us <= best) {
+      best = us;
+      p.mb = std::min(rows, q * kTileM);
+    }
+  }
+  // a plane's row index is a 32-bit tensor coordinate, a grid dimension at most 65535
+  if (kRnsModuli * b_pad > INT32_MAX / 2 || cdiv(N, kColTile) > 65535 || p.mb > 65535 || cdiv(K, kStatK) > 65535) return p;
+  p.bytes = layout(p, nullptr).bytes + 1024;
+  p.use = true;
+  return p;
+}
+
+int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat C, void* ws, double* dws, int splits,
+             bool reuse_b) {
+  if (!plan.use || !ws) return MCNLA_B200_ERR_ARG;
+  if (C.cs != 1) return MCNLA_B200_ERR_LAYOUT;
+  if ((A.cs != 1 && A.rs != 1) || (B.cs != 1 && B.rs != 1)) return MCNLA_B200_ERR_LAYOUT;
+  if (rows < 1 || rows > plan.M || (plan.same && rows != plan.N)) return MCNLA_B200_ERR_SHAPE;
+  const Work w = layout(plan, reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~uintptr_t(1023)));
+  const bool keep_b = reuse_b && plan.chunks == 1 && !plan.same;
+  // `any` and the flags collect over chunks and blocks; a kept B keeps its own flags
+  if (keep_b) MB_CHECK_CUDA(cudaMemsetAsync(w.row_flag, 0, size_t(rows), c->stream));
+  else MB_CHECK_CUDA(cudaMemsetAsync(w.any, 0, up(sizeof(int)) + up(size_t(w.b_pad)) + (plan.same ? 0 : size_t(rows)),
+                                     c->stream));
+  static std::atomic<uint64_t> attr_set{0};   // the shared-memory opt-in: one bit per device
+  const uint64_t bit = uint64_t(1) << (c->device & 63);
+  if (!(attr_set.load(std::memory_order_acquire) & bit)) {
+    MB_CHECK_CUDA(cudaFuncSetAttribute(rns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGemmSmem)));
+    attr_set.fetch_or(bit, std::memory_order_acq_rel);
+  }
+  for (int ch = 0; ch < plan.chunks; ++ch) {
+    const int64_t k0 = ch * plan.kc, kn = std::min(plan.kc, plan.K - k0);
+    const int64_t kp = cdiv(kn, kKTile) * kKTile;
+    if (!keep_b) {
+      const Out ob{w.pb, w.b_pad, kp, w.ub, w.col_flag, w.any};
+      const CMat b = cm(B.p + k0 * B.rs, B.cs, B.rs);
+      if (b.cs != 1) MB_CHECK(strided_scales(c, b, plan.N, kn, !plan.same, w, ob));
+      MB_CHECK(residues(c, b, plan.N, kn, !plan.same, w.scale, ob));
+    }
+    // A's strided scales: all rows at once (after B's residues, which share the scratch)
+    const CMat ak = cm(A.p + k0 * A.cs, A.rs, A.cs);
+    const bool strided = !plan.same && A.cs != 1;
+    if (strided) MB_CHECK(strided_scales(c, ak, rows, kn, false, w, Out{nullptr, 0, kp, w.ua, w.row_flag, w.any}));
+    CUtensorMap tb;
+    MB_CHECK(make_map_u8(&tb, w.pb, kRnsModuli * w.b_pad, kp, kp, kKTile, kTileN));
+    for (int64_t r0 = 0; r0 < rows; r0 += plan.mb) {
+      const int64_t rn = std::min(plan.mb, rows - r0);
+      CUtensorMap ta;
+      if (!plan.same) {
+        const Out oa{w.pa, w.a_pad, kp, w.ua + r0, w.row_flag + r0, w.any};
+        MB_CHECK(residues(c, cm(ak.p + r0 * A.rs, A.rs, A.cs), rn, kn, false, w.scale + r0, oa));
+        MB_CHECK(make_map_u8(&ta, w.pa, kRnsModuli * w.a_pad, kp, kp, kKTile, kTileM));
+      } else {
+        MB_CHECK(make_map_u8(&ta, w.pb, kRnsModuli * w.b_pad, kp, kp, kKTile, kTileM));
+      }
+      GemmArgs g;
+      g.a_rows_pad = plan.same ? w.b_pad : w.a_pad;
+      g.b_rows_pad = w.b_pad;
+      g.a_row0 = plan.same ? int(r0) : 0;
+      g.mt = int(cdiv(rn, kTileM));
+      g.nt = int(cdiv(plan.N, kTileN));
+      g.kt = int(kp / kKTile);
+      g.lower = plan.same ? 1 : 0;
+      g.jobs = int64_t(kRnsModuli) * g.mt * g.nt;
+      g.y = w.y;
+      g.y_rows = w.y_rows;
+      g.ldy = w.ldy;
+      g.row_flag = w.row_flag + r0;
+      g.col_flag = w.col_flag;
+      g.any = w.any;
+      g.M = int(rn);
+      g.N = int(plan.N);
+      g.status = &c->scal->wait_status;
+      rns_gemm_kernel<<<unsigned(std::min<int64_t>(g.jobs, c->num_sms)), kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
+      MB_CHECK_CUDA(cudaGetLastError());
+      k_rns_crt<<<dim3(unsigned(cdiv(plan.N, 1024)), unsigned(rn)), 256, 0, c->stream>>>(
+          w.y, w.y_rows, w.ldy, rn, plan.N, w.ua + r0, w.ub, C.p + r0 * C.rs, C.rs, ch > 0,
+          plan.same ? r0 : -1, w.row_flag + r0);
+      MB_CHECK_CUDA(cudaGetLastError());
+      c->kernels_launched += 2;
+    }
+  }
+  // what was flagged, over the whole K
+  GemmFlags fl;
+  fl.row = w.row_flag;
+  fl.col = w.col_flag;
+  fl.any = w.any;
+  return dgemm(c, rows, plan.N, plan.K, 1.0, A, B, 0.0, C, GemmBatch(), dws, splits, plan.same, &fl);
+}
+
+}  // namespace mb

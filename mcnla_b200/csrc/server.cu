@@ -12,6 +12,7 @@
 // block nothing are kept.  Results do not depend on what else is in flight:
 // every kernel reduces in a fixed order.
 #include "common.cuh"
+#include "rns.cuh"
 #include "solve.cuh"
 
 #include <algorithm>
@@ -52,9 +53,15 @@ int64_t problem_bytes(const mcnla_b200_problem& p) {
   int64_t bytes = (m * L + m * l) * 8 + (mixed ? L * round8(n) * 2 : n * L * 8);  // Q, Qbar, Omega
   int64_t stage = m * L * 8 + 5 * l * l * p.params.num_sketch * 8;              // orthogonalizer
   stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + 4 * m * 2 * l * 8);   // integrators
+  // the int8 products' workspaces past the 64 MB below: an FP64 sketch's (a mixed solve is counted with it too, and
+  // leaves it unused), and a KN Gramian's beside its state
+  const int64_t small = int64_t(64) << 20;
+  stage = std::max(stage, int64_t(mb::plan_rns(nullptr, m, L, n, false).bytes) - small);
+  if (p.integrator == MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO)
+    stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + int64_t(mb::plan_rns(nullptr, L, L, m, true).bytes) - small);
   stage = std::max(stage, 4 * l * n * 8 + n * l * 8);                           // formers
   if (mixed) stage = std::max(stage, 3 * l * round8(m) * 2 + 16 * l * n * 8);   // precision former
-  bytes += stage + (int64_t(64) << 20);                                         // + split-K partials, small terms
+  bytes += stage + small;                                                       // + split-K partials, small terms
   bytes += int64_t(mb::problem_scratch_bytes(p));                               // FP64 copy or BF16 parts of A, A'
   const bool gramian = p.integrator == MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO ||
                        p.integrator == MCNLA_B200_ROW_BLOCK_GRAMIAN_WEN_YIN;

@@ -12,6 +12,7 @@
 #include "dgemm.cuh"
 #include "kernels.cuh"
 #include "bf16.cuh"
+#include "rns.cuh"
 #include "solve.cuh"
 #include <algorithm>
 #include <array>
@@ -91,18 +92,28 @@ int run_sketch(Context* c, const Dims& d, const double* A, int layout, int64_t l
   if (layout == MCNLA_B200_ROW_MAJOR ? lda < d.n : lda < d.m) return MCNLA_B200_ERR_SHAPE;
   if (exponent < 0) return MCNLA_B200_ERR_ARG;
   const CMat Am = layout == MCNLA_B200_ROW_MAJOR ? crow(A, lda) : ccol(A, lda);
+  // large products run on the int8 tensor cores (rns.cuh)
+  const RnsPlan fwd = plan_rns(c, d.m, d.L, d.n, false);
+  const RnsPlan back = exponent > 0 ? plan_rns(c, d.n, d.L, d.m, false) : RnsPlan();
+  const size_t wsr = std::max(fwd.bytes, back.bytes);
   Plan pl;
   pl.add(gemm_ws(c, {{d.m, d.L, d.n, 1}, {d.n, d.L, d.m, 1}}) / 8 + 1);
+  pl.add(wsr, 1);
   MB_CHECK(ctx_reserve(c, pl.bytes));
   double* ws = take_ws(c, gemm_ws(c, {{d.m, d.L, d.n, 1}, {d.n, d.L, d.m, 1}}));
+  char* wr = ctx_take<char>(c, wsr);
   MB_CHECK(check_arena(c));
+  auto mul = [&](const RnsPlan& plan, int64_t rows, int64_t k, CMat x, double* in, double* out) -> int {
+    if (plan.use) return rns_gemm(c, plan, rows, x, crow(in, d.L), drow(out, d.L), wr, ws, 0, false);
+    return dgemm(c, rows, d.L, k, 1.0, x, crow(in, d.L), 0.0, drow(out, d.L), GemmBatch(), ws);
+  };
   if (!timed_generation) { MB_CHECK(ctx_tic(c)); MB_CHECK(ctx_toc(c)); }   // "random generating" part
   // Q := A * Omega   (gaussian_projection_sketcher.hpp:96)
-  MB_CHECK(dgemm(c, d.m, d.L, d.n, 1.0, Am, crow(omega, d.L), 0.0, drow(Q, d.L), GemmBatch(), ws));
+  MB_CHECK(mul(fwd, d.m, d.n, Am, omega, Q));
   // power iterations (gaussian_projection_sketcher.hpp:97-100)
   for (int i = 0; i < exponent; ++i) {
-    MB_CHECK(dgemm(c, d.n, d.L, d.m, 1.0, ctr(Am), crow(Q, d.L), 0.0, drow(omega, d.L), GemmBatch(), ws));
-    MB_CHECK(dgemm(c, d.m, d.L, d.n, 1.0, Am, crow(omega, d.L), 0.0, drow(Q, d.L), GemmBatch(), ws));
+    MB_CHECK(mul(back, d.n, d.m, ctr(Am), Q, omega));
+    MB_CHECK(mul(fwd, d.m, d.n, Am, omega, Q));
   }
   MB_CHECK(ctx_toc(c));
   return MCNLA_B200_OK;
@@ -379,9 +390,13 @@ int gramian_bs_bf16(Context* c, const Dims& d, const double* Qs, double* Bs, uin
 // Bs := Qs' Qs with the reference's triangle convention (see launch_gramian_prepare):
 // the lower triangle only (the reference's syrk), mirrored afterwards.
 // x: gramian_bs16_count(d) BF16 elements of workspace when c->mixed_gramian
+// plan, wr: the int8 product's plan and workspace.  The Wen-Yin integrator passes none: it carries a rounding
+// of Bs into its step sizes (a change of 1e-16 moves its result by up to 1e-7), so it
+// keeps the sums of the DMMA GEMM.
 int gramian_bs(Context* c, const Dims& d, const double* Qs, double* Bs, double* Bc, int64_t ldbc, double* ws,
-               uint16_t* x) {
+               uint16_t* x, const RnsPlan& plan, void* wr) {
   if (c->mixed_gramian) MB_CHECK(gramian_bs_bf16(c, d, Qs, Bs, x));
+  else if (plan.use) MB_CHECK(rns_gemm(c, plan, d.L, cm(Qs, 1, d.L), crow(Qs, d.L), drow(Bs, d.L), wr, ws, 0, false));
   else MB_CHECK(dgemm(c, d.L, d.L, d.m, 1.0, cm(Qs, 1, d.L), crow(Qs, d.L), 0.0, drow(Bs, d.L), GemmBatch(), ws, 0,
                       true));
   // row blocks over ranks (row_block_gramian_kolmogorov_nagumo_integrator.hpp:117,
@@ -432,6 +447,11 @@ int gramian_form_qbar(Context* c, const Dims& d, const double* Qs, const double*
 size_t gkn_ws_bytes(const Context* c, const Dims& d) {
   const int64_t L = d.L, l = d.l, m = d.m;
   return gemm_ws(c, {{L, L, m, 1}, {L, l, L, 1}, {l, 2 * l, L, 1}, {L, l, 2 * l, 2}, {m, l, L, 1}});
+}
+
+// The int8 plan of Bs = Qs' Qs.
+RnsPlan gkn_bs_plan(const Context* c, const Dims& d) {
+  return c->mixed_gramian ? RnsPlan() : plan_rns(c, d.L, d.L, d.m, true);
 }
 
 // Visits the buffers in carve order: fn(count, element bytes).
@@ -523,10 +543,11 @@ GknJob gkn_job(const Context* c, const Dims& d, const GknBufs& b, int it0, int m
 }
 
 // Bs := Qs' Qs; Bc := Bs(:, 0:l); F~ := I; E~ := 0   (:112-133)
-int gkn_prepare(Context* c, const Dims& d, const double* Qs, const GknBufs& b, double* ws) {
+int gkn_prepare(Context* c, const Dims& d, const double* Qs, const GknBufs& b, double* ws, const RnsPlan& plan,
+                void* wr) {
   const int l = d.l;
   const int64_t L = d.L, l3 = 3 * l;
-  MB_CHECK(gramian_bs(c, d, Qs, b.Bs, b.EB[0] + l, l3, ws, b.bs16));
+  MB_CHECK(gramian_bs(c, d, Qs, b.Bs, b.EB[0] + l, l3, ws, b.bs16, plan, wr));
   MB_CHECK(launch_fill(c, L, l, 0.0, b.EB[0], l3));
   MB_CHECK(launch_set_identity(c, l, b.FF[0], l));
   const int64_t ldL = (L + 7) & ~int64_t(7);
@@ -586,6 +607,8 @@ int run_rb_gramian_kn(Context* c, const Dims& d, const double* Qs, int maxit, do
   Plan pl;
   gkn_layout(c, d, [&](size_t count, size_t elem) { pl.add(count, elem); });
   pl.add(wsb / 8 + 1);
+  const RnsPlan plan = gkn_bs_plan(c, d);
+  pl.add(plan.bytes, 1);
   MB_CHECK(ctx_reserve(c, pl.bytes));
   GknBufs b;
   gkn_carve(c, d, [&](size_t count, size_t elem) -> char* {
@@ -593,9 +616,10 @@ int run_rb_gramian_kn(Context* c, const Dims& d, const double* Qs, int maxit, do
                      : reinterpret_cast<char*>(ctx_take<double>(c, count));
   }, b);
   double* ws = take_ws(c, wsb);
+  char* wr = ctx_take<char>(c, plan.bytes);
   MB_CHECK(check_arena(c));
   MB_CHECK(ctx_tic(c));
-  MB_CHECK(gkn_prepare(c, d, Qs, b, ws));
+  MB_CHECK(gkn_prepare(c, d, Qs, b, ws, plan, wr));
   MB_CHECK(ctx_toc(c));
   auto body = [&](int i, bool allow_series) -> int { return gkn_iteration(c, d, b, i, allow_series, tol, ws); };
   int it = 0;
@@ -675,7 +699,7 @@ int run_rb_wy(Context* c, const Dims& d, const double* Qs, int maxit, double tol
   double* partials = ctx_take<double>(c, size_t(np));
   double* ws = take_ws(c, wsb);
   MB_CHECK(check_arena(c));
-  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+  MB_CHECK(ctx_reset_scalars(c));
   MB_CHECK(ctx_tic(c));
   // Initializing (:112-143)
   MB_CHECK(copy2d(c, QG[0], l2, Qs, L, m, l));                                                        // Qc := Q0
@@ -777,10 +801,10 @@ int run_rb_gramian_wy(Context* c, const Dims& d, const double* Qs, int maxit, do
   double* partials = ctx_take<double>(c, size_t(np));
   double* ws = take_ws(c, wsb);
   MB_CHECK(check_arena(c));
-  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+  MB_CHECK(ctx_reset_scalars(c));
   MB_CHECK(ctx_tic(c));
   // Initializing (:121-155)
-  MB_CHECK(gramian_bs(c, d, Qs, Bs, EB[0] + l, l3, ws, bs16));
+  MB_CHECK(gramian_bs(c, d, Qs, Bs, EB[0] + l, l3, ws, bs16, RnsPlan(), nullptr));
   MB_CHECK(dgemm(c, L, l, L, inv_n, crow(Bs, L), crow(EB[0] + l, l3), 0.0, drow(EB[0] + l2, l3), GemmBatch(), ws));
   MB_CHECK(dgemm(c, l, l2, L, inv_n, cm(EB[0] + l, 1, l3), crow(EB[0] + l, l3), 0.0, drow(DD[0], l2), GemmBatch(), ws));
   MB_CHECK(launch_set_identity(c, l, FF[0], l));
@@ -863,7 +887,7 @@ int run_integrate(Context* c, const Dims& d, int kind, const double* Qs, int max
   if (!Qs || !Qbar || !iters) return MCNLA_B200_ERR_ARG;
   if (maxit < 0 || !(tol >= 0.0)) return MCNLA_B200_ERR_ARG;
   // device status, convergence scalars and grid-barrier counters start clean
-  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+  MB_CHECK(ctx_reset_scalars(c));
   switch (kind) {
     case MCNLA_B200_KOLMOGOROV_NAGUMO: return run_kn(c, d, Qs, maxit, tol, Qbar, iters);
     case MCNLA_B200_ROW_BLOCK_KOLMOGOROV_NAGUMO: return run_rb_kn(c, d, Qs, maxit, tol, Qbar, iters);
@@ -1087,6 +1111,7 @@ struct RowBlocks {
   int64_t first;      // rows of the first block
   int nblocks;
   int splits;
+  RnsPlan rns;        // the whole product's int8 plan, for blocks of rows_per rows
   int64_t start(int b) const { return b == 0 ? 0 : first + int64_t(b - 1) * rows_per; }
   int64_t rows(int b, int64_t m) const { return std::min<int64_t>(b == 0 ? first : rows_per, m - start(b)); }
 };
@@ -1098,6 +1123,7 @@ RowBlocks stream_blocks(Context* c, const Dims& d) {
   rb.first = std::min<int64_t>(rb.rows_per, std::max<int64_t>(128, int64_t((size_t(128) << 20) / row_bytes)));
   rb.nblocks = 1 + int(cdiv(std::max<int64_t>(0, d.m - rb.first), rb.rows_per));
   rb.splits = dgemm_heuristic_splits(c, d.m, d.L, d.n, 1);
+  rb.rns = plan_rns(c, d.m, d.L, d.n, false, rb.rows_per);
   return rb;
 }
 
@@ -1107,6 +1133,7 @@ RowBlocks stream_blocks(Context* c, const Dims& d) {
 struct StreamSetup {
   std::vector<cudaEvent_t> ev;
   double* ws = nullptr;
+  char* wr = nullptr;   // the int8 product's workspace (Omega's residues stay in it from block to block)
   ~StreamSetup() {
     for (auto e : ev)
       if (e) cudaEventDestroy(e);
@@ -1118,8 +1145,10 @@ int stream_setup(Context* c, const Dims& d, const RowBlocks& rb, const double* o
   const size_t wsb = rb.splits > 1 ? size_t(rb.splits) * rb.rows_per * d.L * sizeof(double) : 0;
   Plan pl;
   pl.add(wsb / 8 + 1);
+  pl.add(rb.rns.bytes, 1);
   MB_CHECK(ctx_reserve(c, pl.bytes));
   st.ws = take_ws(c, wsb);
+  st.wr = ctx_take<char>(c, rb.rns.bytes);
   MB_CHECK(check_arena(c));
   if (!c->copy_stream) MB_CHECK_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
   st.ev.assign(size_t(rb.nblocks) + 1, nullptr);
@@ -1138,6 +1167,9 @@ int sketch_block(Context* c, const Dims& d, const RowBlocks& rb, const StreamSet
                  const double* omega, double* Q) {
   const int64_t r0 = rb.start(b), rows = rb.rows(b, d.m);
   MB_CHECK_CUDA(cudaStreamWaitEvent(c->stream, st.ev[b], 0));
+  if (rb.rns.use)
+    return rns_gemm(c, rb.rns, rows, crow(A + r0 * d.n, d.n), crow(omega, d.L), drow(Q + r0 * d.L, d.L), st.wr, st.ws,
+                    rb.splits, b > 0);
   return dgemm(c, rows, d.L, d.n, 1.0, crow(A + r0 * d.n, d.n), crow(omega, d.L), 0.0, drow(Q + r0 * d.L, d.L),
                GemmBatch(), st.ws, rb.splits);
 }
@@ -1212,7 +1244,7 @@ int run_isvd_mixed(Context* c, const Dims& d, int integrator, int former, const 
   double* Q = reinterpret_cast<double*>(take(size_t(d.m) * d.L * 8));
   double* Qbar = reinterpret_cast<double*>(take(size_t(d.m) * d.l * 8));
   uint16_t* omega_t = reinterpret_cast<uint16_t*>(take(size_t(d.L) * ldo * 2));
-  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+  MB_CHECK(ctx_reset_scalars(c));
   MB_CHECK(ctx_tic(c));
   MB_CHECK(launch_gaussian_bf16(c, seed, d.n, d.L, omega_t, ldo, nullptr));
   MB_CHECK(ctx_toc(c));
@@ -1267,6 +1299,9 @@ size_t stage_bytes_upper(Context* c, const Dims& d) {
   b = std::max(b, size_t(L) * L * 8 + 8 * size_t(L) * 3 * l * 8 + 4 * size_t(m) * 2 * l * 8 +
                       gemm_ws(c, {{L, L, m, 1}, {L, l, m, 1}, {m, l, L, 1}, {l, 2 * l, L, 1}}));
   b = std::max(b, 3 * size_t(l) * n * 8 + size_t(n) * l * 8 + gemm_ws(c, {{l, n, m, 1}, {n, l, m, 1}, {l, l, n, 1}}));
+  // the int8 products: the sketch alone, Bs beside the Gramian integrator's state
+  b = std::max(b, plan_rns(c, m, L, n, false).bytes + gemm_ws(c, {{m, L, n, 1}}));
+  b = std::max(b, gkn_bs_plan(c, d).bytes + gkn_state_bytes(c, d) + gkn_ws_bytes(c, d));
   return b + (64 << 20);
 }
 
@@ -1495,16 +1530,19 @@ int gitem_phase_a(Context* c, GItem& it, SolveScratch& s) {
     int64_t ld16 = 0;
     MB_CHECK(problem_parts(c, p, s, part, &ld16));
     const int64_t ldo = (d.n + 7) & ~int64_t(7);
-    MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+    MB_CHECK(ctx_reset_scalars(c));
     MB_CHECK(launch_gaussian_bf16(c, p.seed, d.n, d.L, it.omega_t, ldo, nullptr));
     MB_CHECK(bf16_gemm(c, d.m, d.L, d.n, part[0], part[1], part[2], ld16, it.omega_t, ldo, it.Q, d.L, true));
   }
   MB_CHECK(run_orthogonalize(c, d, it.Q));
-  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+  MB_CHECK(ctx_reset_scalars(c));
   const size_t wsb = gkn_ws_bytes(c, d);
-  MB_CHECK(ctx_reserve(c, wsb + 512));
+  const RnsPlan plan = gkn_bs_plan(c, d);
+  MB_CHECK(ctx_reserve(c, arena_bytes_for(wsb + 8, 1) + arena_bytes_for(plan.bytes, 1)));
   double* ws = take_ws(c, wsb);
-  MB_CHECK(gkn_prepare(c, d, it.Q, it.b, ws));
+  char* wr = ctx_take<char>(c, plan.bytes);
+  MB_CHECK(check_arena(c));
+  MB_CHECK(gkn_prepare(c, d, it.Q, it.b, ws, plan, wr));
   MB_CHECK(ctx_sync_scalars(c));
   return c->scal_host->status;
 }
@@ -1516,7 +1554,7 @@ int gitem_fallback(Context* c, GItem& it, int r) {
   const size_t wsb = gkn_ws_bytes(c, d);
   MB_CHECK(ctx_reserve(c, wsb + 512));
   double* ws = take_ws(c, wsb);
-  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+  MB_CHECK(ctx_reset_scalars(c));
   MB_CHECK_CUDA(cudaMemsetAsync(&c->scal->stop_it, 0x7f, sizeof(int), c->stream));
   {
     struct Reset { Context* c; ~Reset() { c->guard_stop = nullptr; c->guard_it = 0; } } reset{c};
@@ -1546,7 +1584,7 @@ int gitem_phase_c(Context* c, GItem& it, SolveScratch& s) {
   const size_t wsb = gkn_ws_bytes(c, d);
   MB_CHECK(ctx_reserve(c, wsb + 512));
   double* ws = take_ws(c, wsb);
-  MB_CHECK_CUDA(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
+  MB_CHECK(ctx_reset_scalars(c));
   MB_CHECK(gkn_finish(c, d, it.Q, it.b, it.iters, it.Qbar, ws));
   if (!problem_mixed(p)) {
     const double* A = nullptr;
@@ -1717,7 +1755,8 @@ int batched_solve(int device, mcnla_b200_problem* problems, int count, int worke
   size_t worker_bytes = 0;
   for (auto& it : items) {
     worker_bytes = std::max(worker_bytes, problem_scratch_bytes(*it.p) + size_t(it.d.m) * it.d.L * 8 +
-                                              gkn_ws_bytes(ctx[0], it.d) + (size_t(64) << 20));
+                                              gkn_ws_bytes(ctx[0], it.d) + gkn_bs_plan(ctx[0], it.d).bytes +
+                                              (size_t(64) << 20));
   }
   const int64_t wave_cap = std::max<int64_t>(1, budget - int64_t(worker_bytes) * workers);
   size_t pos = 0;
@@ -1949,7 +1988,7 @@ int mcnla_b200_isvd_stream(mcnla_b200_ctx* ctx, const mcnla_b200_params* params,
   double* Qbar = reinterpret_cast<double*>(base + mb::arena_bytes_for(size_t(d.m) * d.L, 8));
   double* omega_dev = reinterpret_cast<double*>(base + mb::arena_bytes_for(size_t(d.m) * d.L, 8) +
                                                 mb::arena_bytes_for(size_t(d.m) * d.l, 8));
-  MB_CHECK_CUDA(cudaMemsetAsync(ctx->scal, 0, sizeof(mb::DevScalars), ctx->stream));
+  MB_CHECK(mb::ctx_reset_scalars(ctx));
   MB_CHECK(mb::run_sketch_ingest(ctx, d, read_rows, user, A, omega_host, omega_dev, Q));
   MB_CHECK(mb::run_orthogonalize(ctx, d, Q));
   MB_CHECK(mb::run_integrate(ctx, d, integrator, Q, max_iteration, tolerance, Qbar, iteration));
@@ -1987,7 +2026,7 @@ int mcnla_b200_dgemm(mcnla_b200_ctx* ctx, int64_t M, int64_t N, int64_t K, doubl
 int mcnla_b200_inverse_batched(mcnla_b200_ctx* ctx, int n, int batch, double* A) {
   if (!ctx || !A || n < 1 || batch < 1) return MCNLA_B200_ERR_ARG;
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  MB_CHECK_CUDA(cudaMemsetAsync(ctx->scal, 0, sizeof(mb::DevScalars), ctx->stream));
+  MB_CHECK(mb::ctx_reset_scalars(ctx));
   MB_CHECK(mb::launch_inverse(ctx, n, batch, A));
   MB_CHECK(mb::ctx_sync_scalars(ctx));
   return ctx->scal_host->status ? ctx->scal_host->status : MCNLA_B200_OK;
@@ -2014,7 +2053,7 @@ int mcnla_b200_gemm_bf16(mcnla_b200_ctx* ctx, int64_t M, int64_t N, int64_t K, c
                          void* D, int64_t ldd, int out_fp64) {
   if (!ctx || !a_hi || !b || !D || ldd < N) return MCNLA_B200_ERR_ARG;
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  MB_CHECK_CUDA(cudaMemsetAsync(ctx->scal, 0, sizeof(mb::DevScalars), ctx->stream));
+  MB_CHECK(mb::ctx_reset_scalars(ctx));
   MB_CHECK(mb::bf16_gemm(ctx, M, N, K, a_hi, a_lo, a_lo2, lda, b, ldb, D, ldd, out_fp64 != 0));
   MB_CHECK(mb::ctx_sync_scalars(ctx));
   return ctx->scal_host->status ? ctx->scal_host->status : MCNLA_B200_OK;
@@ -2027,7 +2066,7 @@ int mcnla_b200_sketch_bf16(mcnla_b200_ctx* ctx, const mcnla_b200_params* params,
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  MB_CHECK_CUDA(cudaMemsetAsync(ctx->scal, 0, sizeof(mb::DevScalars), ctx->stream));
+  MB_CHECK(mb::ctx_reset_scalars(ctx));
   MB_CHECK(mb::ctx_tic(ctx));
   MB_CHECK(mb::ctx_toc(ctx));
   MB_CHECK(mb::bf16_gemm(ctx, d.m, d.L, d.n, a_hi, a_lo, a_lo2, lda16, omega_t, ldo, Q, d.L, true));
@@ -2044,7 +2083,7 @@ int mcnla_b200_form_bf16(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, i
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  MB_CHECK_CUDA(cudaMemsetAsync(ctx->scal, 0, sizeof(mb::DevScalars), ctx->stream));
+  MB_CHECK(mb::ctx_reset_scalars(ctx));
   mb::AtParts at;
   at.hi = at_hi;
   at.lo = at_lo;
