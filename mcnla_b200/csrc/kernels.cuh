@@ -10,8 +10,10 @@ namespace mb {
 // batch stride a_bs): eigenvalues to W (batch stride n), eigenvectors as the
 // columns of V (row-major n x n, batch stride n*n).  order 0: ascending;
 // order 1: descending by |lambda| with W = |lambda| (gesvd of a PSD matrix).
+// work: syev_work_bytes(n, batch) bytes of device memory, 256-byte aligned.
 int launch_syev(Context* c, int n, int batch, const double* A, int64_t lda, int64_t a_bs, double* W, double* V,
-                int order);
+                int order, void* work);
+size_t syev_work_bytes(int n, int batch);
 
 // Scales the columns of V (row-major n x n, batch) by 1/sqrt(W): T = V diag(W^-1/2)
 // (the orthogonalizer's Q_i := Y_i V_i S_i^-1/2 step).

@@ -49,63 +49,6 @@ __device__ small::JacobiScratch carve_jacobi(SmemCarve& sc, int n) {
   return js;
 }
 
-// rank[j] = position of eigenvalue j in the requested order (ties by index).
-__device__ void eig_ranks(const double* a, int lda, int n, int order, int* rank) {
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const double dj = order ? fabs(a[j * lda + j]) : a[j * lda + j];
-    int r = 0;
-    for (int i = 0; i < n; ++i) {
-      const double di = order ? fabs(a[i * lda + i]) : a[i * lda + i];
-      const bool before = order ? (di > dj || (di == dj && i < j)) : (di < dj || (di == dj && i < j));
-      r += before ? 1 : 0;
-    }
-    rank[j] = r;
-  }
-  __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
-// batched symmetric eigendecomposition
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kSyevThreads) k_syev(int n, const double* A, int64_t lda, int64_t a_bs,
-                                                        double* W, double* V, int order, int v_smem,
-                                                        double* vwork_all) {
-  extern __shared__ __align__(16) char smem_raw[];
-  SmemCarve sc(smem_raw);
-  const int ld = n + 1;
-  double* a = sc.take<double>(size_t(n) * ld);
-  double* v;
-  int ldv;
-  if (v_smem) { v = sc.take<double>(size_t(n) * ld); ldv = ld; }
-  else { v = vwork_all + size_t(blockIdx.x) * n * n; ldv = n; }
-  small::JacobiScratch js = carve_jacobi(sc, n);
-  int* rank = sc.take<int>(n);
-  const double* Ab = A + blockIdx.x * a_bs;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) a[(e / n) * ld + (e % n)] = Ab[(e / n) * lda + (e % n)];
-  __syncthreads();
-  small::cta_jacobi_eig(a, ld, v, ldv, n, true, js, kMaxSweeps);
-  eig_ranks(a, ld, n, order, rank);
-  double* Wb = W + size_t(blockIdx.x) * n;
-  double* Vb = V + size_t(blockIdx.x) * n * n;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const double d = a[j * ld + j];
-    Wb[rank[j]] = order ? fabs(d) : d;
-  }
-  if (v_smem) {
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const int i = e / n, j = e % n;
-      Vb[i * n + rank[j]] = v[j * ldv + i];
-    }
-  } else {
-    __syncthreads();
-    // eigenvectors (rows of the global work copy) to ranked columns
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const int i = e / n, j = e % n;
-      Vb[i * n + rank[j]] = v[j * ldv + i];
-    }
-  }
-}
-
 __global__ void k_scale_cols_rsqrt(int n, int batch, const double* V, const double* W, double* T) {
   const int64_t total = int64_t(batch) * n * n;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
@@ -889,8 +832,6 @@ size_t small_smem_syev(int n, bool v_smem) {
   return mat * (v_smem ? 2 : 1) + jacobi_scratch_bytes(n) + (n + 4) * sizeof(int) + 64;
 }
 
-
-
 }  // namespace
 
 // Opts a kernel in to all the dynamic shared memory the device allows it (the
@@ -915,25 +856,6 @@ int set_smem(const Context* c, const void* fn, size_t bytes) {
 }
 
 int reduce_partials(const Context* c) { return c->num_sms * 2; }
-
-int launch_syev(Context* c, int n, int batch, const double* A, int64_t lda, int64_t a_bs, double* W, double* V,
-                int order) {
-  if (n < 1 || n > MCNLA_B200_MAX_DIM_SKETCH || batch < 1) return MCNLA_B200_ERR_UNSUPPORTED;
-  bool v_smem = small_smem_syev(n, true) <= c->smem_optin;
-  double* vwork = nullptr;
-  if (!v_smem) {
-    // global eigenvector work copies (one n x n per matrix); from the arena
-    vwork = ctx_take<double>(c, size_t(batch) * n * n);
-    if (!vwork) return MCNLA_B200_ERR_WORKSPACE;
-  }
-  const size_t smem = small_smem_syev(n, v_smem);
-  if (smem > c->smem_optin) return MCNLA_B200_ERR_UNSUPPORTED;
-  MB_CHECK(set_smem(c, reinterpret_cast<const void*>(k_syev), smem));
-  k_syev<<<batch, kSyevThreads, smem, c->stream>>>(n, A, lda, a_bs, W, V, order, v_smem ? 1 : 0, vwork);
-  c->kernels_launched++;
-  MB_CHECK_CUDA(cudaGetLastError());
-  return MCNLA_B200_OK;
-}
 
 int launch_scale_cols_rsqrt(Context* c, int n, int batch, const double* V, const double* W, double* T) {
   const int64_t total = int64_t(batch) * n * n;

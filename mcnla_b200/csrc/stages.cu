@@ -128,14 +128,16 @@ int run_orthogonalize(Context* c, const Dims& d, double* Q) {
   const size_t ll = size_t(l) * l;
   const size_t wsb = gemm_ws(c, {{l, l, m, N}, {m, l, l, N}});
   Plan pl;
-  pl.add(ll * N); pl.add(size_t(l) * N); pl.add(ll * N); pl.add(ll * N); pl.add(size_t(m) * L);
-  pl.add(wsb / 8 + 1); pl.add(ll * N);
+  // one buffer for the eigensolver's logs and then, where the rescale is not in place, the copy of Q
+  const size_t tmp_count = std::max(size_t(m) * L, syev_work_bytes(l, N) / 8 + 1);
+  pl.add(ll * N); pl.add(size_t(l) * N); pl.add(ll * N); pl.add(ll * N); pl.add(tmp_count);
+  pl.add(wsb / 8 + 1);
   MB_CHECK(ctx_reserve(c, pl.bytes));
   double* W = ctx_take<double>(c, ll * N);
   double* S = ctx_take<double>(c, size_t(l) * N);
   double* V = ctx_take<double>(c, ll * N);
   double* T = ctx_take<double>(c, ll * N);
-  double* tmp = ctx_take<double>(c, size_t(m) * L);
+  double* tmp = ctx_take<double>(c, tmp_count);
   double* ws = take_ws(c, wsb);
   MB_CHECK(check_arena(c));
   MB_CHECK(ctx_tic(c));
@@ -143,7 +145,7 @@ int run_orthogonalize(Context* c, const Dims& d, double* Q) {
   MB_CHECK(dgemm(c, l, l, m, 1.0, cm(Q, 1, L), cm(Q, L, 1), 0.0, drow(W, l), GemmBatch{N, l, l, int64_t(ll)}, ws));
   MB_CHECK(ctx_allreduce(c, W, int64_t(ll) * N));   // row blocks over ranks (row_block_gramian_orthogonalizer.hpp:86)
   // eig(W_i) = V_i S_i V_i', descending (gesvd<'N','O'> of an SPD matrix, :89-91)
-  MB_CHECK(launch_syev(c, l, N, W, l, int64_t(ll), S, V, 1));
+  MB_CHECK(launch_syev(c, l, N, W, l, int64_t(ll), S, V, 1, tmp));
   // T_i := V_i diag(S_i)^(-1/2)   (:94-99)
   MB_CHECK(launch_scale_cols_rsqrt(c, l, N, V, S, T));
   // Q_i := Q_i T_i in place: each CTA reads its rows of Q_i before it writes them (the reference
@@ -960,7 +962,8 @@ int run_form_svd(Context* c, const Dims& d, const CMat& Am, const double* Qbar, 
   pl.add(size_t(l) * n); pl.add(size_t(l) * n); pl.add(size_t(l) * n);
   for (int i = 0; i < 6; ++i) pl.add(ll);
   pl.add(size_t(2) * l); pl.add(wsb / 8 + 1);
-  for (int i = 0; i < 4; ++i) pl.add(ll);   // on-chip solver spill copies (l > 112)
+  pl.add(ll);   // the small SVD's spill copy (l > 112)
+  pl.add(syev_work_bytes(l, 1), 1);
   const size_t n16 = at ? form16_count(d) : 0, nsp = at ? form_split_doubles(c, d) : 0;
   pl.add(n16, sizeof(uint16_t)); pl.add(nsp);
   MB_CHECK(ctx_reserve(c, pl.bytes));
@@ -977,6 +980,7 @@ int run_form_svd(Context* c, const Dims& d, const CMat& Am, const double* Qbar, 
   double* Zm = ctx_take<double>(c, ll);
   double* w = ctx_take<double>(c, size_t(2) * l);
   double* sig = w + l;
+  char* eigw = ctx_take<char>(c, syev_work_bytes(l, 1));
   double* ws = take_ws(c, wsb);
   MB_CHECK(check_arena(c));
   MB_CHECK(ctx_tic(c));
@@ -990,7 +994,7 @@ int run_form_svd(Context* c, const Dims& d, const CMat& Am, const double* Qbar, 
   double* Yout[2] = {Y1, Y2};
   for (int pass = 0; pass < 2; ++pass) {
     MB_CHECK(dgemm(c, l, l, n, 1.0, crow(Yin, n), cm(Yin, 1, n), 0.0, drow(G, l), GemmBatch(), ws));
-    MB_CHECK(launch_syev(c, l, 1, G, l, 0, w, Ue, 1));
+    MB_CHECK(launch_syev(c, l, 1, G, l, 0, w, Ue, 1, eigw));
     MB_CHECK(launch_rsqrt_rows_t(c, l, Ue, w, P));
     MB_CHECK(dgemm(c, l, n, l, 1.0, crow(P, l), crow(Yin, n), 0.0, drow(Yout[pass], n), GemmBatch(), ws));
     Yin = Yout[pass];
@@ -1018,7 +1022,7 @@ int run_form_gramian(Context* c, const Dims& d, const CMat& Am, const double* Qb
   Plan pl;
   pl.add(size_t(n) * l); pl.add(ll); pl.add(ll); pl.add(ll); pl.add(size_t(2) * l);
   pl.add(wsb / 8 + 1);
-  for (int i = 0; i < 2; ++i) pl.add(ll);   // on-chip solver spill copy (l > 112)
+  pl.add(syev_work_bytes(l, 1), 1);
   const size_t n16 = at ? form16_count(d) : 0, nsp = at ? form_split_doubles(c, d) : 0;
   pl.add(n16, sizeof(uint16_t)); pl.add(nsp);
   MB_CHECK(ctx_reserve(c, pl.bytes));
@@ -1030,6 +1034,7 @@ int run_form_gramian(Context* c, const Dims& d, const CMat& Am, const double* Qb
   double* Wk = ctx_take<double>(c, ll);
   double* w = ctx_take<double>(c, size_t(2) * l);
   double* s = w + l;
+  char* eigw = ctx_take<char>(c, syev_work_bytes(l, 1));
   double* ws = take_ws(c, wsb);
   MB_CHECK(check_arena(c));
   MB_CHECK(ctx_tic(c));
@@ -1040,7 +1045,7 @@ int run_form_gramian(Context* c, const Dims& d, const CMat& Am, const double* Qb
   MB_CHECK(ctx_toc(c));
   // W := Z' Z; eig(W) = W S W' (descending); S := sqrt(S)   (:108-115)
   MB_CHECK(dgemm(c, l, l, n, 1.0, cm(Z, 1, l), crow(Z, l), 0.0, drow(W, l), GemmBatch(), ws));
-  MB_CHECK(launch_syev(c, l, 1, W, l, 0, w, Ue, 1));
+  MB_CHECK(launch_syev(c, l, 1, W, l, 0, w, Ue, 1, eigw));
   MB_CHECK(launch_sqrt_vec(c, l, w, s));
   MB_CHECK(ctx_toc(c));
   // U := Q W(:, 0:k); V := Z W(:, 0:k) diag(1/S)   (:123-128)
@@ -2120,8 +2125,9 @@ int mcnla_b200_syev_batched(mcnla_b200_ctx* ctx, int n, int batch, const double*
                             int order) {
   if (!ctx || !A || !W || !V || n < 1 || batch < 1 || (order != 0 && order != 1)) return MCNLA_B200_ERR_ARG;
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  MB_CHECK(mb::ctx_reserve(ctx, mb::arena_bytes_for(size_t(batch) * n * n, 8)));
-  return mb::launch_syev(ctx, n, batch, A, n, int64_t(n) * n, W, V, order);
+  const size_t work = mb::syev_work_bytes(n, batch);
+  MB_CHECK(mb::ctx_reserve(ctx, mb::arena_bytes_for(work, 1)));
+  return mb::launch_syev(ctx, n, batch, A, n, int64_t(n) * n, W, V, order, mb::ctx_take<char>(ctx, work));
 }
 
 }  // extern "C"

@@ -87,6 +87,38 @@ def test_syev_batched(cuda, n, batch):
             assert np.abs(vn[b].T @ vn[b] - np.eye(n)).max() <= 1e-13 * n
 
 
+@pytest.mark.parametrize("n,batch", [(3, 2), (4, 2), (5, 1), (6, 1), (7, 3), (31, 2), (33, 2), (63, 1), (65, 1), (95, 1),
+                                     (97, 2), (127, 1), (159, 1), (160, 90)])
+def test_syev_batched_sizes(cuda, n, batch):
+    """Odd and even sizes around the warps and pair counts of the Jacobi kernels, more matrices than one launch takes;
+    Gram matrices with a wide spectrum, a diagonal one, zero, and one with NaN (its neighbours are not touched)."""
+    from mcnla_b200 import isvd, _lib
+    import ctypes
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((batch, n, n)) * np.logspace(0, -3, n)[None, None, :]
+    a = x.transpose(0, 2, 1) @ x
+    if batch > 2:
+        a[0] = np.diag(rng.standard_normal(n))
+        a[1] = 0.0
+        a[2, n // 2, :] = a[2, :, n // 2] = np.nan
+    at = dev(a, cuda)
+    w = torch.empty(batch, n, dtype=torch.float64, device=cuda)
+    v = torch.empty(batch, n, n, dtype=torch.float64, device=cuda)
+    ctx = isvd.context()
+    _lib.check(ctx.lib.mcnla_b200_syev_batched(ctx.bind(), n, batch, ctypes.c_void_p(at.data_ptr()),
+                                               ctypes.c_void_p(w.data_ptr()), ctypes.c_void_p(v.data_ptr()), 1), "syev")
+    wn, vn = host(w), host(v)
+    for b in range(batch):
+        if batch > 2 and b == 2:
+            continue
+        lam = np.sort(np.abs(np.linalg.eigvalsh(a[b])))[::-1]
+        scale = max(lam[0], 1e-300)
+        assert np.abs(wn[b] - lam).max() <= 1e-13 * scale * n
+        lam_signed = np.diag(vn[b].T @ a[b] @ vn[b])
+        assert np.abs(a[b] @ vn[b] - vn[b] * lam_signed).max() <= 1e-12 * scale * n
+        assert np.abs(vn[b].T @ vn[b] - np.eye(n)).max() <= 1e-13 * n
+
+
 @pytest.mark.parametrize("n", [1, 5, 22, 128, 160])
 def test_inverse_batched(cuda, n):
     from mcnla_b200 import isvd, _lib
