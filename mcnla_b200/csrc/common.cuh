@@ -56,6 +56,7 @@ struct DevScalars {
   unsigned bar_count; // grid barrier of cooperative kernels: arrivals (only grows within a stage)
   unsigned bar_spare;
   int resume_it;      // persistent integrator: iteration it handed back to the host (-1: none)
+  int eig_needed;     // SVD former: 1 when the second Gram matrix is not close to the identity
   int kn_ns_failed;   // 1: the Newton-Schulz KN step with its matrices in global memory failed
   int wait_status;    // a bounded wait of the int8 GEMM ran out: kept (ctx_reset_scalars) until it is reported
 };

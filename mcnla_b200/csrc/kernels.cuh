@@ -10,10 +10,14 @@ namespace mb {
 // batch stride a_bs): eigenvalues to W (batch stride n), eigenvectors as the
 // columns of V (row-major n x n, batch stride n*n).  order 0: ascending;
 // order 1: descending by |lambda| with W = |lambda| (gesvd of a PSD matrix).
-// work: syev_work_bytes(n, batch) bytes of device memory, 256-byte aligned.
+// work: syev_work_bytes(n, batch) bytes of device memory, 256-byte aligned.  only_if: nothing happens when
+// *only_if is zero.
 int launch_syev(Context* c, int n, int batch, const double* A, int64_t lda, int64_t a_bs, double* W, double* V,
-                int order, void* work);
+                int order, void* work, const int* only_if = nullptr);
 size_t syev_work_bytes(int n, int batch);
+// The same by the solver whose roundings the mixed solves keep; vwork: batch n x n doubles.
+int launch_syev_square(Context* c, int n, int batch, const double* A, int64_t lda, int64_t a_bs, double* W, double* V,
+                       int order, double* vwork);
 
 // Scales the columns of V (row-major n x n, batch) by 1/sqrt(W): T = V diag(W^-1/2)
 // (the orthogonalizer's Q_i := Y_i V_i S_i^-1/2 step).
@@ -131,7 +135,11 @@ int launch_wy_gramian_phis(Context* c, int l, const double* F, const double* dc,
 int launch_svd_small(Context* c, int n, const double* M, double* W, double* sig, double* Z);
 // P := diag(w^-1/2) Ue' for the eigenpairs (w descending, Ue columns) of a
 // Gram matrix; rows whose w_i <= (n eps)^2 w_0 are set to zero.
-int launch_rsqrt_rows_t(Context* c, int n, const double* Ue, const double* w, double* P);
+int launch_rsqrt_rows_t(Context* c, int n, const double* Ue, const double* w, double* P, const int* only_if = nullptr);
+
+// P := G^(-1/2) for a Gram matrix G (n x n) close to the identity on the rows that P1 := launch_rsqrt_rows_t(., w)
+// kept, zero elsewhere; *needed := 0.  Not close (or not finite): *needed := 1, P is left alone.
+int launch_near_identity_rsqrt(Context* c, int n, const double* G, const double* w, double* P, int* needed);
 // Y(:, j) := X(:, j) * f(s_j) for j < cols; mode 0: f = 1/s, mode 1: f = s, mode 2: f = 1/sqrt(s).
 int launch_scale_cols(Context* c, int64_t rows, int64_t cols, const double* X, int64_t ldx, const double* s,
                       int mode, double* Y, int64_t ldy);

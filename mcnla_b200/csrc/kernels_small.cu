@@ -49,6 +49,66 @@ __device__ small::JacobiScratch carve_jacobi(SmemCarve& sc, int n) {
   return js;
 }
 
+// rank[j] = position of eigenvalue j in the requested order (ties by index).
+__device__ void eig_ranks(const double* a, int lda, int n, int order, int* rank) {
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const double dj = order ? fabs(a[j * lda + j]) : a[j * lda + j];
+    int r = 0;
+    for (int i = 0; i < n; ++i) {
+      const double di = order ? fabs(a[i * lda + i]) : a[i * lda + i];
+      const bool before = order ? (di > dj || (di == dj && i < j)) : (di < dj || (di == dj && i < j));
+      r += before ? 1 : 0;
+    }
+    rank[j] = r;
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// batched symmetric eigendecomposition of the mixed solves' orthogonalizer.  Their former reads
+// Qbar in BF16 parts, whose rounding (6e-8) is drawn anew when the sketches' bases move by 1e-10, as a
+// solver with other roundings (syev.cu) moves them: results would change by 1e-8.  So this one keeps
+// both triangles and its operation order, at 1.4-2.9 times the other's time.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kSyevThreads) k_syev_square(int n, const double* A, int64_t lda, int64_t a_bs,
+                                                        double* W, double* V, int order, int v_smem,
+                                                        double* vwork_all) {
+  extern __shared__ __align__(16) char smem_raw[];
+  SmemCarve sc(smem_raw);
+  const int ld = n + 1;
+  double* a = sc.take<double>(size_t(n) * ld);
+  double* v;
+  int ldv;
+  if (v_smem) { v = sc.take<double>(size_t(n) * ld); ldv = ld; }
+  else { v = vwork_all + size_t(blockIdx.x) * n * n; ldv = n; }
+  small::JacobiScratch js = carve_jacobi(sc, n);
+  int* rank = sc.take<int>(n);
+  const double* Ab = A + blockIdx.x * a_bs;
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) a[(e / n) * ld + (e % n)] = Ab[(e / n) * lda + (e % n)];
+  __syncthreads();
+  small::cta_jacobi_eig(a, ld, v, ldv, n, true, js, kMaxSweeps);
+  eig_ranks(a, ld, n, order, rank);
+  double* Wb = W + size_t(blockIdx.x) * n;
+  double* Vb = V + size_t(blockIdx.x) * n * n;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const double d = a[j * ld + j];
+    Wb[rank[j]] = order ? fabs(d) : d;
+  }
+  if (v_smem) {
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e / n, j = e % n;
+      Vb[i * n + rank[j]] = v[j * ldv + i];
+    }
+  } else {
+    __syncthreads();
+    // eigenvectors (rows of the global work copy) to ranked columns
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e / n, j = e % n;
+      Vb[i * n + rank[j]] = v[j * ldv + i];
+    }
+  }
+}
+
 __global__ void k_scale_cols_rsqrt(int n, int batch, const double* V, const double* W, double* T) {
   const int64_t total = int64_t(batch) * n * n;
   for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
@@ -507,12 +567,15 @@ __global__ void __launch_bounds__(small::kGjThreads) k_wy_trial(int l, const dou
 // ---------------------------------------------------------------------------
 // One-sided (Hestenes) Jacobi SVD of one n x n matrix: columns p, q of a are
 // rotated until all pairs are orthogonal; a = W diag(sig), and the rotations
-// accumulated in z give M = W diag(sig) Z'.  Per round: the angles of the
-// n/2 disjoint pairs (a warp per pair: column dot products by shuffles), then
-// the rotations of a's columns and of z spread over the CTA as (pair, row)
-// items.  z is kept transposed (z[k * ldz + i] = Z(i, k)) so that a rotation
-// touches two contiguous rows when it lives in global memory.
-__global__ void __launch_bounds__(kSmallThreads) k_svd_small(int n, const double* M, double* W, double* sig,
+// accumulated in z give M = W diag(sig) Z'.  A round's n/2 pairs are disjoint, so a
+// warp takes a pair alone: both columns in registers, the three dot products by
+// shuffles, the angle, and the rotation of the columns and of z's two rows (z is kept
+// transposed, z[k * ldz + i] = Z(i, k), so that these are contiguous); one barrier a round.
+// Latency-bound: with the angles and the rotations as two phases (two barriers) a solve of nearly orthogonal
+// columns took 1023 us at n = 96; now 680 us (with the roots and divisions of the textbook angle, 789 us).
+constexpr int kSvdRows = 5;   // rows a lane holds, n <= 160
+static_assert(MCNLA_B200_MAX_DIM_SKETCH <= 32 * kSvdRows, "a warp holds a column");
+__global__ void __launch_bounds__(kSyevThreads) k_svd_small(int n, const double* M, double* W, double* sig,
                                                              double* Z, double* zwork, int z_smem) {
   extern __shared__ __align__(16) char smem_raw[];
   SmemCarve sc(smem_raw);
@@ -522,14 +585,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_svd_small(int n, const double
   int ldz;
   if (z_smem) { z = sc.take<double>(size_t(n) * ld); ldz = ld; }
   else { z = zwork; ldz = n; }
-  int* count = sc.take<int>(4);
   int* rank = sc.take<int>(n);
   double* nrm = sc.take<double>(n);
   const int P = (n + 1) & ~1, npairs = P / 2;
-  double* rc = sc.take<double>(npairs);
-  double* rs = sc.take<double>(npairs);
-  int* rp = sc.take<int>(npairs);
-  int* rq = sc.take<int>(npairs);
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
   for (int e = tid; e < n * n; e += nt) {
@@ -538,61 +596,62 @@ __global__ void __launch_bounds__(kSmallThreads) k_svd_small(int n, const double
     z[i * ldz + j] = (i == j) ? 1.0 : 0.0;
   }
   __syncthreads();
-  const int items = npairs * n;
-  for (int sweep = 0; sweep < 40 && n > 1; ++sweep) {
-    int rotated = 0;
-    for (int r = 0; r < P - 1; ++r) {
-      // angles: a warp per pair
-      int mine = 0;
-      for (int k = warp; k < npairs; k += nwarps) {
-        int p, q;
-        small::rr_pair(P, r, k, p, q);
-        double c = 1.0, sn = 0.0;
-        if (q < n) {
-          double al = 0.0, be = 0.0, ga = 0.0;
-          for (int i = lane; i < n; i += 32) {
-            const double x = a[i * ld + p], y = a[i * ld + q];
-            al = fma(x, x, al);
-            be = fma(y, y, be);
-            ga = fma(x, y, ga);
-          }
-          for (int o = 16; o > 0; o >>= 1) {
-            al += __shfl_xor_sync(0xffffffffu, al, o);
-            be += __shfl_xor_sync(0xffffffffu, be, o);
-            ga += __shfl_xor_sync(0xffffffffu, ga, o);
-          }
-          if (fabs(ga) > 1e-15 * sqrt(al * be) && ga * ga > 1e-300) {
-            const double zeta = (be - al) / (2.0 * ga);
-            const double az = fabs(zeta);
-            const double t = (az > 1e150) ? 0.5 / zeta : ((zeta >= 0.0 ? 1.0 : -1.0) / (az + sqrt(1.0 + zeta * zeta)));
-            c = 1.0 / sqrt(1.0 + t * t);
-            sn = c * t;
-            if (lane == 0) ++mine;
-          }
-        }
-        if (lane == 0) { rc[k] = c; rs[k] = sn; rp[k] = p; rq[k] = q; }
+  int quiet = 0;                                  // rounds without a rotation, one after the other
+  for (int round = 0, r = 0; n > 1 && round < 40 * (P - 1) && quiet < P - 1; ++round, r = r + 1 == P - 1 ? 0 : r + 1) {
+    int mine = 0;
+    for (int k = warp; k < npairs; k += nwarps) {
+      int p, q;
+      small::rr_pair(P, r, k, p, q);
+      if (q >= n) continue;
+      double x[kSvdRows], y[kSvdRows];
+      double al = 0.0, be = 0.0, ga = 0.0;
+#pragma unroll
+      for (int u = 0; u < kSvdRows; ++u) {
+        const int i = lane + 32 * u;
+        x[u] = i < n ? a[i * ld + p] : 0.0;
+        y[u] = i < n ? a[i * ld + q] : 0.0;
       }
-      // the barrier also counts the rotations set up this round
-      const int cnt = __syncthreads_count(mine);
-      if (cnt == 0) continue;
-      rotated += cnt;
-      // rotations: (pair, row) items over the CTA
-      for (int e = tid; e < items; e += nt) {
-        const int k = e / n, i = e - k * n;
-        const double sn = rs[k];
-        if (sn == 0.0) continue;
-        const double c = rc[k];
-        const int p = rp[k], q = rq[k];
-        const double x = a[i * ld + p], y = a[i * ld + q];
-        a[i * ld + p] = c * x - sn * y;
-        a[i * ld + q] = sn * x + c * y;
+#pragma unroll
+      for (int u = 0; u < kSvdRows; ++u) {
+        al = fma(x[u], x[u], al);
+        be = fma(y[u], y[u], be);
+        ga = fma(x[u], y[u], ga);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        al += __shfl_xor_sync(0xffffffffu, al, o);
+        be += __shfl_xor_sync(0xffffffffu, be, o);
+        ga += __shfl_xor_sync(0xffffffffu, ga, o);
+      }
+      const double ga2 = ga * ga;
+      if (!(ga2 > 1e-30 * al * be && ga2 > 1e-300)) continue;   // the same on all lanes
+      // cos 2x = |d| / sqrt(d^2 + g^2): the angle by two reciprocal square roots (every lane computes it, and the
+      // FP64 pipe is what the pairs share); d and g far from 1 are scaled together, exactly
+      double d = be - al, g = 2.0 * ga;
+      const int e = max(__double2hiint(d) & 0x7ff00000, __double2hiint(g) & 0x7ff00000) >> 20;
+      const double scale = e > 1023 + 480 ? 0x1p-600 : (e < 1023 - 480 ? 0x1p600 : 1.0);
+      d *= scale;
+      g *= scale;
+      const double h = rsqrt(fma(d, d, g * g));
+      const double c2 = fma(0.5 * fabs(d), h, 0.5);
+      const double ic = rsqrt(c2);
+      double c = c2 * ic, sn = (d >= 0.0 ? 0.5 : -0.5) * g * h * ic;
+      const double f = 0.5 * fma(-sn, sn, fma(-c, c, 1.0));     // one step towards c^2 + s^2 = 1
+      c = fma(c, f, c);
+      sn = fma(sn, f, sn);
+      mine = 1;
+#pragma unroll
+      for (int u = 0; u < kSvdRows; ++u) {
+        const int i = lane + 32 * u;
+        if (i >= n) continue;
+        a[i * ld + p] = c * x[u] - sn * y[u];
+        a[i * ld + q] = sn * x[u] + c * y[u];
         const double zx = z[p * ldz + i], zy = z[q * ldz + i];
         z[p * ldz + i] = c * zx - sn * zy;
         z[q * ldz + i] = sn * zx + c * zy;
       }
-      __syncthreads();
     }
-    if (rotated == 0) break;
+    quiet = __syncthreads_or(mine) ? 0 : quiet + 1;
   }
   for (int j = warp; j < n; j += nwarps) {
     double s = 0.0;
@@ -616,12 +675,45 @@ __global__ void __launch_bounds__(kSmallThreads) k_svd_small(int n, const double
   }
 }
 
-__global__ void k_rsqrt_rows_t(int n, const double* Ue, const double* w, double* P) {
-  const double floor = (n * 2.220446049250313e-16) * (n * 2.220446049250313e-16) * fabs(w[0]);
+// Eigenvalues at or below this are taken as zero (an exactly rank-deficient Vt).
+__device__ __forceinline__ double rank_floor(int n, double w0) {
+  return (n * 2.220446049250313e-16) * (n * 2.220446049250313e-16) * fabs(w0);
+}
+
+__global__ void k_rsqrt_rows_t(int n, const double* Ue, const double* w, double* P, const int* only_if) {
+  if (only_if && *only_if == 0) return;
+  const double floor = rank_floor(n, w[0]);
   for (int e = threadIdx.x + blockIdx.x * blockDim.x; e < n * n; e += blockDim.x * gridDim.x) {
     const int i = e / n, j = e % n;
     const double wi = w[i];
     P[e] = (wi > floor && wi > 0.0) ? Ue[j * n + i] / sqrt(wi) : 0.0;
+  }
+}
+
+// P := (D + E)^(-1/2) = D - E/2 + 3/8 E^2 - ..., D the identity on the kept rows, E = G - D, where ||E||_F <= 1e-6:
+// the terms left out are below 0.32 ||E||^3 < 1e-18 (rows that are not kept are zero in G and stay so).
+// One CTA; E^2 is formed only where it can matter.
+__global__ void __launch_bounds__(kSyevThreads) k_near_identity_rsqrt(int n, const double* G, const double* w,
+                                                                      double* P, int* needed) {
+  __shared__ double red[32];
+  const double floor = rank_floor(n, w[0]);
+  auto entry = [&](int i, int j) { return G[i * n + j] - ((i == j && w[i] > floor && w[i] > 0.0) ? 1.0 : 0.0); };
+  double part = 0.0;
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    const double x = entry(e / n, e % n);
+    part = fma(x, x, part);
+  }
+  const double e2 = small::cta_sum(part, red);
+  const bool near = e2 <= 1e-12;                       // false for NaN
+  if (threadIdx.x == 0) *needed = near ? 0 : 1;
+  if (!near) return;
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    const int i = e / n, j = e % n;
+    const double d = (i == j && w[i] > floor && w[i] > 0.0) ? 1.0 : 0.0;
+    double q = 0.0;
+    if (e2 > 1e-18)
+      for (int k = 0; k < n; ++k) q = fma(entry(i, k), entry(k, j), q);
+    P[e] = fma(0.375, q, d - 0.5 * (G[e] - d));
   }
 }
 
@@ -857,6 +949,20 @@ int set_smem(const Context* c, const void* fn, size_t bytes) {
 
 int reduce_partials(const Context* c) { return c->num_sms * 2; }
 
+int launch_syev_square(Context* c, int n, int batch, const double* A, int64_t lda, int64_t a_bs, double* W,
+                       double* V, int order, double* vwork) {
+  if (n < 1 || n > MCNLA_B200_MAX_DIM_SKETCH || batch < 1) return MCNLA_B200_ERR_UNSUPPORTED;
+  bool v_smem = small_smem_syev(n, true) <= c->smem_optin;
+  if (!v_smem && !vwork) return MCNLA_B200_ERR_WORKSPACE;
+  const size_t smem = small_smem_syev(n, v_smem);
+  if (smem > c->smem_optin) return MCNLA_B200_ERR_UNSUPPORTED;
+  MB_CHECK(set_smem(c, reinterpret_cast<const void*>(k_syev_square), smem));
+  k_syev_square<<<batch, kSyevThreads, smem, c->stream>>>(n, A, lda, a_bs, W, V, order, v_smem ? 1 : 0, vwork);
+  c->kernels_launched++;
+  MB_CHECK_CUDA(cudaGetLastError());
+  return MCNLA_B200_OK;
+}
+
 int launch_scale_cols_rsqrt(Context* c, int n, int batch, const double* V, const double* W, double* T) {
   const int64_t total = int64_t(batch) * n * n;
   k_scale_cols_rsqrt<<<grid_for(c, total, 256), 256, 0, c->stream>>>(n, batch, V, W, T);
@@ -1007,22 +1113,28 @@ int launch_wy_gramian_phis(Context* c, int l, const double* F, const double* dc,
 int launch_svd_small(Context* c, int n, const double* M, double* W, double* sig, double* Z) {
   if (n < 1 || n > MCNLA_B200_MAX_DIM_SKETCH) return MCNLA_B200_ERR_UNSUPPORTED;
   const size_t mat = size_t(n) * (n + 1) * 8 + 16;
-  const int npairs = (n + 2) / 2;
-  const size_t extra = 64 + n * 4 + 16 + n * 8 + 16 + 2 * (npairs * 8 + 16) + 2 * (npairs * 4 + 16) + 64;
+  const size_t extra = n * 4 + 16 + n * 8 + 16 + 64;
   const bool z_smem = 2 * mat + extra <= c->smem_optin;
   const size_t smem = (z_smem ? 2 : 1) * mat + extra;
   if (smem > c->smem_optin) return MCNLA_B200_ERR_UNSUPPORTED;
   double* zwork = z_smem ? nullptr : ctx_take<double>(c, size_t(n) * n);
   if (!z_smem && !zwork) return MCNLA_B200_ERR_WORKSPACE;
   MB_CHECK(set_smem(c, reinterpret_cast<const void*>(k_svd_small), smem));
-  k_svd_small<<<1, kSmallThreads, smem, c->stream>>>(n, M, W, sig, Z, zwork, z_smem ? 1 : 0);
+  k_svd_small<<<1, kSyevThreads, smem, c->stream>>>(n, M, W, sig, Z, zwork, z_smem ? 1 : 0);
   c->kernels_launched++;
   MB_CHECK_CUDA(cudaGetLastError());
   return MCNLA_B200_OK;
 }
 
-int launch_rsqrt_rows_t(Context* c, int n, const double* Ue, const double* w, double* P) {
-  k_rsqrt_rows_t<<<grid_for(c, int64_t(n) * n, 256), 256, 0, c->stream>>>(n, Ue, w, P);
+int launch_near_identity_rsqrt(Context* c, int n, const double* G, const double* w, double* P, int* needed) {
+  k_near_identity_rsqrt<<<1, kSyevThreads, 0, c->stream>>>(n, G, w, P, needed);
+  c->kernels_launched++;
+  MB_CHECK_CUDA(cudaGetLastError());
+  return MCNLA_B200_OK;
+}
+
+int launch_rsqrt_rows_t(Context* c, int n, const double* Ue, const double* w, double* P, const int* only_if) {
+  k_rsqrt_rows_t<<<grid_for(c, int64_t(n) * n, 256), 256, 0, c->stream>>>(n, Ue, w, P, only_if);
   c->kernels_launched++;
   MB_CHECK_CUDA(cudaGetLastError());
   return MCNLA_B200_OK;

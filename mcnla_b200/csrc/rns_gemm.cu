@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(256) k_rns_cols(const double* __restrict__ B, 
     for (int j = 0; j < 4; ++j) u[j] = to_int(tile[i][4 * lane + j], s1, s2);
     uint8_t* dst = o.planes + row * o.kp + k0 + 4 * lane;
 #pragma unroll
-    for (int m = 0; m < kRnsModuli; ++m) *reinterpret_cast<uint32_t*>(dst + m * plane) = pack4(u, IS_B ? kT.b : kT.a, m);
+    for (int m = 0; m < kRnsModuli; ++m)
+      *reinterpret_cast<uint32_t*>(dst + m * plane) = pack4(u, IS_B ? kT.b : kT.a, m);
   }
 }
 
@@ -384,8 +385,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         for (int e = 0; e < 32; ++e) r[e] = rns::digit(int32_t(r[e]), kT, jb.p, with_inverse);
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-          w[e] = __byte_perm(__byte_perm(r[4 * e], r[4 * e + 1], 0x0040), __byte_perm(r[4 * e + 2], r[4 * e + 3], 0x0040),
-                             0x5410);
+          w[e] = __byte_perm(__byte_perm(r[4 * e], r[4 * e + 1], 0x0040),
+                             __byte_perm(r[4 * e + 2], r[4 * e + 3], 0x0040), 0x5410);
         uint4* d = reinterpret_cast<uint4*>(dst + c * 32);
         d[0] = make_uint4(w[0], w[1], w[2], w[3]);
         d[1] = make_uint4(w[4], w[5], w[6], w[7]);
@@ -521,7 +522,8 @@ RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, i
   const double m = double(M), n = double(N), k = double(K), half = same ? 0.5 : 1.0;
   const double n128 = double(cdiv(N, 128)) * 128.0;
   const double tiles = double(cdiv(M, kTileM)) * double(cdiv(N, kTileN));
-  const double computed = same ? 0.5 * (tiles + 2.0 * double(cdiv(N, kTileM))) : tiles;   // a triangle's diagonal tiles are whole
+  // a triangle's tiles on the diagonal are whole
+  const double computed = same ? 0.5 * (tiles + 2.0 * double(cdiv(N, kTileM))) : tiles;
   const double dmma = half * 2.0 * m * n128 * k / 31e6;
   const double int8 = 40.0 + (same ? 0.0 : 8.5e-6 * m * k) + 10e-6 * n * k + half * 12e-6 * m * n +
                       computed * double(kTileM) * kTileN * 2.0 * kRnsModuli * std::max(k, 1024.0) / 2.6e9;
@@ -551,7 +553,8 @@ RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, i
     }
   }
   // a plane's row index is a 32-bit tensor coordinate, a grid dimension at most 65535
-  if (kRnsModuli * b_pad > INT32_MAX / 2 || cdiv(N, kColTile) > 65535 || p.mb > 65535 || cdiv(K, kStatK) > 65535) return p;
+  if (kRnsModuli * b_pad > INT32_MAX / 2 || cdiv(N, kColTile) > 65535 || p.mb > 65535 || cdiv(K, kStatK) > 65535)
+    return p;
   p.bytes = layout(p, nullptr).bytes + 1024;
   p.use = true;
   return p;
@@ -618,7 +621,8 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
       g.M = int(rn);
       g.N = int(plan.N);
       g.status = &c->scal->wait_status;
-      rns_gemm_kernel<<<unsigned(std::min<int64_t>(g.jobs, c->num_sms)), kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
+      const unsigned ctas = unsigned(std::min<int64_t>(g.jobs, c->num_sms));
+      rns_gemm_kernel<<<ctas, kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
       MB_CHECK_CUDA(cudaGetLastError());
       k_rns_crt<<<dim3(unsigned(cdiv(plan.N, 1024)), unsigned(rn)), 256, 0, c->stream>>>(
           w.y, w.y_rows, w.ldy, rn, plan.N, w.ua + r0, w.ub, C.p + r0 * C.rs, C.rs, ch > 0,

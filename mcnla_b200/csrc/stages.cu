@@ -122,14 +122,15 @@ int run_sketch(Context* c, const Dims& d, const double* A, int layout, int64_t l
 // ---------------------------------------------------------------------------
 // Gramian orthogonalizer (gramian_orthogonalizer.hpp:62-104)
 // ---------------------------------------------------------------------------
-int run_orthogonalize(Context* c, const Dims& d, double* Q) {
+// mixed: for a mixed solve (see launch_syev_square).
+int run_orthogonalize(Context* c, const Dims& d, double* Q, bool mixed = false) {
   const int l = d.l, N = d.N;
   const int64_t m = d.m, L = d.L;
   const size_t ll = size_t(l) * l;
   const size_t wsb = gemm_ws(c, {{l, l, m, N}, {m, l, l, N}});
   Plan pl;
   // one buffer for the eigensolver's logs and then, where the rescale is not in place, the copy of Q
-  const size_t tmp_count = std::max(size_t(m) * L, syev_work_bytes(l, N) / 8 + 1);
+  const size_t tmp_count = std::max(size_t(m) * L, std::max(syev_work_bytes(l, N) / 8 + 1, ll * N));
   pl.add(ll * N); pl.add(size_t(l) * N); pl.add(ll * N); pl.add(ll * N); pl.add(tmp_count);
   pl.add(wsb / 8 + 1);
   MB_CHECK(ctx_reserve(c, pl.bytes));
@@ -145,7 +146,8 @@ int run_orthogonalize(Context* c, const Dims& d, double* Q) {
   MB_CHECK(dgemm(c, l, l, m, 1.0, cm(Q, 1, L), cm(Q, L, 1), 0.0, drow(W, l), GemmBatch{N, l, l, int64_t(ll)}, ws));
   MB_CHECK(ctx_allreduce(c, W, int64_t(ll) * N));   // row blocks over ranks (row_block_gramian_orthogonalizer.hpp:86)
   // eig(W_i) = V_i S_i V_i', descending (gesvd<'N','O'> of an SPD matrix, :89-91)
-  MB_CHECK(launch_syev(c, l, N, W, l, int64_t(ll), S, V, 1, tmp));
+  if (mixed) MB_CHECK(launch_syev_square(c, l, N, W, l, int64_t(ll), S, V, 1, tmp));
+  else MB_CHECK(launch_syev(c, l, N, W, l, int64_t(ll), S, V, 1, tmp));
   // T_i := V_i diag(S_i)^(-1/2)   (:94-99)
   MB_CHECK(launch_scale_cols_rsqrt(c, l, N, V, S, T));
   // Q_i := Q_i T_i in place: each CTA reads its rows of Q_i before it writes them (the reference
@@ -905,7 +907,7 @@ int run_integrate(Context* c, const Dims& d, int kind, const double* Qs, int max
 // ---------------------------------------------------------------------------
 // SvdFormer<_, true> (svd_former.hpp:70-116).  gesvd(Vt) is replaced by an
 // accuracy-preserving equivalent: two Gram re-orthonormalizations of the rows
-// of Vt give Y2 (orthonormal rows spanning the same space), M := Vt Y2' is
+// of Vt (the second by a series, see below) give Y2 (orthonormal rows spanning the same space), M := Vt Y2' is
 // formed by a GEMM, and M's SVD is taken by one-sided Jacobi:
 // Vt = M Y2 = W S (Y2' Z)'.
 // BF16 parts of A' (n x m, K-major: row j of A' is column j of A) for the
@@ -994,8 +996,20 @@ int run_form_svd(Context* c, const Dims& d, const CMat& Am, const double* Qbar, 
   double* Yout[2] = {Y1, Y2};
   for (int pass = 0; pass < 2; ++pass) {
     MB_CHECK(dgemm(c, l, l, n, 1.0, crow(Yin, n), cm(Yin, 1, n), 0.0, drow(G, l), GemmBatch(), ws));
-    MB_CHECK(launch_syev(c, l, 1, G, l, 0, w, Ue, 1, eigw));
-    MB_CHECK(launch_rsqrt_rows_t(c, l, Ue, w, P));
+    // The first pass leaves rows that are orthonormal to eps times the condition of G, so the second Gram matrix is the
+    // identity but for that (unless Vt is near rank deficiency): its inverse root by two terms of the series, and its
+    // eigendecomposition only where the series does not hold.  Besides the eigensolve (1.5 ms at l = 96) this keeps
+    // the order of the first pass's directions, so M's columns below are nearly orthogonal and the one-sided
+    // Jacobi method needs two or three sweeps instead of nine.
+    int* needed = nullptr;
+    double* wp = w;
+    if (pass == 1) {
+      needed = &c->scal->eig_needed;
+      wp = sig;                       // w has the first pass's eigenvalues
+      MB_CHECK(launch_near_identity_rsqrt(c, l, G, w, P, needed));
+    }
+    MB_CHECK(launch_syev(c, l, 1, G, l, 0, wp, Ue, 1, eigw, needed));
+    MB_CHECK(launch_rsqrt_rows_t(c, l, Ue, wp, P, needed));
     MB_CHECK(dgemm(c, l, n, l, 1.0, crow(P, l), crow(Yin, n), 0.0, drow(Yout[pass], n), GemmBatch(), ws));
     Yin = Yout[pass];
   }
@@ -1255,7 +1269,7 @@ int run_isvd_mixed(Context* c, const Dims& d, int integrator, int former, const 
   MB_CHECK(ctx_toc(c));
   MB_CHECK(bf16_gemm(c, d.m, d.L, d.n, a_hi, a_lo, a_lo2, lda16, omega_t, ldo, Q, d.L, true));
   MB_CHECK(ctx_toc(c));
-  MB_CHECK(run_orthogonalize(c, d, Q));
+  MB_CHECK(run_orthogonalize(c, d, Q, true));
   // The Gramian integrators' Bs (and the loop's Bs Bc) from BF16 parts (the
   // precision form) only where the FP64 product is long: below ~1e11 flops it
   // takes a few milliseconds at most, less than the split and the FP64
@@ -1277,7 +1291,7 @@ int run_isvd_mixed(Context* c, const Dims& d, int integrator, int former, const 
     Dims one = d;
     one.N = 1;
     one.L = d.l;
-    MB_CHECK(run_orthogonalize(c, one, Qbar));
+    MB_CHECK(run_orthogonalize(c, one, Qbar, true));
   }
   MB_CHECK(run_form(c, d, former, A, layout, lda, Qbar, S, U, V, at));
   MB_CHECK(ctx_sync_scalars(c));
@@ -1539,7 +1553,7 @@ int gitem_phase_a(Context* c, GItem& it, SolveScratch& s) {
     MB_CHECK(launch_gaussian_bf16(c, p.seed, d.n, d.L, it.omega_t, ldo, nullptr));
     MB_CHECK(bf16_gemm(c, d.m, d.L, d.n, part[0], part[1], part[2], ld16, it.omega_t, ldo, it.Q, d.L, true));
   }
-  MB_CHECK(run_orthogonalize(c, d, it.Q));
+  MB_CHECK(run_orthogonalize(c, d, it.Q, problem_mixed(p)));
   MB_CHECK(ctx_reset_scalars(c));
   const size_t wsb = gkn_ws_bytes(c, d);
   const RnsPlan plan = gkn_bs_plan(c, d);

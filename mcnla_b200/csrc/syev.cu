@@ -66,9 +66,9 @@ __device__ __forceinline__ Rotation rotation_of(double app, double aqq, double a
   Rotation r{1.0, 0.0, 0.0};
   const double apq2 = apq * apq;
   if (apq2 > eps2 * fabs(app * aqq) && apq2 > abs_floor) {
-    // d = aqq - app, g = 2 apq: cos 2x = |d| / sqrt(d^2 + g^2), c = sqrt((1 + cos 2x) / 2), s = sgn(d) sin 2x / (2 c) by
-    // two reciprocal square roots (the round's critical path), |x| <= pi / 4.  The matrix is scaled to entries of
-    // at most 1 and g is above the floor, so nothing overflows or underflows.
+    // d = aqq - app, g = 2 apq: cos 2x = |d| / sqrt(d^2 + g^2), c = sqrt((1 + cos 2x) / 2) and
+    // s = sgn(d) sin 2x / (2 c) by two reciprocal square roots (the round's critical path), |x| <= pi / 4.  The matrix
+    // is scaled to entries of at most 1 and g is above the floor, so nothing overflows or underflows.
     const double d = aqq - app, g = 2.0 * apq;
     const double h = rsqrt(fma(d, d, g * g));
     const double c2 = fma(0.5 * fabs(d), h, 0.5);
@@ -128,8 +128,9 @@ __device__ __forceinline__ Block rotate_block(const Block& b, double2 r1, double
 template <bool WITH_V>
 __global__ void __launch_bounds__(kJacThreads) k_jacobi_rotations(int n, const double* A, int64_t lda, int64_t a_bs,
                                                                  double* W, double* V, int order, char* work,
-                                                                 size_t per) {
+                                                                 size_t per, const int* only_if) {
   extern __shared__ __align__(16) double jac_smem[];
+  if (only_if && *only_if == 0) return;
   __shared__ double red[32];
   __shared__ int ex_s, rank_s[WITH_V ? kFusedMax : 1];
   const int np = jac_pairs(n), P = 2 * np, R = P - 1;      // an odd n gets a zero row and column
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(kJacThreads) k_jacobi_rotations(int n, const d
     items[u] = -1;
     const int t = tid - t0 + u * (nt - t0);
     if (tid < t0 || np < 3) continue;
-    const int f = t / np, j = t - f * np;                        // diagonals f + 1 and np - 1 - f: np - 1 - f and f + 1 blocks
+    const int f = t / np, j = t - f * np;   // diagonals f + 1 (np - 1 - f blocks) and np - 1 - f (f + 1)
     int D = f + 1, i = j;
     if (j >= np - 1 - f) {
       D = np - 1 - f;
@@ -358,11 +359,13 @@ __global__ void __launch_bounds__(kJacThreads) k_jacobi_rotations(int n, const d
 
 // V := the product of the logged rotations, columns ranked.  A CTA carries kVecCols components of every
 // eigenvector (32 components took 1545 instead of 1105 us on 16 matrices of n = 160); a half-warp applies a pair's
-// rotation to them, and the half-warps of a round meet at a barrier.  Bound by that chain of barriers and shared-memory round trips; the rounds' rotations come through
-// a ring of kVecRing rounds in shared memory.
+// rotation to them, and the half-warps of a round meet at a barrier.  Bound by that chain of barriers and
+// shared-memory round trips; the rounds' rotations come through a ring of kVecRing rounds in shared memory.
 constexpr int kVecRing = 8;
-__global__ void __launch_bounds__(kVecThreads) k_jacobi_vectors(int n, double* V, char* work, size_t per) {
+__global__ void __launch_bounds__(kVecThreads) k_jacobi_vectors(int n, double* V, char* work, size_t per,
+                                                                const int* only_if) {
   extern __shared__ __align__(16) double vec_smem[];
+  if (only_if && *only_if == 0) return;
   const int np = jac_pairs(n), P = 2 * np, R = P - 1;
   const int lane = threadIdx.x % kVecCols, h = threadIdx.x / kVecCols;
   constexpr int H = kVecGroups;
@@ -453,7 +456,7 @@ int jac_group(int n, int batch) {
 size_t syev_work_bytes(int n, int batch) { return n <= kFusedMax ? 0 : jac_bytes(n) * jac_group(n, batch); }
 
 int launch_syev(Context* c, int n, int batch, const double* A, int64_t lda, int64_t a_bs, double* W, double* V,
-                int order, void* work) {
+                int order, void* work, const int* only_if) {
   if (n < 1 || n > MCNLA_B200_MAX_DIM_SKETCH || batch < 1) return MCNLA_B200_ERR_UNSUPPORTED;
   const size_t smem = jac_smem_bytes(n);
   if (smem > c->smem_optin) return MCNLA_B200_ERR_UNSUPPORTED;
@@ -461,7 +464,8 @@ int launch_syev(Context* c, int n, int batch, const double* A, int64_t lda, int6
     // V in the same CTA: n = 12 (8 matrices) 56 us against 53 + 18 in two kernels, n = 32 (16) 256 against 188 + 69,
     // n = 64 (64) 919 against 497 + 318
     MB_CHECK(set_smem(c, reinterpret_cast<const void*>(k_jacobi_rotations<true>), smem));
-    k_jacobi_rotations<true><<<batch, jac_threads(n), smem, c->stream>>>(n, A, lda, a_bs, W, V, order, nullptr, 0);
+    k_jacobi_rotations<true><<<batch, jac_threads(n), smem, c->stream>>>(n, A, lda, a_bs, W, V, order, nullptr, 0,
+                                                                        only_if);
     MB_CHECK_CUDA(cudaGetLastError());
     c->kernels_launched++;
     return MCNLA_B200_OK;
@@ -473,11 +477,11 @@ int launch_syev(Context* c, int n, int batch, const double* A, int64_t lda, int6
   const size_t per = jac_bytes(n);
   for (int b0 = 0; b0 < batch; b0 += group) {
     const int m = std::min(group, batch - b0);
-    k_jacobi_rotations<false><<<m, jac_threads(n), smem, c->stream>>>(n, A + b0 * a_bs, lda, a_bs, W + size_t(b0) * n, V,
-                                                                   order, static_cast<char*>(work), per);
+    k_jacobi_rotations<false><<<m, jac_threads(n), smem, c->stream>>>(
+        n, A + b0 * a_bs, lda, a_bs, W + size_t(b0) * n, V, order, static_cast<char*>(work), per, only_if);
     MB_CHECK_CUDA(cudaGetLastError());
     k_jacobi_vectors<<<dim3(unsigned(cdiv(n, kVecCols)), unsigned(m)), kVecThreads, vsmem, c->stream>>>(
-        n, V + size_t(b0) * n * n, static_cast<char*>(work), per);
+        n, V + size_t(b0) * n * n, static_cast<char*>(work), per, only_if);
     MB_CHECK_CUDA(cudaGetLastError());
     c->kernels_launched += 2;
   }

@@ -647,3 +647,28 @@ def test_persistent_integrator_bits_do_not_depend_on_its_cta_share(cuda, l, N):
     for q in outs[1:]:
         assert torch.equal(q, outs[0])
     assert np.abs(host(outs[-1]) - qo).max() < TOL
+
+
+@pytest.mark.parametrize("l,k", [(5, 3), (33, 20), (64, 50), (96, 64), (160, 128)])
+@pytest.mark.parametrize("decay", [1.0, 4.5, 9.0])
+def test_svd_former_conditions(cuda, l, k, decay):
+    """The SVD former on Q'A with singular values from 1 down to 10^-decay: the second re-orthonormalization by the
+    series (mild decay) and by the eigendecomposition (steep), and l at the edges of the small SVD's tiles."""
+    from mcnla_b200 import isvd
+    m, n = 3 * l + 7, 2 * l + 5
+    rng = np.random.default_rng(l)
+    u = np.linalg.qr(rng.standard_normal((m, l)))[0]
+    v = np.linalg.qr(rng.standard_normal((n, l)))[0]
+    s = np.logspace(0, -decay, l)
+    a = (u * s) @ v.T
+    qbar = u @ np.linalg.qr(rng.standard_normal((l, l)))[0]
+    prm = isvd.Parameters().setSize(m, n).setRank(k).setOverRank(l - k).setNumSketch(1).sync()
+    st = isvd.SvdFormer(prm)
+    st.initialize()
+    st(dev(a, cuda), dev(qbar, cuda))
+    ref = np.linalg.svd(qbar.T @ a, compute_uv=False)[:k]
+    assert np.abs(host(st.vectorS()) - ref).max() <= 1e-13 * l
+    un, vn, sn = host(st.matrixU()), host(st.matrixV()), host(st.vectorS())
+    assert np.abs(un.T @ un - np.eye(k)).max() <= 1e-13 * l
+    # A V = U S on the kept directions, to rounding of A's norm
+    assert np.abs(a @ vn - un * sn).max() <= 1e-13 * l
