@@ -100,6 +100,9 @@ struct Context {
   bool tune_hot = false;
   // KN iteration loops replay one captured CUDA graph per chunk of iterations
   bool graph_loop = true;
+  // large products on the int8 tensor cores (rns.cuh, slice.cuh); off while a stage whose int8 workspace did not
+  // fit on the device runs again without
+  bool int8 = true;
   // precision form: the Gramian integrators form Bs = Qs' Qs from BF16 parts of Qs
   bool mixed_gramian = false;
   // row-block decomposition over several GPUs: the stages sum their row-dependent

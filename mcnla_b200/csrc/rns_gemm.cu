@@ -528,7 +528,7 @@ RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, i
   const double int8 = 40.0 + (same ? 0.0 : 8.5e-6 * m * k) + 10e-6 * n * k + half * 12e-6 * m * n +
                       computed * double(kTileM) * kTileN * 2.0 * kRnsModuli * std::max(k, 1024.0) / 2.6e9;
   if (int8 >= dmma) return p;
-  if (c && c->smem_optin < kGemmSmem) return p;
+  if (c && (!c->int8 || c->smem_optin < kGemmSmem)) return p;
   // B's planes within ~1.3 GB (a Gramian's, beside the integrator's state, 0.5 GB): K in chunks of equal size
   const int64_t b_pad = cdiv(N, kTileN) * kTileN;
   const int64_t b_most = int64_t(same ? 512 : 1300) << 20;

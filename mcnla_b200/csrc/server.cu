@@ -13,6 +13,7 @@
 // every kernel reduces in a fixed order.
 #include "common.cuh"
 #include "rns.cuh"
+#include "slice.cuh"
 #include "solve.cuh"
 
 #include <algorithm>
@@ -57,8 +58,11 @@ int64_t problem_bytes(const mcnla_b200_problem& p) {
   // leaves it unused), and a KN Gramian's beside its state
   const int64_t small = int64_t(64) << 20;
   stage = std::max(stage, int64_t(mb::plan_rns(nullptr, m, L, n, false).bytes) - small);
-  if (p.integrator == MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO)
-    stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + int64_t(mb::plan_rns(nullptr, L, L, m, true).bytes) - small);
+  if (p.integrator == MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO) {
+    const mb::SlicePlan sp = mb::plan_slices(nullptr, L, L, int(l));
+    stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + int64_t(sp.a_bytes + sp.w_bytes) +
+                                int64_t(mb::plan_rns(nullptr, L, L, m, true).bytes) - small);
+  }
   stage = std::max(stage, 4 * l * n * 8 + n * l * 8);                           // formers
   if (mixed) stage = std::max(stage, 3 * l * round8(m) * 2 + 16 * l * n * 8);   // precision former
   bytes += stage + small;                                                       // + split-K partials, small terms

@@ -13,6 +13,7 @@
 #include "kernels.cuh"
 #include "bf16.cuh"
 #include "rns.cuh"
+#include "slice.cuh"
 #include "solve.cuh"
 #include <algorithm>
 #include <array>
@@ -81,6 +82,16 @@ int copy2d(Context* c, double* dst, int64_t ldd, const double* src, int64_t lds,
   MB_CHECK_CUDA(cudaMemcpy2DAsync(dst, ldd * sizeof(double), src, lds * sizeof(double), cols * sizeof(double), rows,
                                   cudaMemcpyDeviceToDevice, c->stream));
   return MCNLA_B200_OK;
+}
+
+// Runs a stage, and once more without the int8 paths where their workspace did not fit on the device (a stage reserves
+// its workspace before anything else).
+template <class F>
+int with_int8_fallback(Context* c, F stage) {
+  const int st = stage();
+  if (st != MCNLA_B200_ERR_NOMEM || !c->int8) return st;
+  struct Off { Context* c; explicit Off(Context* x) : c(x) { c->int8 = false; } ~Off() { c->int8 = true; } } off(c);
+  return stage();
 }
 
 // ---------------------------------------------------------------------------
@@ -271,6 +282,48 @@ int kn_loop(Context* c, int maxit, Body body, int* iters) {
   return MCNLA_B200_OK;
 }
 
+// The products of an iteration loop with Qs and Qs', Qs cut into int8 slices once in each layout
+// (slice.cuh).  14 bytes an element of Qs next to its 8, so not in the server's workers (their memory is admitted
+// by an estimate without them), and not for a handful of iterations.
+struct QsProducts {
+  SlicePlan rows, cols;            // Qs B (K = L), Qs' X (K = m)
+  double *rows8 = nullptr, *cols8 = nullptr, *work = nullptr;
+  const double* Qs = nullptr;
+  int64_t m = 0, L = 0;
+  int l = 0;
+  double* ws = nullptr;
+
+  QsProducts(const Context* c, const Dims& d, int maxit, const double* q) : Qs(q), m(d.m), L(d.L), l(d.l) {
+    if (c->coop_cta_limit > 0 || maxit < 8) return;
+    rows = plan_slices(c, m, L, l);
+    cols = plan_slices(c, L, m, l);
+  }
+  void plan(Plan& pl) const {
+    pl.add(rows.a_bytes, 1); pl.add(cols.a_bytes, 1); pl.add(std::max(rows.w_bytes, cols.w_bytes), 1);
+  }
+  void take(Context* c, double* gemm_ws) {
+    rows8 = reinterpret_cast<double*>(ctx_take<char>(c, rows.a_bytes));
+    cols8 = reinterpret_cast<double*>(ctx_take<char>(c, cols.a_bytes));
+    work = reinterpret_cast<double*>(ctx_take<char>(c, std::max(rows.w_bytes, cols.w_bytes)));
+    ws = gemm_ws;
+  }
+  int prepare(Context* c) {
+    if (rows.use) MB_CHECK(slice_a(c, rows, crow(Qs, L), rows8));
+    if (cols.use) MB_CHECK(slice_a(c, cols, cm(Qs, 1, L), cols8));
+    return MCNLA_B200_OK;
+  }
+  // C (m x l) := alpha Qs B
+  int mul(Context* c, double alpha, const double* B, int64_t ldb, double* C, int64_t ldc) const {
+    if (rows.use) return slice_mul(c, rows, rows8, crow(B, ldb), alpha, drow(C, ldc), work);
+    return dgemm(c, m, l, L, alpha, crow(Qs, L), crow(B, ldb), 0.0, drow(C, ldc), GemmBatch(), ws);
+  }
+  // C (L x l) := Qs' X
+  int mul_t(Context* c, const double* X, int64_t ldx, double* C, int64_t ldc) const {
+    if (cols.use) return slice_mul(c, cols, cols8, crow(X, ldx), 1.0, drow(C, ldc), work);
+    return dgemm(c, L, l, m, 1.0, cm(Qs, 1, L), crow(X, ldx), 0.0, drow(C, ldc), GemmBatch(), ws);
+  }
+};
+
 // KolmogorovNagumoIntegrator (kolmogorov_nagumo_integrator.hpp:76-185)
 int run_kn(Context* c, const Dims& d, const double* Qs, int maxit, double tol, double* Qbar, int* iters) {
   const int l = d.l;
@@ -280,6 +333,8 @@ int run_kn(Context* c, const Dims& d, const double* Qs, int maxit, double tol, d
   Plan pl;
   pl.add(size_t(m) * 2 * l); pl.add(size_t(m) * 2 * l); pl.add(size_t(L) * l); pl.add(size_t(l) * l);
   pl.add(size_t(l) * l); pl.add(size_t(2) * l * l); pl.add(kn_series_work_doubles(l)); pl.add(wsb / 8 + 1);
+  QsProducts qs(c, d, maxit, Qs);
+  qs.plan(pl);
   MB_CHECK(ctx_reserve(c, pl.bytes));
   double* QX[2] = {ctx_take<double>(c, size_t(m) * 2 * l), ctx_take<double>(c, size_t(m) * 2 * l)};
   double* B = ctx_take<double>(c, size_t(L) * l);
@@ -288,11 +343,13 @@ int run_kn(Context* c, const Dims& d, const double* Qs, int maxit, double tol, d
   double* CC = ctx_take<double>(c, size_t(2) * l * l);
   double* vwork = ctx_take<double>(c, kn_series_work_doubles(l));
   double* ws = take_ws(c, wsb);
+  qs.take(c, ws);
   MB_CHECK(check_arena(c));
   const int64_t lq = 2 * l;
   MB_CHECK(ctx_tic(c));
   // Qc := Q0   (:105)
   MB_CHECK(copy2d(c, QX[0], lq, Qs, L, m, l));
+  MB_CHECK(qs.prepare(c));
   MB_CHECK(ctx_toc(c));
   int it = 0;
   MB_CHECK(kn_loop(c, maxit, [&](int i) -> int {
@@ -300,12 +357,12 @@ int run_kn(Context* c, const Dims& d, const double* Qs, int maxit, double tol, d
     double* Qc = QX[cur];
     double* X = QX[cur] + l;
     // B := Qs' Qc   (:117)
-    MB_CHECK(dgemm(c, L, l, m, 1.0, cm(Qs, 1, L), crow(Qc, lq), 0.0, drow(B, l), GemmBatch(), ws));
+    MB_CHECK(qs.mul_t(c, Qc, lq, B, l));
     MB_CHECK(ctx_allreduce(c, B, L * l));   // row blocks over ranks
     // D := B' B   (:123)
     MB_CHECK(dgemm(c, l, l, L, 1.0, cm(B, 1, l), crow(B, l), 0.0, drow(D, l), GemmBatch(), ws));
     // X := Qs B / N;  X -= Qc D / N   (:126-129)
-    MB_CHECK(dgemm(c, m, l, L, inv_n, crow(Qs, L), crow(B, l), 0.0, drow(X, lq), GemmBatch(), ws));
+    MB_CHECK(qs.mul(c, inv_n, B, l, X, lq));
     MB_CHECK(dgemm(c, m, l, l, -inv_n, crow(Qc, lq), crow(D, l), 1.0, drow(X, lq), GemmBatch(), ws));
     // Z := X' X   (:143)
     MB_CHECK(dgemm(c, l, l, m, 1.0, cm(X, 1, lq), crow(X, lq), 0.0, drow(Z, l), GemmBatch(), ws));
@@ -332,6 +389,8 @@ int run_rb_kn(Context* c, const Dims& d, const double* Qs, int maxit, double tol
   Plan pl;
   for (int i = 0; i < 2; ++i) { pl.add(size_t(m) * 2 * l); pl.add(size_t(L) * 2 * l); }
   pl.add(size_t(2) * l * l); pl.add(size_t(2) * l * l); pl.add(kn_series_work_doubles(l)); pl.add(wsb / 8 + 1);
+  QsProducts qs(c, d, maxit, Qs);
+  qs.plan(pl);
   MB_CHECK(ctx_reserve(c, pl.bytes));
   double* QG[2] = {ctx_take<double>(c, size_t(m) * 2 * l), ctx_take<double>(c, size_t(m) * 2 * l)};
   double* BB[2] = {ctx_take<double>(c, size_t(L) * 2 * l), ctx_take<double>(c, size_t(L) * 2 * l)};
@@ -339,21 +398,23 @@ int run_rb_kn(Context* c, const Dims& d, const double* Qs, int maxit, double tol
   double* FC = ctx_take<double>(c, size_t(2) * l * l);
   double* vwork = ctx_take<double>(c, kn_series_work_doubles(l));
   double* ws = take_ws(c, wsb);
+  qs.take(c, ws);
   MB_CHECK(check_arena(c));
   const int64_t l2 = 2 * l;
   MB_CHECK(ctx_tic(c));
   // Qc := Q0; Bc := Qs' Qc   (:110-113)
   MB_CHECK(copy2d(c, QG[0], l2, Qs, L, m, l));
-  MB_CHECK(dgemm(c, L, l, m, 1.0, cm(Qs, 1, L), crow(QG[0], l2), 0.0, drow(BB[0], l2), GemmBatch(), ws));
+  MB_CHECK(qs.prepare(c));
+  MB_CHECK(qs.mul_t(c, QG[0], l2, BB[0], l2));
   MB_CHECK(ctx_allreduce2d(c, BB[0], l2, L, l));   // (:115)
   MB_CHECK(ctx_toc(c));
   int it = 0;
   MB_CHECK(kn_loop(c, maxit, [&](int i) -> int {
     const int cur = i & 1;
     // Gc := 1/N Qs Bc   (:138)
-    MB_CHECK(dgemm(c, m, l, L, inv_n, crow(Qs, L), crow(BB[cur], l2), 0.0, drow(QG[cur] + l, l2), GemmBatch(), ws));
+    MB_CHECK(qs.mul(c, inv_n, BB[cur], l2, QG[cur] + l, l2));
     // Bgc := Qs' Gc   (:141)
-    MB_CHECK(dgemm(c, L, l, m, 1.0, cm(Qs, 1, L), crow(QG[cur] + l, l2), 0.0, drow(BB[cur] + l, l2), GemmBatch(), ws));
+    MB_CHECK(qs.mul_t(c, QG[cur] + l, l2, BB[cur] + l, l2));
     MB_CHECK(ctx_allreduce2d(c, BB[cur] + l, l2, L, l));   // (:143)
     // [Dc | Dgc] := 1/N Bc' [Bc | Bgc]   (:147-150)
     MB_CHECK(dgemm(c, l, l2, L, inv_n, cm(BB[cur], 1, l2), crow(BB[cur], l2), 0.0, drow(DD, l2), GemmBatch(), ws));
@@ -416,7 +477,7 @@ struct GknBufs {
   uint16_t* bs16 = nullptr;   // precision form: BF16 parts of Qs', of Bs and of Bc', split-K slices
   uint16_t* bsp = nullptr;
   uint16_t* bcp = nullptr;
-  double* slices = nullptr;
+  double* bgc_slices = nullptr;
   double* Bs = nullptr;       // L x L
   double* EB[2] = {nullptr, nullptr};   // [E~ | Bc | Bgc] (L x 3l), current / next
   double* DD = nullptr;       // [Dc | Dgc] (l x 2l)
@@ -430,6 +491,9 @@ struct GknBufs {
   double* job = nullptr;      // device GknJob and work-queue counter (the grouped kernel's single-job use)
   Bf16Split spb;
   bool bf16_bgc = false;
+  SlicePlan slices;           // Bs Bc on the int8 tensor cores: Bs' slices, and Bc's with the partial sums
+  double* bs8 = nullptr;
+  double* bc8 = nullptr;
 };
 
 // Qbar := Q0 F~ + Qs E~ = Qs (E~ + [F~; 0])
@@ -458,6 +522,11 @@ RnsPlan gkn_bs_plan(const Context* c, const Dims& d) {
   return c->mixed_gramian ? RnsPlan() : plan_rns(c, d.L, d.L, d.m, true);
 }
 
+// The int8 plan of the loop's Bs Bc.
+SlicePlan gkn_loop_plan(const Context* c, const Dims& d) {
+  return c->mixed_gramian ? SlicePlan() : plan_slices(c, d.L, d.L, d.l);
+}
+
 // Visits the buffers in carve order: fn(count, element bytes).
 template <class Fn>
 void gkn_layout(const Context* c, const Dims& d, Fn fn, Bf16Split* spb_out = nullptr) {
@@ -479,6 +548,8 @@ void gkn_layout(const Context* c, const Dims& d, Fn fn, Bf16Split* spb_out = nul
   fn(size_t(l2) * l, 8); fn(size_t(l2) * l, 8); fn(size_t(l) * l, 8); fn(size_t(l) * l, 8);
   fn(size_t(L) * l, 8); fn(kn_series_work_doubles(int(l)), 8); fn(size_t(l) * l, 8);
   fn(gkn_grouped_ddp_doubles(int(l), L), 8); fn((sizeof(GknJob) + 64) / 8, 8);
+  const SlicePlan sp = gkn_loop_plan(c, d);
+  fn((sp.a_bytes + 7) / 8, 8); fn((sp.w_bytes + 7) / 8, 8);
 }
 
 size_t gkn_state_bytes(const Context* c, const Dims& d) {
@@ -490,14 +561,14 @@ size_t gkn_state_bytes(const Context* c, const Dims& d) {
 // Carves the buffers with take(count, elem) (returns char*, null past the end).
 template <class Take>
 void gkn_carve(const Context* c, const Dims& d, Take take, GknBufs& b) {
-  char* p[17];
+  char* p[19];
   int i = 0;
   gkn_layout(c, d, [&](size_t count, size_t elem) { p[i++] = take(count, elem); }, &b.spb);
   b.bf16_bgc = c->mixed_gramian;
   b.bs16 = reinterpret_cast<uint16_t*>(p[0]);
   b.bsp = reinterpret_cast<uint16_t*>(p[1]);
   b.bcp = reinterpret_cast<uint16_t*>(p[2]);
-  b.slices = reinterpret_cast<double*>(p[3]);
+  b.bgc_slices = reinterpret_cast<double*>(p[3]);
   b.Bs = reinterpret_cast<double*>(p[4]);
   b.EB[0] = reinterpret_cast<double*>(p[5]);
   b.EB[1] = reinterpret_cast<double*>(p[6]);
@@ -511,6 +582,9 @@ void gkn_carve(const Context* c, const Dims& d, Take take, GknBufs& b) {
   b.cbuf = reinterpret_cast<double*>(p[14]);
   b.ddp = reinterpret_cast<double*>(p[15]);
   b.job = reinterpret_cast<double*>(p[16]);
+  b.slices = gkn_loop_plan(c, d);
+  b.bs8 = reinterpret_cast<double*>(p[17]);
+  b.bc8 = reinterpret_cast<double*>(p[18]);
 }
 
 // Cluster size of the grouped kernel for a problem: about three 64-row units
@@ -554,6 +628,7 @@ int gkn_prepare(Context* c, const Dims& d, const double* Qs, const GknBufs& b, d
   MB_CHECK(gramian_bs(c, d, Qs, b.Bs, b.EB[0] + l, l3, ws, b.bs16, plan, wr));
   MB_CHECK(launch_fill(c, L, l, 0.0, b.EB[0], l3));
   MB_CHECK(launch_set_identity(c, l, b.FF[0], l));
+  if (b.slices.use) MB_CHECK(slice_a(c, b.slices, crow(b.Bs, L), b.bs8));
   const int64_t ldL = (L + 7) & ~int64_t(7);
   const size_t bpart = size_t(L) * ldL;
   if (b.bf16_bgc)
@@ -577,10 +652,12 @@ int gkn_iteration(Context* c, const Dims& d, const GknBufs& b, int i, bool allow
     const int64_t ldL = (L + 7) & ~int64_t(7);
     const size_t bpart = size_t(L) * ldL, cpart = size_t(l) * ldL;
     MB_CHECK(launch_split_bf16(c, Bc, MCNLA_B200_COL_MAJOR, l3, l, L, b.bcp, b.bcp + cpart, b.bcp + 2 * cpart, ldL));
-    MB_CHECK(bf16_gemm_split(c, L, 3 * l, L, b.bsp, b.bsp + bpart, b.bsp + 2 * bpart, ldL, b.bcp, ldL, b.slices,
+    MB_CHECK(bf16_gemm_split(c, L, 3 * l, L, b.bsp, b.bsp + bpart, b.bsp + 2 * bpart, ldL, b.bcp, ldL, b.bgc_slices,
                              3 * l, true, false, false, b.spb));
-    MB_CHECK(launch_sum_splits(c, b.slices, b.spb.splits, b.spb.split_stride, L, l, 3 * l, Bgc, l3, false, inv_n, 3,
+    MB_CHECK(launch_sum_splits(c, b.bgc_slices, b.spb.splits, b.spb.split_stride, L, l, 3 * l, Bgc, l3, false, inv_n, 3,
                                l));
+  } else if (b.slices.use) {
+    MB_CHECK(slice_mul(c, b.slices, b.bs8, crow(Bc, l3), inv_n, drow(Bgc, l3), b.bc8));
   } else {
     MB_CHECK(dgemm(c, L, l, L, inv_n, crow(b.Bs, L), crow(Bc, l3), 0.0, drow(Bgc, l3), GemmBatch(), ws));
   }
@@ -892,14 +969,16 @@ int run_integrate(Context* c, const Dims& d, int kind, const double* Qs, int max
   if (maxit < 0 || !(tol >= 0.0)) return MCNLA_B200_ERR_ARG;
   // device status, convergence scalars and grid-barrier counters start clean
   MB_CHECK(ctx_reset_scalars(c));
-  switch (kind) {
-    case MCNLA_B200_KOLMOGOROV_NAGUMO: return run_kn(c, d, Qs, maxit, tol, Qbar, iters);
-    case MCNLA_B200_ROW_BLOCK_KOLMOGOROV_NAGUMO: return run_rb_kn(c, d, Qs, maxit, tol, Qbar, iters);
-    case MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO: return run_rb_gramian_kn(c, d, Qs, maxit, tol, Qbar, iters);
-    case MCNLA_B200_ROW_BLOCK_WEN_YIN: return run_rb_wy(c, d, Qs, maxit, tol, Qbar, iters);
-    case MCNLA_B200_ROW_BLOCK_GRAMIAN_WEN_YIN: return run_rb_gramian_wy(c, d, Qs, maxit, tol, Qbar, iters);
-    default: return MCNLA_B200_ERR_ARG;
-  }
+  return with_int8_fallback(c, [&]() -> int {
+    switch (kind) {
+      case MCNLA_B200_KOLMOGOROV_NAGUMO: return run_kn(c, d, Qs, maxit, tol, Qbar, iters);
+      case MCNLA_B200_ROW_BLOCK_KOLMOGOROV_NAGUMO: return run_rb_kn(c, d, Qs, maxit, tol, Qbar, iters);
+      case MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO: return run_rb_gramian_kn(c, d, Qs, maxit, tol, Qbar, iters);
+      case MCNLA_B200_ROW_BLOCK_WEN_YIN: return run_rb_wy(c, d, Qs, maxit, tol, Qbar, iters);
+      case MCNLA_B200_ROW_BLOCK_GRAMIAN_WEN_YIN: return run_rb_gramian_wy(c, d, Qs, maxit, tol, Qbar, iters);
+      default: return MCNLA_B200_ERR_ARG;
+    }
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -1107,7 +1186,7 @@ int run_isvd(Context* c, const Dims& d, int integrator, int former, const double
   } else {
     omega = const_cast<double*>(omega_in);   // read only: the sketch runs without power iterations
   }
-  MB_CHECK(run_sketch(c, d, A, layout, lda, omega, 0, Q, false));
+  MB_CHECK(with_int8_fallback(c, [&] { return run_sketch(c, d, A, layout, lda, omega, 0, Q, false); }));
   MB_CHECK(run_orthogonalize(c, d, Q));
   MB_CHECK(run_integrate(c, d, integrator, Q, maxit, tol, Qbar, iters));
   MB_CHECK(run_form(c, d, former, A, layout, lda, Qbar, S, U, V));
@@ -1543,7 +1622,7 @@ int gitem_phase_a(Context* c, GItem& it, SolveScratch& s) {
     int64_t lda = 0;
     MB_CHECK(problem_a64(c, p, s, &A, &lda));
     MB_CHECK(launch_gaussian(c, p.seed, int64_t(d.n) * d.L, it.omega));
-    MB_CHECK(run_sketch(c, d, A, p.a_layout, lda, it.omega, 0, it.Q, false));
+    MB_CHECK(with_int8_fallback(c, [&] { return run_sketch(c, d, A, p.a_layout, lda, it.omega, 0, it.Q, false); }));
   } else {
     const uint16_t* part[3];
     int64_t ld16 = 0;
@@ -1556,8 +1635,13 @@ int gitem_phase_a(Context* c, GItem& it, SolveScratch& s) {
   MB_CHECK(run_orthogonalize(c, d, it.Q, problem_mixed(p)));
   MB_CHECK(ctx_reset_scalars(c));
   const size_t wsb = gkn_ws_bytes(c, d);
-  const RnsPlan plan = gkn_bs_plan(c, d);
-  MB_CHECK(ctx_reserve(c, arena_bytes_for(wsb + 8, 1) + arena_bytes_for(plan.bytes, 1)));
+  RnsPlan plan = gkn_bs_plan(c, d);
+  int st = ctx_reserve(c, arena_bytes_for(wsb + 8, 1) + arena_bytes_for(plan.bytes, 1));
+  if (st == MCNLA_B200_ERR_NOMEM && plan.use) {
+    plan = RnsPlan();
+    st = ctx_reserve(c, arena_bytes_for(wsb + 8, 1) + arena_bytes_for(0, 1));
+  }
+  MB_CHECK(st);
   double* ws = take_ws(c, wsb);
   char* wr = ctx_take<char>(c, plan.bytes);
   MB_CHECK(check_arena(c));
@@ -1877,8 +1961,7 @@ int mcnla_b200_initialize(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, 
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  MB_CHECK(mb::ctx_reserve(ctx, mb::stage_bytes_upper(ctx, d)));
-  return MCNLA_B200_OK;
+  return mb::with_int8_fallback(ctx, [&] { return mb::ctx_reserve(ctx, mb::stage_bytes_upper(ctx, d)); });
 }
 
 int mcnla_b200_sketch(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, const double* A, int a_layout,
@@ -1887,7 +1970,7 @@ int mcnla_b200_sketch(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, cons
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  return mb::run_sketch(ctx, d, A, a_layout, lda, omega, exponent, Q, false);
+  return mb::with_int8_fallback(ctx, [&] { return mb::run_sketch(ctx, d, A, a_layout, lda, omega, exponent, Q, false); });
 }
 
 int mcnla_b200_gaussian(mcnla_b200_ctx* ctx, uint64_t seed, int64_t count, double* out) {
@@ -1963,7 +2046,8 @@ int mcnla_b200_isvd_host(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, i
   const int64_t lda = a_layout == MCNLA_B200_ROW_MAJOR ? d.n : d.m;
   if (a_layout == MCNLA_B200_ROW_MAJOR && a_elems * sizeof(double) >= (size_t(64) << 20)) {
     // large row-major A: copied in row blocks behind the sketch
-    MB_CHECK(mb::run_sketch_streamed(ctx, d, A_host, A, omega_host, omega_dev, Q));
+    MB_CHECK(mb::with_int8_fallback(
+        ctx, [&] { return mb::run_sketch_streamed(ctx, d, A_host, A, omega_host, omega_dev, Q); }));
     MB_CHECK(mb::run_orthogonalize(ctx, d, Q));
     MB_CHECK(mb::run_integrate(ctx, d, integrator, Q, max_iteration, tolerance, Qbar, iteration));
     MB_CHECK(mb::run_form(ctx, d, former, A, a_layout, lda, Qbar, S, U, V));
@@ -2008,7 +2092,8 @@ int mcnla_b200_isvd_stream(mcnla_b200_ctx* ctx, const mcnla_b200_params* params,
   double* omega_dev = reinterpret_cast<double*>(base + mb::arena_bytes_for(size_t(d.m) * d.L, 8) +
                                                 mb::arena_bytes_for(size_t(d.m) * d.l, 8));
   MB_CHECK(mb::ctx_reset_scalars(ctx));
-  MB_CHECK(mb::run_sketch_ingest(ctx, d, read_rows, user, A, omega_host, omega_dev, Q));
+  MB_CHECK(mb::with_int8_fallback(
+      ctx, [&] { return mb::run_sketch_ingest(ctx, d, read_rows, user, A, omega_host, omega_dev, Q); }));
   MB_CHECK(mb::run_orthogonalize(ctx, d, Q));
   MB_CHECK(mb::run_integrate(ctx, d, integrator, Q, max_iteration, tolerance, Qbar, iteration));
   MB_CHECK(mb::run_form(ctx, d, former, A, MCNLA_B200_ROW_MAJOR, d.n, Qbar, S, U, V));

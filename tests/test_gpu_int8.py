@@ -82,7 +82,8 @@ def test_rows_and_columns_left_to_the_fp64_units(cuda):
     ref = a @ omega
     assert torch.equal(torch.isnan(q), torch.isnan(ref))
     fin = torch.isfinite(ref)
-    assert torch.equal(fin, torch.isfinite(q)) and torch.equal(q[~fin & ~torch.isnan(ref)], ref[~fin & ~torch.isnan(ref)])
+    inf = ~fin & ~torch.isnan(ref)
+    assert torch.equal(fin, torch.isfinite(q)) and torch.equal(q[inf], ref[inf])
     assert torch.equal(q[304][fin[304]], 2.0 * omega[9][fin[304]])
     assert torch.equal(q[:, 503][fin[:, 503]], a[:, 30][fin[:, 503]])
     assert (q[301][fin[301]] == 0).all() and (q[:, 502][fin[:, 502]] == 0).all()
@@ -133,3 +134,70 @@ def test_gramian(cuda):
         out.append((qbar, st.iteration()))
     assert out[0][1] == out[1][1]
     assert float((out[0][0] - out[1][0]).abs().max()) < 1e-12
+
+
+def _bases(cuda, m, l, N, seed):
+    g = torch.Generator(device=cuda)
+    g.manual_seed(seed)
+    base = torch.linalg.qr(torch.randn(m, l, generator=g, dtype=torch.float64, device=cuda))[0]
+    noise = torch.randn(N, m, l, generator=g, dtype=torch.float64, device=cuda) / m ** 0.5
+    return torch.linalg.qr(base[None] + 0.3 * noise)[0].permute(1, 0, 2).reshape(m, -1).contiguous()
+
+
+def _kn(q, l, N, maxit, tol):
+    """The Kolmogorov-Nagumo average by its definition, in FP64."""
+    qc = q[:, :l].clone()
+    for it in range(1, maxit + 1):
+        b = q.T @ qc
+        x = (q @ b - qc @ (b.T @ b)) / N
+        lam, vec = torch.linalg.eigh(x.T @ x)
+        e = torch.sqrt(0.5 + torch.sqrt(0.25 - lam))
+        qc = qc @ ((vec * e) @ vec.T) + x @ ((vec / e) @ vec.T)
+        if not float(torch.linalg.norm(e - 1)) >= tol:
+            break
+    return qc, it
+
+
+@pytest.mark.parametrize("cls,m,k,p,N", [
+    ("KolmogorovNagumoIntegrator", 8192, 20, 11, 33), ("KolmogorovNagumoIntegrator", 12001, 20, 12, 24),
+    ("KolmogorovNagumoIntegrator", 20000, 20, 13, 13), ("RowBlockKolmogorovNagumoIntegrator", 8001, 50, 14, 16),
+    ("RowBlockKolmogorovNagumoIntegrator", 8193, 50, 15, 16), ("RowBlockKolmogorovNagumoIntegrator", 20000, 3, 2, 129),
+    ("RowBlockKolmogorovNagumoIntegrator", 6000, 128, 32, 10),
+    ("RowBlockGramianKolmogorovNagumoIntegrator", 3001, 50, 14, 45),
+    ("RowBlockGramianKolmogorovNagumoIntegrator", 3100, 20, 9, 99)])
+def test_iteration_products(cuda, cls, m, k, p, N):
+    """The loops' products with Qs, Qs' and Bs in int8 slices (csrc/slice_gemm.cu): rows, columns and K around the
+    tiles (128, 32 or 64 columns a group, 128 of K, parts of K).  The products are off by about 1e-15 of the bases'
+    scale an iteration, as a running FP64 sum is; 1e-12 leaves room for the iterations' growth."""
+    from mcnla_b200 import isvd
+    l = k + p
+    q = _bases(cuda, m, l, N, m + k)
+    prm = isvd.Parameters().setSize(m, m).setRank(k).setOverRank(p).setNumSketch(N).sync()
+    st = getattr(isvd, cls)(prm, 64, 1e-6)
+    st.initialize()
+    qbar = prm.createMatrixQbar()
+    st(q, qbar)
+    ref, it = _kn(q, l, N, 64, 1e-6)
+    assert st.iteration() == it
+    assert float((qbar - ref).abs().max()) < 1e-12
+
+
+def test_iteration_products_scales_and_nan(cuda):
+    """Rows of very different magnitude keep their relative accuracy (the plain integrator: the row-block ones assume
+    orthonormal bases, which the scaled row ends); a NaN in Qs reaches the result and the iteration ends."""
+    from mcnla_b200 import isvd
+    m, k, p, N = 8192, 50, 14, 16
+    l = k + p
+    q = _bases(cuda, m, l, N, 3)
+    q[100] *= 1e-12
+    prm = isvd.Parameters().setSize(m, m).setRank(k).setOverRank(p).setNumSketch(N).sync()
+    st = isvd.KolmogorovNagumoIntegrator(prm, 12, 1e-9)
+    st.initialize()
+    qbar = prm.createMatrixQbar()
+    st(q, qbar)
+    ref, it = _kn(q, l, N, 12, 1e-9)
+    assert st.iteration() == it and float((qbar - ref).abs().max()) < 1e-12
+    assert float((qbar[100] - ref[100]).abs().max()) < 1e-12 * float(ref[100].abs().max())
+    q[7, 3] = float("nan")
+    st(q, qbar)
+    assert st.iteration() == 1 and torch.isnan(qbar).any()
