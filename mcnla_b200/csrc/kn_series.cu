@@ -8,8 +8,6 @@
 namespace mb {
 namespace {
 
-constexpr int kSerThreads = 256;
-
 struct StepArgs {
   SeriesArgs s;
   double tol;
@@ -42,7 +40,7 @@ size_t kn_series_work_doubles(int l) {
   // the series' scratch, or the four padded l x l matrices of the Newton-Schulz step where they do
   // not fit in shared memory (l > 80)
   const size_t lp = (size_t(l) + 15) & ~size_t(15);
-  return std::max(2 * size_t(l) * l + 3 * size_t((l + 7) / 8) + 8, l > 80 ? 4 * lp * (lp + 4) : 0);
+  return std::max(2 * size_t(l) * l + 3 * ((size_t(l) + 7) & ~size_t(7)) + 8, l > 80 ? 4 * lp * (lp + 4) : 0);
 }
 
 int launch_kn_series(Context* c, int l, const double* z, const double* dd, double inv_n, double* out, double* outn,

@@ -31,6 +31,7 @@
 namespace mb {
 namespace {
 
+constexpr int kSerThreads = 256;        // of the CTAs that take the step: a warp a row of the CTA's eight
 constexpr int kSerCoefs = 320;          // series coefficients kept in constant memory
 constexpr int kSerMaxDegree = 300;      // degree search limit
 constexpr int kSerMaxS = 18;            // most power slabs Z^1 .. Z^s on chip (fewer when they do not fit)
@@ -62,6 +63,7 @@ constexpr SeriesCoefs make_series_coefs() {
 }
 
 __constant__ SeriesCoefs c_series = make_series_coefs();
+__device__ const SeriesCoefs g_series = make_series_coefs();   // for lanes that read different n
 
 // Operands of one step (all l x l blocks row-major with row stride l).
 struct SeriesArgs {
@@ -81,16 +83,16 @@ struct SeriesArgs {
 };
 
 // Shared memory of the step: smax + 4 slabs of 8 rows, reduction space and,
-// for l <= kSerZsMax, a copy of Z (l rows, the slab row stride).
+// for l <= kSerZsMax, an l x l operand padded to whole tiles (the slab row stride).
 __host__ __device__ constexpr size_t kn_series_smem_doubles(int l, int smax) {
   return size_t(smax + 4) * 8 * (((l + 7) & ~7) + 4) + 32 +
-         (l <= kSerZsMax ? size_t(l) * (((l + 7) & ~7) + 4) : 0);
+         (l <= kSerZsMax ? size_t((l + 7) & ~7) * (((l + 7) & ~7) + 4) : 0);
 }
 
 // Most power slabs (<= kSerMaxS) whose step fits `optin` bytes of shared
-// memory next to `extra` doubles of the calling kernel (0 when even 4 do not).
+// memory next to `extra` doubles of the calling kernel (0 when even 5 do not).
 inline int kn_series_smax(int l, size_t optin, size_t extra) {
-  for (int smax = kSerMaxS; smax >= 4; --smax)
+  for (int smax = kSerMaxS; smax >= 5; --smax)
     if ((kn_series_smem_doubles(l, smax) + extra) * sizeof(double) + 1024 <= optin) return smax;
   return 0;
 }
@@ -108,7 +110,7 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
 // next multiple of gridDim.x.  One release (fence + relaxed add) per CTA and
 // acquire polls: no reset on the critical path.  Returns false when the wait
 // gave up (MCNLA_B200_ERR_DEVICE_TIMEOUT is recorded); the kernel returns.
-__device__ bool grid_sync(DevScalars* scal, volatile int* flag) {
+__device__ __noinline__ bool grid_sync(DevScalars* scal, volatile int* flag) {
   __syncthreads();
   if (gridDim.x == 1) return true;
   if (threadIdx.x == 0) {
@@ -260,18 +262,100 @@ inline SeriesArgs series_args(Context* c, int l, const double* z, const double* 
 
 enum : int { kStepTimeout = -1, kStepDeclined = 0, kStepDone = 1 };
 
-// One KN step (see the file comment).  Every CTA of the grid calls it; CTAs
-// [0, ceil(l/8)) do the work.  Returns kStepDone (C / Fc / inv(C) / F~+ in
+// An l x l matrix (row stride lds) into shared memory (row stride ld, zero up to
+// whole tiles): a warp per row, asynchronous 16-byte copies where rows start on
+// 16 bytes (l even).  Complete after copies_landed() and a block barrier.
+__device__ __noinline__ void load_square(double* dst, int ld, const double* src, int lds, int l) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, lp8 = (l + 7) & ~7;
+#pragma unroll 1
+  for (int i = warp; i < lp8; i += nw) {
+    double* d = dst + i * ld;
+    const double* s = src + size_t(i) * lds;
+    const int n = i < l ? l : 0;
+    if ((l & 1) == 0) {
+#pragma unroll 1
+      for (int j = 2 * lane; j < n; j += 64)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(unsigned(__cvta_generic_to_shared(d + j))),
+                     "l"(s + j)
+                     : "memory");
+    } else {
+#pragma unroll 1
+      for (int j = lane; j < n; j += 32) d[j] = __ldcg(s + j);
+    }
+#pragma unroll 1
+    for (int j = n + lane; j < lp8; j += 32) d[j] = 0.0;
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// Sums that a product's owner lanes update with its elements: F += f C1, G += g C1, D += h C2 (F, G, D slabs).
+struct SlabSums {
+  double *F, *G, *D;
+  double f, g, h;
+};
+
+// C1 = A1 Y (and C2 = A2 Y where A2 is given): 8 x l slabs (row stride ld, zero up to whole tiles) in shared memory,
+// Y(k, n) = Y[k ys + n yn] in shared or global memory.  A warp per 8-column tile, two accumulation chains: the two
+// products', or one's even and odd k-steps.  The precision form's BF16 loop turns other roundings here into 1e-9 of
+// its result, so the order of the sums is part of the step.
+// One copy of this code for every product of the step (see kn_series_step).  No barrier at the end.
+__device__ __noinline__ void slab_product(const double* A1, const double* A2, int ld, const double* Y, int ys, int yn,
+                                          int l, double* C1, double* C2, SlabSums sum) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int lp8 = (l + 7) & ~7;
+#pragma unroll 1
+  for (int t = warp; t * 8 < lp8; t += kSerThreads / 32) {
+    const int n = t * 8 + g;
+    const double* y = Y + (n < l ? n * yn : 0);
+    const int kn = n < l ? l : 0;
+    double c0 = 0.0, c1 = 0.0, e0 = 0.0, e1 = 0.0, d0 = 0.0, d1 = 0.0;
+    const int o = g * ld + t4;
+#pragma unroll 4
+    for (int k = 0; k < lp8; k += 8) {
+      const double y0 = k + t4 < kn ? y[(k + t4) * ys] : 0.0, y1 = k + 4 + t4 < kn ? y[(k + 4 + t4) * ys] : 0.0;
+      if (A2) {
+        dmma(c0, c1, A1[o + k], y0);
+        dmma(d0, d1, A2[o + k], y0);
+        dmma(c0, c1, A1[o + k + 4], y1);
+        dmma(d0, d1, A2[o + k + 4], y1);
+      } else {
+        dmma(c0, c1, A1[o + k], y0);
+        dmma(e0, e1, A1[o + k + 4], y1);
+      }
+    }
+    c0 += e0; c1 += e1;
+    const int q = g * ld + t * 8 + 2 * t4;
+    C1[q] = c0; C1[q + 1] = c1;
+    if (A2) { C2[q] = d0; C2[q + 1] = d1; }
+    if (sum.F) { sum.F[q] += sum.f * c0; sum.F[q + 1] += sum.f * c1; }
+    if (sum.G) { sum.G[q] += sum.g * c0; sum.G[q + 1] += sum.g * c1; }
+    if (sum.D) { sum.D[q] += sum.h * d0; sum.D[q + 1] += sum.h * d1; }
+  }
+}
+
+// One KN step (see the file comment).  Every CTA of the grid calls it
+// (kSerThreads threads); CTAs [0, ceil(l/8)) do the work.  Returns kStepDone (C / Fc / inv(C) / F~+ in
 // global memory, *norm = ||C - I||_F and *degree in every thread),
 // kStepDeclined (4 min(||Z||_F, ||Z||_inf) > 0.9 or not finite; nothing
 // written but Z) or
 // kStepTimeout.  end_barrier: end with a grid barrier after [Fc; inv(C)] are
 // written (when other CTAs read them next); F~+ is written after it.
+//
+// Latency-bound: a few barriers (1.4 us each) and a chain of small products, and bound by the fetching of its own
+// instructions when each of a dozen products is inlined (the stand-alone kernel's code was 155 KB, the persistent
+// kernel's 231 KB, run through once an iteration; now 54 and 80): all products are one function, and loops are not
+// unrolled but where loads have to be in flight together.  The l x l operands come in by asynchronous copies; the
+// plain powers' sums belong to the lanes that form the products, so a power is one call and one block barrier; row
+// sums and the degree search are a warp's work without block reductions.  The stand-alone step went from 27 to 20 us
+// at l = 64 and from 14.5 to 10.8 at l = 20, an iteration of the persistent kernel from 24.6 to 20.9 us (l = 12,
+// N l = 96), 37.4 to 31 (48, 384) and 69 to 61 (96, 768).  16 warps a CTA were slower (registers: 21.2 and 12.8 us).
 __device__ int kn_series_step(const SeriesArgs& a, double* sm, volatile int* flag, bool end_barrier, double* norm,
                               int* degree) {
   __shared__ int s_d, s_s;
   __shared__ double s_norm;
   const int l = a.l, tid = threadIdx.x, nt = blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31;
   const int gkn = (l + 7) >> 3;
   const bool mine = int(blockIdx.x) < gkn;
   const int lp8 = (l + 7) & ~7, ld = lp8 + 4;
@@ -284,99 +368,174 @@ __device__ int kn_series_step(const SeriesArgs& a, double* sm, volatile int* fla
   double* tF = accG + slab;
   double* tG = tF + slab;
   double* red = tG + slab;
+  double* DW = P + 4 * slab;                        // the plain powers: rows of sum g_j Dc Z^j
+  double* zs = red + 32;                            // an l x l operand: Dc, then Z, then Fc
   const double* coefF = c_series.f;                 // c^(-1/2): C
   const double* coefG = c_series.g;                 // c^(1/2):  inv(C)
   const int ldd = 2 * l;
+  const bool rb = a.dd != nullptr;
+  const bool zs_smem = l <= kSerZsMax;
+  double* sq = a.partials;                          // per row: squares, absolute values; then ||C - I||_F^2's parts
+  double* ab = sq + lp8;
+  double* np = ab + lp8;
   if (mine) {
-    for (int e = tid; e < (smax + 4) * slab; e += nt) sm[e] = 0.0;
-    __syncthreads();
-    // ---- Z rows [r0, r0 + 8)
-    if (a.dd != nullptr) {
-      // Z := Dgc - Dc Dc'   (row_block_kolmogorov_nagumo_integrator.hpp:150-156): Dc rows into tF,
-      // Dc Dc' rows into tG on the MMA
-      for (int e = tid; e < 8 * lp8; e += nt) {
-        const int rr = e / lp8, j = e % lp8, i = r0 + rr;
-        tF[rr * ld + j] = (i < l && j < l) ? __ldcg(a.dd + size_t(i) * ldd + j) : 0.0;
+    // ---- Z rows [r0, r0 + 8), a warp per row
+    const int i = r0 + warp;
+    if (rb) {
+      // Z := Dgc - Dc Dc'   (row_block_kolmogorov_nagumo_integrator.hpp:150-156): Dc rows in tF, Dgc's in P
+      if (zs_smem) load_square(zs, ld, a.dd, ldd, l);
+#pragma unroll 1
+      for (int j = lane; j < lp8; j += 32) {
+        const bool in = i < l && j < l;
+        const double* row = a.dd + size_t(in ? i : 0) * ldd + (in ? j : 0);
+        const double x = __ldcg(row), y = __ldcg(row + l);
+        tF[warp * ld + j] = in ? x : 0.0;
+        P[warp * ld + j] = in ? y : 0.0;
       }
+      copies_landed();
       __syncthreads();
-      slab_mm<true>(tF, nullptr, ld, a.dd, ldd, l, tG, nullptr);
+      slab_product(tF, nullptr, ld, zs_smem ? zs : a.dd, 1, zs_smem ? ld : ldd, l, tG, nullptr, SlabSums{});
+      __syncthreads();
     }
-    double part = 0.0;
-    for (int e = tid; e < 8 * l; e += nt) {
-      const int rr = e / l, j = e % l, i = r0 + rr;
-      if (i >= l) continue;
-      double v;
-      if (a.dd == nullptr) {
-        // the upper triangle mirrored (the reference's symmetric eigensolver reads one triangle)
-        v = __ldcg(a.z_in + size_t(min(i, j)) * l + max(i, j));
-      } else {
-        v = __ldcg(a.dd + size_t(i) * ldd + l + j) - tG[rr * ld + j];
-      }
-      P[rr * ld + j] = v;
-      a.zg[size_t(i) * l + j] = v;
-      part += v * v;
+    double ss = 0.0, rs = 0.0;
+#pragma unroll 1
+    for (int j = lane; j < lp8; j += 32) {
+      const bool in = i < l && j < l;
+      const int o = warp * ld + j;
+      double z;
+      // plain: the upper triangle mirrored (the reference's symmetric eigensolver reads one triangle)
+      if (rb) z = P[o] - tG[o];
+      else z = in ? __ldcg(a.z_in + size_t(min(i, j)) * l + max(i, j)) : 0.0;
+      P[o] = z;
+      if (in) a.zg[size_t(i) * l + j] = z;
+      ss += z * z;
+      rs += fabs(z);
+      // the plain powers' first terms
+      const double id = i == j ? 1.0 : 0.0;
+      accF[o] = coefF[0] * id + coefF[1] * z;
+      accG[o] = coefG[0] * id + coefG[1] * z;
+      if (rb) DW[o] = coefG[0] * tF[o];
     }
-    part = block_sum(part, red);
-    if (tid == 0) a.partials[blockIdx.x] = part;
-    // absolute row sums of the CTA's rows (a warp per row, fixed order) for
-    // the infinity-norm bound; red[16 ..] is clear of block_sum's slots
-    const int warp = tid >> 5, lane = tid & 31;
-    if (warp < 8) {
-      double rs = 0.0;
-      for (int j = lane; j < l; j += 32) rs += fabs(P[warp * ld + j]);
-      for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
-      if (lane == 0) red[16 + warp] = rs;
+    for (int o = 16; o > 0; o >>= 1) {
+      ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      rs += __shfl_xor_sync(0xffffffffu, rs, o);
     }
-    __syncthreads();
-    if (tid == 0) {
-      double mx = 0.0;
-      for (int w = 0; w < 8; ++w) mx = fmax(mx, red[16 + w]);
-      a.partials[2 * gkn + blockIdx.x] = mx;
+    if (lane == 0) {
+      sq[i] = ss;
+      ab[i] = rs;
     }
   }
   if (!grid_sync(a.scal, flag)) return kStepTimeout;
 
-  // ---- degree from z = min(||Z||_F, ||Z||_inf) >= ||Z||_2 (the same arithmetic in every CTA)
-  if (tid == 0) {
+  // Z for the products below: a shared-memory copy when it fits, in flight behind the degree search
+  if (mine && zs_smem) load_square(zs, ld, a.zg, l, l);
+  // ---- degree from z = min(||Z||_F, ||Z||_inf) >= ||Z||_2 (the same arithmetic in every CTA): lane n - 1 tests n
+  if (warp == 0) {
+    double cn = fmax(fabs(__ldg(g_series.f + lane + 1)), fabs(__ldg(g_series.g + lane + 1)));
     double s2 = 0.0, zi = 0.0;
-    for (int b = 0; b < gkn; ++b) {
-      s2 += __ldcg(a.partials + b);
-      zi = fmax(zi, __ldcg(a.partials + 2 * gkn + b));
+#pragma unroll 1
+    for (int b = lane; b < lp8; b += 32) {
+      s2 += __ldcg(sq + b);
+      zi = fmax(zi, __ldcg(ab + b));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      zi = fmax(zi, __shfl_xor_sync(0xffffffffu, zi, o));
     }
     const double z = fmin(sqrt(s2), zi);
     int d = -1;
-    if (4.0 * z <= kSerMaxRho) {                    // false for NaN
+    if (4.0 * z <= kSerMaxRho) {                    // false for NaN; the same in every lane
       const double scale = 1.0 / (1.0 - 4.0 * z);
-      double zn = 1.0;
-      for (int n = 1; n <= kSerMaxDegree + 1; ++n) {
-        zn *= z;
-        if (fmax(fabs(coefF[n]), fabs(coefG[n])) * zn * scale <= kSerTail) { d = n - 1; break; }
+      double zn = 1.0, base = z;                    // zn = z^(lane + 1)
+#pragma unroll
+      for (int e = 0; e < 6; ++e) {
+        if (((lane + 1) >> e) & 1) zn *= base;
+        base *= base;
+      }
+      const double z32 = __shfl_sync(0xffffffffu, zn, 31);
+#pragma unroll 1
+      for (int n0 = 0; n0 <= kSerMaxDegree; n0 += 32) {
+        const int n = n0 + lane + 1;
+        const unsigned hit = __ballot_sync(0xffffffffu, n <= kSerMaxDegree + 1 && cn * zn * scale <= kSerTail);
+        if (hit) {
+          d = n0 + __ffs(int(hit)) - 1;             // n - 1
+          break;
+        }
+        zn *= z32;
+        const int nn = min(n + 32, kSerCoefs - 1);
+        cn = fmax(fabs(__ldg(g_series.f + nn)), fabs(__ldg(g_series.g + nn)));
       }
       if (d == 0) d = 1;
     }
     int s = 1;
+#pragma unroll 1
     while (d >= 0 && s * s < d + 1) ++s;
-    if (s > smax) s = smax;
-    s_d = d;
-    s_s = s;
+    if (lane == 0) {
+      s_d = d;
+      s_s = min(s, smax);
+    }
   }
+  copies_landed();
   __syncthreads();
   const int d = s_d;
   if (d < 0) return kStepDeclined;                  // uniform over the grid
   const int s = s_s;
   const int nq = (d + s) / s;                       // blocks of s coefficients: degree nq*s - 1 >= d
   double* cinv = a.out + size_t(l) * l;
-  const bool rb = a.dd != nullptr;
-  // Z for the products below: a shared-memory copy when it fits
-  const bool zs_smem = l <= kSerZsMax;
-  double* zs = red + 32;
-  if (mine && zs_smem) {
-    for (int e = tid; e < l * l; e += nt) zs[(e / l) * ld + (e % l)] = __ldcg(a.zg + e);
+  const double* zy = zs_smem ? zs : a.zg;
+  const int zys = zs_smem ? ld : l;
+  // C1 = A1 Z, C2 = A2 Z
+  auto mm_z = [&](const double* A1, const double* A2, double* C1, double* C2, SlabSums sum) {
+    slab_product(A1, A2, ld, zy, zys, 1, l, C1, C2, sum);
     __syncthreads();
-  }
-  auto mm_z = [&](const double* A1, const double* A2, double* C1, double* C2) {
-    if (zs_smem) slab_mm<false, true>(A1, A2, ld, zs, ld, l, C1, C2);
-    else slab_mm(A1, A2, ld, a.zg, l, l, C1, C2);
+  };
+  // ||C - I||_F from the rows' parts, by warp 0 (read by all threads after the next block barrier)
+  auto norm_of = [&]() {
+    if (warp == 0) {
+      double s2 = 0.0;
+#pragma unroll 1
+      for (int b = lane; b < lp8; b += 32) s2 += __ldcg(np + b);
+      for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      if (lane == 0) s_norm = sqrt(s2);
+    }
+  };
+  // F~+ := F~c Fc   (row_block_gramian_kolmogorov_nagumo_integrator.hpp:197), after the barrier behind Fc
+  auto ff_rows = [&]() {
+    if (zs_smem) load_square(zs, ld, a.out, l, l);
+#pragma unroll 1
+    for (int j = lane; j < lp8; j += 32)
+      tF[warp * ld + j] = (r0 + warp < l && j < l) ? __ldcg(a.ff + size_t(r0 + warp) * l + j) : 0.0;
+    copies_landed();
+    __syncthreads();
+    slab_product(tF, nullptr, ld, zs_smem ? zs : a.out, zs_smem ? ld : l, 1, l, tG, nullptr, SlabSums{});
+    __syncthreads();
+#pragma unroll 1
+    for (int j = lane; j < l; j += 32)
+      if (r0 + warp < l) a.ffn[size_t(r0 + warp) * l + j] = tG[warp * ld + j];
+  };
+  // The CTA's rows of the results from C in F, inv(C) in G and Dc inv(C) in W (row block), with ||C - I||_F^2's part
+  auto put_rows = [&](const double* F, const double* G, const double* W) {
+    const int i = r0 + warp;
+    double part = 0.0;
+    if (i < l) {
+#pragma unroll 1
+      for (int j = lane; j < l; j += 32) {
+        const int o = warp * ld + j;
+        const size_t e = size_t(i) * l + j;
+        const double c = F[o], ci = G[o], dlt = c - (i == j ? 1.0 : 0.0);
+        part += dlt * dlt;
+        cinv[e] = ci;
+        // Fc := C - Dc inv(C)   (row_block_kolmogorov_nagumo_integrator.hpp:186)
+        const double fc = rb ? c - W[o] : c;
+        a.out[e] = fc;
+        if (rb && a.outn) {
+          a.outn[e] = fc;
+          a.outn[size_t(l) * l + e] = ci * a.inv_n;
+        }
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) np[i] = part;
   };
 
   if (d <= kSerDirectMax) {
@@ -385,84 +544,22 @@ __device__ int kn_series_step(const SeriesArgs& a, double* sm, volatile int* fla
     // CTA's rows of Z^j and Dc Z^j (products with the full Z only), so Fc
     // = C - Dc inv(C) needs no exchange of C or inv(C).
     if (mine) {
-      double* Pa = P;                               // rows of Z (from above)
-      double* Pb = P + 1 * slab;
-      double* Wa = P + 2 * slab;                    // rows of Dc Z^j
-      double* Wb = P + 3 * slab;
-      double* DW = P + 4 * slab;                    // rows of sum g_j Dc Z^j
-      for (int e = tid; e < 8 * lp8; e += nt) {
-        const int rr = e / lp8, j = e % lp8, i = r0 + rr;
-        const int o = rr * ld + j;
-        const double id = (i == j && i < l) ? 1.0 : 0.0;
-        accF[o] = coefF[0] * id + coefF[1] * Pa[o];
-        accG[o] = coefG[0] * id + coefG[1] * Pa[o];
-        if (rb) DW[o] = coefG[0] * tF[o];           // tF: rows of Dc
-      }
-      __syncthreads();
-      if (rb) {
-        mm_z(tF, nullptr, Wa, nullptr);
-        for (int e = tid; e < 8 * lp8; e += nt) {
-          const int o = (e / lp8) * ld + e % lp8;
-          DW[o] += coefG[1] * Wa[o];
-        }
-        __syncthreads();
-      }
-      double *pc = Pa, *pn = Pb, *wc = Wa, *wn = Wb;
+      const double* pc = P;                          // rows of Z^(j-1)
+      const double* wc = P + 2 * slab;               // rows of Dc Z^(j-1)
+      if (rb) mm_z(tF, nullptr, P + 2 * slab, nullptr, SlabSums{DW, nullptr, nullptr, coefG[1], 0.0, 0.0});
+#pragma unroll 1
       for (int j = 2; j <= d; ++j) {
-        mm_z(pc, rb ? wc : nullptr, pn, rb ? wn : nullptr);
-        for (int e = tid; e < 8 * lp8; e += nt) {
-          const int o = (e / lp8) * ld + e % lp8;
-          accF[o] += coefF[j] * pn[o];
-          accG[o] += coefG[j] * pn[o];
-          if (rb) DW[o] += coefG[j] * wn[o];
-        }
-        __syncthreads();
-        double* x = pc; pc = pn; pn = x;
-        x = wc; wc = wn; wn = x;
+        double* pn = P + (j & 1 ? 0 : 1) * slab;
+        double* wn = P + (j & 1 ? 2 : 3) * slab;
+        mm_z(pc, rb ? wc : nullptr, pn, wn, SlabSums{accF, accG, rb ? DW : nullptr, coefF[j], coefG[j], coefG[j]});
+        pc = pn;
+        wc = wn;
       }
-      double part = 0.0;
-      for (int e = tid; e < 8 * l; e += nt) {
-        const int rr = e / l, j = e % l, i = r0 + rr;
-        if (i >= l) continue;
-        const int o = rr * ld + j;
-        const double c = accF[o], ci = accG[o];
-        const double dlt = c - (i == j ? 1.0 : 0.0);
-        part += dlt * dlt;
-        cinv[size_t(i) * l + j] = ci;
-        if (!rb) {
-          a.out[size_t(i) * l + j] = c;
-        } else {
-          // Fc := C - Dc inv(C)   (row_block_kolmogorov_nagumo_integrator.hpp:186)
-          const double fc = c - DW[o];
-          a.out[size_t(i) * l + j] = fc;
-          if (a.outn) {
-            a.outn[size_t(i) * l + j] = fc;
-            a.outn[size_t(l) * l + size_t(i) * l + j] = ci * a.inv_n;
-          }
-        }
-      }
-      part = block_sum(part, red);
-      if (tid == 0) a.partials[gkn + blockIdx.x] = part;
+      put_rows(accF, accG, DW);
     }
     if (!grid_sync(a.scal, flag)) return kStepTimeout;
-    if (tid == 0) {
-      double s2 = 0.0;
-      for (int b = 0; b < gkn; ++b) s2 += __ldcg(a.partials + gkn + b);
-      s_norm = sqrt(s2);
-    }
-    if (rb && a.ff && a.ffn && mine) {
-      // F~+ := F~c Fc   (row_block_gramian_kolmogorov_nagumo_integrator.hpp:197)
-      for (int e = tid; e < 8 * lp8; e += nt) {
-        const int rr = e / lp8, j = e % lp8, i = r0 + rr;
-        tF[rr * ld + j] = (i < l && j < l) ? __ldcg(a.ff + size_t(i) * l + j) : 0.0;
-      }
-      __syncthreads();
-      slab_mm(tF, nullptr, ld, a.out, l, l, tG, nullptr);
-      for (int e = tid; e < 8 * l; e += nt) {
-        const int rr = e / l, j = e % l, i = r0 + rr;
-        if (i < l) a.ffn[size_t(i) * l + j] = tG[rr * ld + j];
-      }
-    }
+    norm_of();
+    if (rb && a.ff && a.ffn && mine) ff_rows();
     __syncthreads();
     *norm = s_norm;
     *degree = d;
@@ -472,8 +569,10 @@ __device__ int kn_series_step(const SeriesArgs& a, double* sm, volatile int* fla
   // ---- rows of Z^2 .. Z^s (Z^s only when a Horner step needs it)
   if (mine) {
     const int top = nq > 1 ? s : s - 1;
-    for (int j = 2; j <= top; ++j) mm_z(P + (j - 2) * slab, nullptr, P + (j - 1) * slab, nullptr);
+#pragma unroll 1
+    for (int j = 2; j <= top; ++j) mm_z(P + (j - 2) * slab, nullptr, P + (j - 1) * slab, nullptr, SlabSums{});
     if (nq > 1) {
+#pragma unroll 1
       for (int e = tid; e < 8 * l; e += nt) {
         const int rr = e / l, j = e % l, i = r0 + rr;
         if (i < l) a.zsg[size_t(i) * l + j] = P[(s - 1) * slab + rr * ld + j];
@@ -485,6 +584,7 @@ __device__ int kn_series_step(const SeriesArgs& a, double* sm, volatile int* fla
   if (mine) {
     // ---- Horner in Z^s:  acc = B_{nq-1};  acc = acc Z^s + B_q,  B_q = sum_j a_{qs+j} Z^j
     auto add_block = [&](int q, double* dF, double* dG, bool accumulate) {
+#pragma unroll 1
       for (int e = tid; e < 8 * lp8; e += nt) {
         const int rr = e / lp8, j = e % lp8, i = r0 + rr;
         double vF = 0.0, vG = 0.0;
@@ -493,6 +593,7 @@ __device__ int kn_series_step(const SeriesArgs& a, double* sm, volatile int* fla
             vF = coefF[q * s];
             vG = coefG[q * s];
           }
+#pragma unroll 1
           for (int p = 1; p < s; ++p) {
             const double x = P[(p - 1) * slab + rr * ld + j];
             vF = fma(coefF[q * s + p], x, vF);
@@ -511,72 +612,45 @@ __device__ int kn_series_step(const SeriesArgs& a, double* sm, volatile int* fla
       __syncthreads();
     };
     add_block(nq - 1, accF, accG, false);
+#pragma unroll 1
     for (int q = nq - 2; q >= 0; --q) {
-      slab_mm(accF, accG, ld, a.zsg, l, l, tF, tG);
+      slab_product(accF, accG, ld, a.zsg, l, 1, l, tF, tG, SlabSums{});
+      __syncthreads();
       add_block(q, tF, tG, true);
       double* x = accF; accF = tF; tF = x;
       x = accG; accG = tG; tG = x;
     }
     // ---- C in accF, inv(C) in accG;  ||e - 1||_2 = ||C - I||_F
-    double part = 0.0;
-    for (int e = tid; e < 8 * l; e += nt) {
-      const int rr = e / l, j = e % l, i = r0 + rr;
-      if (i >= l) continue;
-      const int o = rr * ld + j;
-      const double c = accF[o];
-      const double dlt = c - (i == j ? 1.0 : 0.0);
-      part += dlt * dlt;
-      cinv[size_t(i) * l + j] = accG[o];
-      if (a.dd == nullptr) a.out[size_t(i) * l + j] = c;
+    if (rb) {
+      // inv(C) for the other CTAs' Dc inv(C)
+#pragma unroll 1
+      for (int j = lane; j < l; j += 32)
+        if (r0 + warp < l) cinv[size_t(r0 + warp) * l + j] = accG[warp * ld + j];
+    } else {
+      put_rows(accF, accG, nullptr);
     }
-    part = block_sum(part, red);
-    if (tid == 0) a.partials[gkn + blockIdx.x] = part;
   }
   if (!grid_sync(a.scal, flag)) return kStepTimeout;
-  if (tid == 0) {
-    double s2 = 0.0;
-    for (int b = 0; b < gkn; ++b) s2 += __ldcg(a.partials + gkn + b);
-    s_norm = sqrt(s2);
-  }
 
   if (rb) {
     if (mine) {
-      // Fc := C - Dc inv(C)   (row_block_kolmogorov_nagumo_integrator.hpp:186)
-      for (int e = tid; e < 8 * lp8; e += nt) {
-        const int rr = e / lp8, j = e % lp8, i = r0 + rr;
-        tF[rr * ld + j] = (i < l && j < l) ? __ldcg(a.dd + size_t(i) * ldd + j) : 0.0;
-      }
+      if (zs_smem) load_square(zs, ld, cinv, l, l);
+#pragma unroll 1
+      for (int j = lane; j < lp8; j += 32)
+        tF[warp * ld + j] = (r0 + warp < l && j < l) ? __ldcg(a.dd + size_t(r0 + warp) * ldd + j) : 0.0;
+      copies_landed();
       __syncthreads();
-      slab_mm(tF, nullptr, ld, cinv, l, l, tG, nullptr);
-      for (int e = tid; e < 8 * l; e += nt) {
-        const int rr = e / l, j = e % l, i = r0 + rr;
-        if (i >= l) continue;
-        const int o = rr * ld + j;
-        const double fc = accF[o] - tG[o];
-        a.out[size_t(i) * l + j] = fc;
-        if (a.outn) {
-          a.outn[size_t(i) * l + j] = fc;
-          a.outn[size_t(l) * l + size_t(i) * l + j] = accG[o] * a.inv_n;
-        }
-      }
-    }
-    const bool ffu = a.ff && a.ffn;
-    if ((end_barrier || ffu) && !grid_sync(a.scal, flag)) return kStepTimeout;
-    if (ffu && mine) {
-      // F~+ := F~c Fc   (row_block_gramian_kolmogorov_nagumo_integrator.hpp:197)
-      for (int e = tid; e < 8 * lp8; e += nt) {
-        const int rr = e / lp8, j = e % lp8, i = r0 + rr;
-        tF[rr * ld + j] = (i < l && j < l) ? __ldcg(a.ff + size_t(i) * l + j) : 0.0;
-      }
+      slab_product(tF, nullptr, ld, zs_smem ? zs : cinv, zs_smem ? ld : l, 1, l, tG, nullptr, SlabSums{});
       __syncthreads();
-      slab_mm(tF, nullptr, ld, a.out, l, l, tG, nullptr);
-      for (int e = tid; e < 8 * l; e += nt) {
-        const int rr = e / l, j = e % l, i = r0 + rr;
-        if (i < l) a.ffn[size_t(i) * l + j] = tG[rr * ld + j];
-      }
+      put_rows(accF, accG, tG);
     }
-  } else if (end_barrier && !grid_sync(a.scal, flag)) {
-    return kStepTimeout;
+    // the parts of ||C - I||_F, and Fc for the next product
+    if (!grid_sync(a.scal, flag)) return kStepTimeout;
+    norm_of();
+    if (a.ff && a.ffn && mine) ff_rows();
+  } else {
+    norm_of();
+    if (end_barrier && !grid_sync(a.scal, flag)) return kStepTimeout;
   }
   __syncthreads();
   *norm = s_norm;

@@ -298,6 +298,29 @@ def test_kn_wide_sketches(cuda, l, cls_name, oracle_name):
         ctx.set_kn_method(_lib.KN_AUTO)
 
 
+@pytest.mark.parametrize("l", [2, 7, 9, 31, 111, 113])
+@pytest.mark.parametrize("cls_name,oracle_name", [
+    ("KolmogorovNagumoIntegrator", "kn"),
+    ("RowBlockKolmogorovNagumoIntegrator", "rb_kn"),
+    ("RowBlockGramianKolmogorovNagumoIntegrator", "rb_gramian_kn"),
+])
+def test_kn_step_tile_edges(cuda, l, cls_name, oracle_name):
+    """The series step at sketch widths off its 8-row tiles: odd rows (no 16-byte copies), the last width whose
+    operands fit in shared memory and the first past it, in the plain, row-block and persistent forms."""
+    from mcnla_b200 import isvd, synthetic
+    m, n, N = 900, 500, 3
+    a = synthetic.lowrank_np(m, n, np.arange(1, n + 1) ** -1.0, seed=l)
+    qs = O.orthogonalize_gramian(a @ np.random.default_rng(l).standard_normal((n, l * N)), l, N)
+    qo, it_ref = O.INTEGRATORS[oracle_name](qs, l, N, 256, 1e-5)
+    prm = params(m, n, l, 0, N)
+    integ = getattr(isvd, cls_name)(prm, 256, 1e-5)
+    integ.initialize()
+    qbar = prm.createMatrixQbar()
+    integ(dev(qs, cuda), qbar)
+    assert integ.iteration() == it_ref
+    assert np.abs(host(qbar) - qo).max() < TOL
+
+
 @pytest.mark.parametrize("cls_name,oracle_name", [
     ("RowBlockWenYinIntegrator", "rb_wy"),
     ("RowBlockGramianWenYinIntegrator", "rb_gramian_wy"),
