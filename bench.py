@@ -33,11 +33,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = "iSVD/s & A-read GB/s, mixed vs FP64 plain on B200 at σ err≤1e-6; p50/p99 ms"
 
-# dram bytes (read + write) per row of A for one launch of the sketch GEMM, from
-# one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum: 22.48 GB +
-# 0.53 GB) of the 16384 x 20000 x 4096 case with the 64 x 128 two-CTA tile;
-# scaled by rows to the benchmark's m (A is re-read ~8.6x through L2)
-SKETCH_TRAFFIC_PER_ROW = (22.475526e9 + 0.534837e9) / 16384
+# dram bytes (read + write) per row of A of the sketch's int8 GEMM at the benchmark's n and N l: not captured.  At
+# 16384 x 4096 x 4096 a row takes 134 KB (15 residue bytes an element of A and of C are 123 KB), DRAM 12 % busy, the
+# int8 pipe 73 %.
+SKETCH_TRAFFIC_PER_ROW = None
 
 
 def parse():
@@ -626,7 +625,11 @@ def run_b200(args, world, rank, local):
 
     stage_roof = stage_rooflines(m, n, k, l, N, args.integrator, args.former, stages, peak64,
                                  _measured_peak("hbm_gbs"))
-    roofline = {"bound": "tensor", "kernel": "dgemm_kernel (sketch Y = A Omega, FP64 DMMA)",
+    # the sketch runs on the int8 tensor cores (15 residue products and the CRT): against the FP64 peak frac is the
+    # speed-up over the FP64 pipe, and int8_tops the rate of the pipe that does the work
+    roofline = {"bound": "tensor",
+                "kernel": "rns_gemm_kernel with its residues and CRT (sketch Y = A Omega, FP64 by int8 residues)",
+                "int8_tops": round(15 * achieved, 1),
                 "achieved": round(achieved, 3), "peak": round(peak64, 3), "unit": "TFLOP/s",
                 "frac": round(achieved / peak64, 4), "traffic": traffic,
                 "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 has no tcgen05 kind; the "
@@ -1228,7 +1231,7 @@ def run_syev(args, dev):
         resid = max(float(np.abs(gn[b] @ vn[b] - vn[b] * wn[b]).max() / wn[b].max()) for b in range(batch))
         orth = max(float(np.abs(vn[b].T @ vn[b] - np.eye(l)).max()) for b in range(batch))
         rows.append({"l": l, "batch": batch, "ms": round(best, 3), "residual": resid, "orthogonality": orth})
-    return {"kernel": "k_syev (batched Jacobi, 1024 threads per matrix)", "rows": rows}
+    return {"kernel": "k_jacobi_rotations / k_jacobi_vectors (batched Jacobi)", "rows": rows}
 
 
 def run_kernel_case(args, dev):
