@@ -172,7 +172,7 @@ __device__ void gemm_unit(const double* A, int64_t ars, int64_t acs, const doubl
 // cluster: block b on CTA b mod ncta, one block after another.  Between the
 // step's phases only global memory carries state (Z, Z^s, the partial sums,
 // inv(C), Fc and C in cbuf), so each block's shared-memory slabs are rebuilt
-// from it, starting from zeroed slabs like a CTA of the cooperative step.
+// from it, starting from zeroed slabs.
 __device__ int kn_series_step_cluster(const SeriesArgs& a, double* sm, double* cbuf, const cg::cluster_group& cl,
                                       int rank, int ncta, double* norm, int* degree) {
   __shared__ int s_d, s_s;
@@ -251,7 +251,7 @@ __device__ int kn_series_step_cluster(const SeriesArgs& a, double* sm, double* c
   }
   cluster_sync(cl);
 
-  // ---- degree (the arithmetic of kn_series_step, the same in every CTA)
+  // ---- degree (the rule of kn_series_step; the same arithmetic in every CTA)
   if (tid == 0) {
     double s2 = 0.0, zi = 0.0;
     for (int b = 0; b < gkn; ++b) {
