@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cooperative_groups.h>
+#include <utility>
 
 namespace mb {
 namespace {
@@ -171,6 +172,8 @@ __global__ void __cluster_dims__(kFewCtas, 1, 1) __launch_bounds__(kFewThreads)
   __shared__ double red[kFewThreads / 32][4];
   __shared__ double cmax[kFewCtas][4];
   auto cluster = cg::this_cluster();
+  // a CTA's shared memory may be written from outside only once the CTA runs; the read of B hides the wait
+  auto started = cluster.barrier_arrive();
   const int rank = int(cluster.block_rank());
   const int c = threadIdx.x & 3, col = int(blockIdx.x / kFewCtas) * 4 + c;
   const double* b = B + col;
@@ -190,6 +193,7 @@ __global__ void __cluster_dims__(kFewCtas, 1, 1) __launch_bounds__(kFewThreads)
   for (int d = 16; d >= 4; d >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, d));
   if ((threadIdx.x & 31) < 4) red[threadIdx.x >> 5][c] = mx;
   __syncthreads();
+  cluster.barrier_wait(std::move(started));
   if (threadIdx.x < 4 * kFewCtas) {        // this CTA's maxima to CTA threadIdx.x / 4
     for (int w = 0; w < kFewThreads / 32; ++w) mx = fmax(mx, red[w][c]);
     *cluster.map_shared_rank(&cmax[rank][c], threadIdx.x >> 2) = mx;
