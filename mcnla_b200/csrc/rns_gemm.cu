@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __shared__ __align__(8) uint64_t empty_bar[kStages];   // the MMAs have read the stage
   __shared__ __align__(8) uint64_t acc_full[2];          // accumulator b is complete
   __shared__ __align__(8) uint64_t acc_empty[2];         // accumulator b has been read
+  __shared__ __align__(8) uint64_t mma_done;             // every issued MMA has completed
   __shared__ uint32_t tmem_base_s;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -290,6 +291,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], kEpiWarps);
     }
+    mbar_init(&mma_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fence_before();
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   if (warp == 0) {
     // ---- producer (the whole warp walks the jobs; one lane copies)
-    int64_t it = 0;
+    int64_t it = 0, issued = 0;
     bool ok = true;
     for (int64_t j = blockIdx.x; j < g.jobs && ok; j += gridDim.x) {
       Job jb;
@@ -311,8 +313,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           const int64_t i = it + kt;
           const int s = int(i % kStages);
           if (i >= kStages && !mbar_wait(&empty_bar[s], uint32_t(((i / kStages) & 1) ^ 1))) {
-            // let the copies in flight land before the CTA's shared memory goes away
-            for (int64_t f = i - kStages; f < i; ++f) mbar_wait(&full_bar[f % kStages], uint32_t((f / kStages) & 1));
             ok = false;
             break;
           }
@@ -320,12 +320,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           uint8_t* sa = smem + s * kStageBytes;
           tma_load_2d(sa, &tm_a, &full_bar[s], kt * kKTile, ya);
           tma_load_2d(sa + kABytes, &tm_b, &full_bar[s], kt * kKTile, yb);
+          ++issued;
         }
       }
       it += g.kt;
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (!ok && lane == 0) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
+    if (lane == 0) {
+      if (!ok) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
+      // the copies in flight land before the CTA's shared memory goes away, whoever gave up
+      for (int64_t f = issued > kStages ? issued - kStages : 0; f < issued; ++f)
+        mbar_wait(&full_bar[f % kStages], uint32_t((f / kStages) & 1));
+    }
   } else if (warp == 1) {
     // ---- MMA issuer
     int64_t it = 0, done = 0;
@@ -356,6 +362,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       it += g.kt;
       ++done;
       ok = __all_sync(0xffffffffu, ok);
+    }
+    if (lane == 0) {
+      umma_commit(&mma_done);      // every MMA issued above completes before TMEM goes back, whatever was given up
+      mbar_wait(&mma_done, 0);
     }
   } else if (warp >= 4) {
     // ---- epilogue: residue sums -> digits

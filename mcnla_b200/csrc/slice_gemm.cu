@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(256, 1)
   using T = SCfg<NB>;
   if (g.guard_stop && *g.guard_stop < g.guard_it) return;
   extern __shared__ uint8_t smem_dyn[];
-  __shared__ __align__(8) uint64_t full_a[kARing], empty_a[kARing], full_b[2], empty_b[2], acc_full;
+  __shared__ __align__(8) uint64_t full_a[kARing], empty_a[kARing], full_b[2], empty_b[2], acc_full, mma_done;
   __shared__ uint32_t tmem_base_s;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_b = smem + kARing * kATile;
@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(256, 1)
       mbar_init(&empty_b[b], 1);
     }
     mbar_init(&acc_full, 1);
+    mbar_init(&mma_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fence_before();
@@ -300,13 +301,11 @@ __global__ void __launch_bounds__(256, 1)
         ++issued_a;
       }
     }
-    if (!ok) {
-      atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
-      // let the copies in flight land before the CTA's shared memory goes away
-      for (int i = max(0, issued_a - kARing); i < issued_a; ++i)
-        mbar_wait(&full_a[i % kARing], uint32_t((i / kARing) & 1));
-      for (int i = max(0, issued_b - 2); i < issued_b; ++i) mbar_wait(&full_b[i & 1], uint32_t((i >> 1) & 1));
-    }
+    if (!ok) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
+    // the copies in flight land before the CTA's shared memory goes away, whoever gave up
+    for (int i = max(0, issued_a - kARing); i < issued_a; ++i)
+      mbar_wait(&full_a[i % kARing], uint32_t((i / kARing) & 1));
+    for (int i = max(0, issued_b - 2); i < issued_b; ++i) mbar_wait(&full_b[i & 1], uint32_t((i >> 1) & 1));
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer
     bool ok = true;
@@ -337,12 +336,10 @@ __global__ void __launch_bounds__(256, 1)
       }
       if (ok) umma_commit(&empty_b[b]);
     }
-    if (ok) {
-      umma_commit(&acc_full);
-      mbar_wait(&acc_full, 0);               // every MMA and its commits have completed
-    } else {
-      atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
-    }
+    if (ok) umma_commit(&acc_full);
+    else atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
+    umma_commit(&mma_done);      // every MMA issued above completes before TMEM goes back, whatever was given up
+    mbar_wait(&mma_done, 0);
   } else if (warp >= 4) {
     // ---- the sums to FP64: D_0 + 2^-8 (D_1 + 2^-8 (...))
     const int q = warp & 3;
