@@ -9,7 +9,7 @@
 // (d >= kSlices, and the integers' rounding) is about 2^-56 sqrt(K) max|a_i| max|b_j|, below the 2^-54 |a_i| |b_j|
 // of a running sum for rows and columns without a few dominating entries.  (Ozaki, Ogita, Oishi and Rump, "Error-free
 // transformations of matrix multiplication", Numer. Algorithms 59, 2012.)  A is cut once (7 bytes an element, less
-// than its FP64 form); a row or column with NaN or infinities makes its results NaN.
+// than its FP64 form).  Any finite magnitude of a row or column is taken; NaN or infinities make its results NaN.
 #pragma once
 #include "common.cuh"
 

@@ -22,30 +22,39 @@ __device__ __forceinline__ double pow2(int e) {   // |e| < 1023
   return __longlong_as_double((long long)(e + 1023) << 52);
 }
 
+constexpr int kNotFinite = INT32_MIN;
+
 // Exponent s with max |x| 2^s below 0.99 2^55 (the largest seven digits hold), and what undoes it per slice base:
-// 2^(48 - s).  Not finite, or out of 2^+-400: NaN.
-__device__ __forceinline__ int scale_of(double mx, double* unscale) {
-  if (mx == 0.0) { *unscale = 0.0; return 0; }
-  if (!(mx >= 0x1p-400) || !(mx <= 0x1p400)) {
-    // NaN and infinities, and magnitudes no orthonormal basis has
-    *unscale = __longlong_as_double(0x7ff8000000000000LL);
+// 2^*unscale = 2^(48 - s).  Any finite maximum, subnormal ones included; not finite: kNotFinite.
+__device__ __forceinline__ int scale_of(double mx, int* unscale) {
+  *unscale = 0;
+  if (mx == 0.0) return 0;
+  if (!(mx <= 1.7976931348623157e308)) {
+    *unscale = kNotFinite;
     return 0;
   }
-  int e = int((__double_as_longlong(mx) >> 52) & 0x7ff) - 1022;         // mx < 2^e
-  if (mx >= 0.99 * pow2(e)) ++e;
-  *unscale = pow2(48 - (55 - e));
+  int e;
+  const double f = frexp(mx, &e);                                       // mx = f 2^e, f in [1/2, 1)
+  if (f >= 0.99) ++e;
+  *unscale = e - 7;
   return 55 - e;
 }
 
-__device__ __forceinline__ unsigned long long digits(double x, double s1, double s2) {
-  return (unsigned long long)(__double2ll_rn(x * s1 * s2) + (long long)kBias);
+// v 2^e for the sum of two such exponents (below 2^-1120 everything here is zero)
+__device__ __forceinline__ double times_pow2(double v, int e) {
+  const int c = max(e, -1120), h = c / 2;
+  return v * pow2(h) * pow2(c - h);
+}
+
+__device__ __forceinline__ unsigned long long digits(double y) {   // y: the scaled entry
+  return (unsigned long long)(__double2ll_rn(y) + (long long)kBias);
 }
 
 // Slices in tiles of `tile` rows by 128 bytes of K, a tile's seven slices one after the other, tiles along K, then
 // along the rows: what a CTA reads is contiguous (128-byte pieces of rows of K bytes apart ran at 2.6 TB/s).
 struct Sliced {
   uint8_t* base;
-  double* unscale;      // [row]
+  int* unscale;         // [row]: exponents
   int64_t kt;           // k-tiles
   int64_t tile;         // rows of a tile
   __device__ __forceinline__ uint8_t* at(int64_t row, int64_t k) const {   // slice 0 (the highest digit)
@@ -83,18 +92,18 @@ __global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();
   for (int w = 0; w < 8; ++w) mx = fmax(mx, red[w]);
-  double un;
+  int un;
   const int e = scale_of(mx, &un);
   if (threadIdx.x == 0) o.unscale[row] = un;
   const int h = e / 2;
   const double s1 = pow2(h), s2 = pow2(e - h);
-  const bool ok = un == un;
+  const bool ok = un != kNotFinite;
   for (int64_t q = threadIdx.x; q < o.kt * (kKTile / 4); q += 256) {
     unsigned long long u[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int64_t k = 4 * q + j;
-      u[j] = ok && k < K ? digits(a[k], s1, s2) : kBias;
+      u[j] = digits(ok && k < K ? a[k] * s1 * s2 : 0.0);
     }
     store4(u, o.at(row, 4 * q), o.plane());
   }
@@ -143,9 +152,9 @@ __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B
   __syncthreads();
   if (w == 0) {
     for (int i = 1; i < 8; ++i) mx = fmax(mx, sm[i][lane]);
-    double un;
+    int un;
     se[lane] = scale_of(mx, &un);
-    sok[lane] = un == un;
+    sok[lane] = un != kNotFinite;
     if (r < R && blockIdx.x == 0) o.unscale[r] = un;
   }
   __syncthreads();
@@ -155,7 +164,7 @@ __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B
     const double s1 = pow2(h), s2 = pow2(e - h);
     unsigned long long u[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) u[j] = sok[i] ? digits(tile[i][4 * lane + j], s1, s2) : kBias;
+    for (int j = 0; j < 4; ++j) u[j] = digits(sok[i] ? tile[i][4 * lane + j] * s1 * s2 : 0.0);
     store4(u, o.at(r0 + i, k0 + 4 * lane), o.plane());
   }
 }
@@ -201,15 +210,15 @@ __global__ void __cluster_dims__(kFewCtas, 1, 1) __launch_bounds__(kFewThreads)
   cluster.sync();
 #pragma unroll
   for (int w = 0; w < kFewCtas; ++w) mx = fmax(mx, cmax[w][c]);
-  double un;
+  int un;
   const int e = scale_of(mx, &un), h = e / 2;
   const double s1 = pow2(h), s2 = pow2(e - h);
-  const bool ok = un == un && col < l;
+  const bool ok = un != kNotFinite && col < l;
   if (rank == 0 && threadIdx.x < 4) o.unscale[col] = un;
   for (int64_t k = k0 + 4 * (threadIdx.x >> 2); k < k1; k += kFewThreads) {
     unsigned long long u[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) u[j] = ok && k + j < K ? digits(b[(k + j) * ld], s1, s2) : kBias;
+    for (int j = 0; j < 4; ++j) u[j] = ok && k + j < K ? digits(b[(k + j) * ld] * s1 * s2) : kBias;
     store4(u, o.at(col, k), o.plane());
   }
 }
@@ -218,7 +227,7 @@ struct SArgs {
   int b_rows;               // rows of B's tiles (columns, padded to the groups)
   int M, l;
   int kt, kt_per;           // k-tiles in all and of a part
-  const double *ua, *ub;
+  const int *ua, *ub;       // exponents of the rows and the columns
   double* out;              // [part][M][l]
   int* status;
   const int* guard_stop;
@@ -349,7 +358,7 @@ __global__ void __launch_bounds__(256, 1)
       if (lane == 0) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
     } else {
       const int row = m0 + q * 32 + lane;
-      const double ua = row < g.M ? g.ua[row] : 0.0;
+      const int ua = row < g.M ? g.ua[row] : 0;
       // every MMA has completed, so the ring is idle: 32 x 32 blocks go through it and out a row at a time
       double* stg = reinterpret_cast<double*>(smem) + q * 32 * 33;
 #pragma unroll 1
@@ -365,13 +374,17 @@ __global__ void __launch_bounds__(256, 1)
           for (int j = 0; j < 32; ++j) acc[j] = fma(acc[j], 0x1p-8, double(int(r[j])));
         }
 #pragma unroll
-        for (int j = 0; j < 32; ++j) stg[lane * 33 + j] = acc[j] * ua;
+        for (int j = 0; j < 32; ++j) stg[lane * 33 + j] = acc[j];
         __syncwarp();
         const int col = grp * NB + c + lane;
-        if (col < g.l) {
-          const double ub = g.ub[col];
-          for (int i = 0; i < 32 && m0 + q * 32 + i < g.M; ++i)
-            g.out[(int64_t(part) * g.M + m0 + q * 32 + i) * g.l + col] = stg[i * 33 + lane] * ub;
+        const int ub = col < g.l ? g.ub[col] : 0;
+#pragma unroll 4
+        for (int i = 0; i < 32; ++i) {
+          const int ui = __shfl_sync(0xffffffffu, ua, i);
+          if (m0 + q * 32 + i < g.M && col < g.l)
+            g.out[(int64_t(part) * g.M + m0 + q * 32 + i) * g.l + col] =
+                ui == kNotFinite || ub == kNotFinite ? __longlong_as_double(0x7ff8000000000000LL)
+                                                     : times_pow2(stg[i * 33 + lane], ui + ub);
         }
         __syncwarp();
       }
@@ -408,8 +421,8 @@ ALayout a_layout(const SlicePlan& p, void* w) {
   char* base = reinterpret_cast<char*>(up(reinterpret_cast<uintptr_t>(w)));
   a.o.base = reinterpret_cast<uint8_t*>(base);
   size_t off = up(size_t(a.rows) * kKTile);
-  a.o.unscale = reinterpret_cast<double*>(base + off);
-  off += up(size_t(p.M) * 8);
+  a.o.unscale = reinterpret_cast<int*>(base + off);
+  off += up(size_t(p.M) * 4);
   a.part = reinterpret_cast<double*>(base + off);
   off += up(size_t(cdiv(p.K, kStatK)) * p.M * 8);
   a.bytes = off + 1024;
@@ -425,8 +438,8 @@ WLayout w_layout(const SlicePlan& p, void* w) {
   char* base = reinterpret_cast<char*>(up(reinterpret_cast<uintptr_t>(w)));
   b.o.base = reinterpret_cast<uint8_t*>(base);
   size_t off = up(size_t(b.rows) * kKTile);
-  b.o.unscale = reinterpret_cast<double*>(base + off);
-  off += up(size_t(b.o.tile) * 8);
+  b.o.unscale = reinterpret_cast<int*>(base + off);
+  off += up(size_t(b.o.tile) * 4);
   b.sums = reinterpret_cast<double*>(base + off);
   off += up(size_t(p.splits) * p.M * p.l * 8);
   b.bytes = off + 1024;
