@@ -14,6 +14,7 @@ namespace cg = cooperative_groups;
 
 constexpr int kKTile = 128;                // bytes of K in a shared-memory tile: one 128-byte swizzle row
 constexpr int kTileM = 128;
+constexpr int kSums = 8;                   // orders d = s + t kept
 constexpr int64_t kMaxK = 18000;           // of a part: 7 K 2^14 < 2^31
 constexpr int kStatK = 256;
 constexpr unsigned long long kBias = 0x80808080808080ull;   // seven digits of 128: digit = byte ^ 0x80, signed
@@ -74,8 +75,13 @@ __device__ __forceinline__ void store4(const unsigned long long (&u)[4], uint8_t
   }
 }
 
-// Rows with K contiguous, one CTA a row.
-__global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A, int64_t lda, int64_t K, Sliced o) {
+// Whether a row has too few entries near its largest for fixed-point digits (see slice.cuh), from the sums over its
+// scaled entries.
+__device__ __forceinline__ bool few_large(double norm2, double mx, int64_t K) { return norm2 * 256.0 < double(K) * mx * mx; }
+
+// Rows with K contiguous, one CTA a row.  *few |= bit: a row that is not for the slices.
+__global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A, int64_t lda, int64_t K, Sliced o,
+                                                    int* few, int bit) {
   __shared__ double red[8];
   const int64_t row = blockIdx.x;
   const double* a = A + row * lda;
@@ -98,19 +104,33 @@ __global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A
   const int h = e / 2;
   const double s1 = pow2(h), s2 = pow2(e - h);
   const bool ok = un != kNotFinite;
+  double ss = 0.0;
   for (int64_t q = threadIdx.x; q < o.kt * (kKTile / 4); q += 256) {
     unsigned long long u[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int64_t k = 4 * q + j;
-      u[j] = digits(ok && k < K ? a[k] * s1 * s2 : 0.0);
+      const double y = ok && k < K ? a[k] * s1 * s2 : 0.0;
+      ss = fma(y, y, ss);
+      u[j] = digits(y);
     }
     store4(u, o.at(row, 4 * q), o.plane());
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ss = 0.0;
+    for (int w = 0; w < 8; ++w) ss += red[w];
+    if (!ok || few_large(ss, mx * s1 * s2, K)) atomicOr(few, bit);
   }
 }
 
 // Rows along the other dimension (element (r, k) at p[k ld + r]): the maxima of chunks of kStatK, then tiles
-// through shared memory; each CTA of the second kernel combines its rows' maxima itself.
+// through shared memory; each CTA of the second kernel combines its rows' maxima itself and leaves the rows' sums of
+// scaled squares over its k-tile (and, the first one, their scaled maxima) to the third.
 __global__ void __launch_bounds__(256) k_slice_max(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
                                                    double* part) {
   __shared__ double sm[8][33];
@@ -136,7 +156,8 @@ __global__ void __launch_bounds__(256) k_slice_max(const double* __restrict__ B,
 }
 
 __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
-                                                    const double* __restrict__ part, int chunks, Sliced o) {
+                                                    const double* __restrict__ part, int chunks, Sliced o,
+                                                    double* sums, double* peak) {
   __shared__ double tile[32][kKTile + 2];
   __shared__ double sm[8][33];
   __shared__ int se[32];
@@ -153,9 +174,13 @@ __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B
   if (w == 0) {
     for (int i = 1; i < 8; ++i) mx = fmax(mx, sm[i][lane]);
     int un;
-    se[lane] = scale_of(mx, &un);
+    const int e = scale_of(mx, &un), h = e / 2;
+    se[lane] = e;
     sok[lane] = un != kNotFinite;
-    if (r < R && blockIdx.x == 0) o.unscale[r] = un;
+    if (r < R && blockIdx.x == 0) {
+      o.unscale[r] = un;
+      peak[r] = mx * pow2(h) * pow2(e - h);
+    }
   }
   __syncthreads();
   for (int i = w; i < 32; i += 8) {
@@ -163,10 +188,28 @@ __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B
     const int e = se[i], h = e / 2;
     const double s1 = pow2(h), s2 = pow2(e - h);
     unsigned long long u[4];
+    double ss = 0.0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) u[j] = digits(sok[i] ? tile[i][4 * lane + j] * s1 * s2 : 0.0);
+    for (int j = 0; j < 4; ++j) {
+      const double y = sok[i] ? tile[i][4 * lane + j] * s1 * s2 : 0.0;
+      ss = fma(y, y, ss);
+      u[j] = digits(y);
+    }
     store4(u, o.at(r0 + i, k0 + 4 * lane), o.plane());
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+    if (lane == 0) sums[int64_t(blockIdx.x) * R + r0 + i] = ss;
   }
+}
+
+__global__ void __launch_bounds__(256) k_slice_few_large(const double* __restrict__ sums, const double* __restrict__ peak,
+                                                         int64_t R, int64_t K, int64_t kt, Sliced o, int* few, int bit) {
+  const int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (r >= R) return;
+  double ss = 0.0;
+#pragma unroll 8
+  for (int64_t t = 0; t < kt; ++t) ss += sums[t * R + r];
+  if (o.unscale[r] == kNotFinite || few_large(ss, peak[r], K)) atomicOr(few, bit);
 }
 
 // The l columns of B (element (k, j) at p[k ld + j]) in one launch: four columns a cluster, K cut over its CTAs, which
@@ -241,17 +284,18 @@ struct SCfg {
   static constexpr int BTILE = NB * kKTile;                      // one slice of a group
   static constexpr int BBYTES = kSlices * BTILE;
   static constexpr size_t SMEM = size_t(kARing) * kATile + 2 * size_t(BBYTES) + 1024;
-  static constexpr uint32_t TMEM = kSlices * NB <= 256 ? 256 : 512;
+  static constexpr uint32_t TMEM = kSums * NB;
+  static_assert(TMEM == 256 || TMEM == 512, "a power of two, the whole of an SM's at most");
 };
 constexpr uint32_t slice_idesc(int n) {   // kind::i8: D s32, A and B signed 8-bit, K-major, M = 128
   return (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(kTileM >> 4) << 24);
 }
 
 // A CTA: 128 rows of A, one column group, one part of K.  For every k-tile the group's seven slices of B are loaded
-// once and the seven slices of A stream past them: slice s of A times the stacked slices 0 .. 6 - s of B
-// accumulates into the sums d = s .. 6, which lie side by side in TMEM (NB columns each).  Warp 0: TMA; warp 1: MMA
-// issue; warps 4-7: the sums to FP64.  Bound by reading A's slices (7 bytes an element) and, about as much, by the
-// 28 int8 products.  Every wait is bounded.
+// once and the seven slices of A stream past them: slice s of A times the stacked slices of B up to order
+// s + t = 7 accumulates into the sums d = s .. 7, which lie side by side in TMEM (NB columns each, all of an SM's TMEM
+// for NB = 64).  Warp 0: TMA; warp 1: MMA issue; warps 4-7: the sums to FP64.  Bound by reading A's slices (7 bytes an
+// element) and, about as much, by the 34 int8 products.  Every wait is bounded.
 template <int NB>
 __global__ void __launch_bounds__(256, 1)
     slice_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, SArgs g) {
@@ -331,15 +375,20 @@ __global__ void __launch_bounds__(256, 1)
         fence_after();
         const uint32_t sa = smem_u32(smem + slot * kATile);
         constexpr int kMaxN = 256;
-        const int n = NB * (kSlices - s);
+        const int n = NB * (s == 0 ? kSlices : kSums - s);      // slice s reaches the orders s .. 7 (0: to 6)
+        // order 7 starts with slice 1, whose last NB columns are an instruction of their own in the first k-step
+        const int cut = s == 1 ? n - NB : n;
 #pragma unroll
         for (int k = 0; k < kKTile / 32; ++k) {
-          const uint32_t fresh = (kt == 0 && s == 0 && k == 0) ? 0u : 1u;
-          const int n1 = n < kMaxN ? n : kMaxN;
-          umma_i8(tmem + uint32_t(s * NB), sw128_desc(sa + k * 32), sw128_desc(sb + k * 32), slice_idesc(n1), fresh);
-          if (n > kMaxN)
-            umma_i8(tmem + uint32_t(s * NB + kMaxN), sw128_desc(sa + k * 32), sw128_desc(sb + kMaxN * kKTile + k * 32),
-                    slice_idesc(n - kMaxN), fresh);
+          auto mma = [&](int c0, int cols, uint32_t accumulate) {
+            umma_i8(tmem + uint32_t(s * NB + c0), sw128_desc(sa + k * 32), sw128_desc(sb + c0 * kKTile + k * 32),
+                    slice_idesc(cols), accumulate);
+          };
+          const bool first = kt == 0 && k == 0;
+          const uint32_t more = first && s == 0 ? 0u : 1u;
+          mma(0, cut < kMaxN ? cut : kMaxN, more);
+          if (cut > kMaxN) mma(kMaxN, cut - kMaxN, more);
+          if (cut < n) mma(cut, n - cut, first ? 0u : 1u);
         }
         umma_commit(&empty_a[slot]);
       }
@@ -367,7 +416,7 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
         for (int j = 0; j < 32; ++j) acc[j] = 0.0;
 #pragma unroll 1
-        for (int d = kSlices - 1; d >= 0; --d) {
+        for (int d = kSums - 1; d >= 0; --d) {
           uint32_t r[32];
           tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(d * NB + c), r);
 #pragma unroll
@@ -412,7 +461,7 @@ __global__ void k_slice_sum(const double* __restrict__ P, int parts, int64_t M, 
 
 size_t up(size_t b) { return (b + 1023) & ~size_t(1023); }
 
-struct ALayout { Sliced o; double* part; int64_t rows; size_t bytes; };
+struct ALayout { Sliced o; double *part, *sums, *peak; int64_t rows; size_t bytes; };
 ALayout a_layout(const SlicePlan& p, void* w) {
   ALayout a;
   a.o.kt = cdiv(p.K, kKTile);
@@ -425,6 +474,10 @@ ALayout a_layout(const SlicePlan& p, void* w) {
   off += up(size_t(p.M) * 4);
   a.part = reinterpret_cast<double*>(base + off);
   off += up(size_t(cdiv(p.K, kStatK)) * p.M * 8);
+  a.sums = reinterpret_cast<double*>(base + off);
+  off += up(size_t(a.o.kt) * p.M * 8);
+  a.peak = reinterpret_cast<double*>(base + off);
+  off += up(size_t(p.M) * 8);
   a.bytes = off + 1024;
   return a;
 }
@@ -466,20 +519,20 @@ int launch_slices(Context* c, const SlicePlan& p, const CUtensorMap& ta, const C
 // Where the line lies: three launches and the summing of the parts against the DMMA GEMM's m K l products.  One
 // iteration of the row-block integrator (Qs B and Qs' X, 48 iterations), us, DMMA -> slices:
 //     l   L     m       M K     us                   l   L     m       M K     us
-//    64   512   8000   4.1e6   107 -> 116           32  1536   4000   6.1e6    97 -> 93
-//    64   512  16000   8.2e6   164 -> 152           32  1536   8000   1.2e7   139 -> 123
-//    64  2048   4000   8.2e6   157 -> 125           12   768   8000   6.1e6    89 -> 93
-//    64  2048  16000   3.3e7   391 -> 213           12   768  16000   1.2e7   127 -> 118
-//    32   512  16000   8.2e6   101 -> 117           96   768   8000   6.1e6   186 -> 151
-//    32   512  32000   1.6e7   164 -> 159          160  1280   8000   1.0e7   389 -> 267
+//    64   512   8000   4.1e6   107 -> 116           32  1536   8000   1.2e7   137 -> 119
+//    64   512  16000   8.2e6   159 -> 154           32  1536  16000   2.5e7   200 -> 152
+//    64  2048   4000   8.2e6   171 -> 129           12   768  16000   1.2e7   132 -> 120
+//    64  2048  16000   3.3e7   409 -> 217           12   768  32000   2.5e7   200 -> 169
+//    32   512  16000   8.2e6   101 -> 117           96   768  16000   1.2e7   304 -> 216
+//    32   512  32000   1.6e7   159 -> 160          160  1280   8000   1.0e7   391 -> 285
 // so from 8e6 elements of A on, and where K or M is short (its slices leave most of a wave idle in one of the two
-// products) only with l enough for 5e8 products.
+// products) only with l enough for 6e8 products.
 SlicePlan plan_slices(const Context* c, int64_t M, int64_t K, int l) {
   SlicePlan p;
   p.M = M; p.K = K; p.l = l;
   const double mk = double(M) * double(K);
   if (l < 1 || M < 256 || K < 512 || mk < 8e6) return p;
-  if (std::min(M, K) < 768 && mk * l < 5e8) return p;
+  if (std::min(M, K) < 768 && mk * l < 6e8) return p;
   p.nb = l <= 32 ? 32 : 64;
   p.groups = int(cdiv(l, p.nb));
   const int64_t sms = c ? c->num_sms : 148;
@@ -500,22 +553,32 @@ SlicePlan plan_slices(const Context* c, int64_t M, int64_t K, int l) {
   return p;
 }
 
-int slice_a(Context* c, const SlicePlan& p, CMat A, void* aw) {
+int slice_a(Context* c, const SlicePlan& p, CMat A, void* aw, int bit) {
   if (!p.use || !aw) return MCNLA_B200_ERR_ARG;
+  int* few = &c->scal->slice_few;
   const ALayout a = a_layout(p, aw);
   if (A.cs == 1) {
-    k_slice_rows<<<unsigned(p.M), 256, 0, c->stream>>>(A.p, A.rs, p.K, a.o);
+    k_slice_rows<<<unsigned(p.M), 256, 0, c->stream>>>(A.p, A.rs, p.K, a.o, few, bit);
     c->kernels_launched++;
   } else if (A.rs == 1) {
     const int chunks = int(cdiv(p.K, kStatK));
     k_slice_max<<<dim3(unsigned(cdiv(p.M, 32)), unsigned(chunks)), 256, 0, c->stream>>>(A.p, A.cs, p.M, p.K, a.part);
     k_slice_cols<<<dim3(unsigned(a.o.kt), unsigned(cdiv(p.M, 32))), 256, 0, c->stream>>>(A.p, A.cs, p.M, p.K, a.part,
-                                                                                       chunks, a.o);
-    c->kernels_launched += 2;
+                                                                                       chunks, a.o, a.sums, a.peak);
+    k_slice_few_large<<<unsigned(cdiv(p.M, 256)), 256, 0, c->stream>>>(a.sums, a.peak, p.M, p.K, a.o.kt, a.o, few, bit);
+    c->kernels_launched += 3;
   } else {
     return MCNLA_B200_ERR_LAYOUT;
   }
   MB_CHECK_CUDA(cudaGetLastError());
+  return MCNLA_B200_OK;
+}
+
+int slice_bits(Context* c, int* bits) {
+  MB_CHECK_CUDA(cudaMemcpyAsync(&c->scal_host->slice_few, &c->scal->slice_few, sizeof(int), cudaMemcpyDeviceToHost,
+                                c->stream));
+  MB_CHECK_CUDA(cudaStreamSynchronize(c->stream));
+  *bits = c->scal_host->slice_few;
   return MCNLA_B200_OK;
 }
 

@@ -1,5 +1,5 @@
 """The loops' int8-slice products (csrc/slice_gemm.cu) on bases outside the dense, evenly scaled ones: rows of any finite
-magnitude."""
+magnitude, and rows and columns in which few entries dominate."""
 import pytest
 import torch
 
@@ -57,3 +57,20 @@ def test_solve_with_a_tiny_row(cuda, integrator):
     assert it == it0 and all(bool(torch.isfinite(x).all()) for x in (s, u, v))
     assert float(((s - s0) / s0).abs().max()) < 1e-12
     assert 1e-140 < float(u[77].abs().max()) < 1e-125
+
+
+@pytest.mark.parametrize("rest", [1e-5, 1e-7])
+@pytest.mark.parametrize("cls", ["KolmogorovNagumoIntegrator", "RowBlockKolmogorovNagumoIntegrator"])
+def test_columns_of_one_dominating_entry(cuda, cls, rest):
+    """Bases of a matrix with localized singular vectors.  Against the definition in FP64 the two differ by a few
+    roundings of every product's result an iteration: 8 maxit 2^-53 ||Qbar||_F, ||Qbar||_F = sqrt(l)."""
+    m, l, N, maxit = 16384, 48, 16, 12
+    g = torch.Generator(device=cuda)
+    g.manual_seed(1)
+    base = rest * torch.randn(m, l, generator=g, dtype=torch.float64, device=cuda)
+    base[torch.randperm(m, generator=g, device=cuda)[:l], torch.arange(l, device=cuda)] = 1.0
+    q = _orth(base[None] + 0.1 * rest * torch.randn(N, m, l, generator=g, dtype=torch.float64, device=cuda))
+    qbar, it = _integrate(cls, q, l, N, maxit, 0.0)
+    ref, itr = _kn(q, l, N, maxit, 0.0)
+    assert it == itr
+    assert float((qbar - ref).norm()) < 8 * maxit * 2.0 ** -53 * l ** 0.5
