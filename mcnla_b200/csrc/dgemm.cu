@@ -33,19 +33,8 @@ struct KArgs {
   const int* guard_stop;   // skip the launch when *guard_stop < guard_it
   int guard_it;
   int lower;               // 1: only tiles touching the lower triangle (row >= column) are computed
-  GemmFlags fl;            // the FLAGGED kernels: only elements with a flagged row or column (batch 1)
+  GemmFlags fl;            // the FLAGGED kernels: only the flagged tiles (batch 1)
 };
-
-// Whether a tile holds a flagged row or column (block-uniform).
-__device__ __forceinline__ bool tile_flagged(const GemmFlags& fl, int64_t m0, int bm, int64_t M, int64_t n0, int bn,
-                                             int64_t N) {
-  int any = 0;
-  for (int i = threadIdx.x; i < bm + bn; i += blockDim.x) {
-    if (i < bm) any |= m0 + i < M && fl.row[m0 + i];
-    else any |= n0 + i - bm < N && fl.col[n0 + i - bm];
-  }
-  return __syncthreads_or(any) != 0;
-}
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
   unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -143,8 +132,7 @@ struct TileLoader {
   }
 };
 
-// FLAGGED: a product restricted by g.fl.  A kernel of its own: the two tests in the epilogue cost the ordinary
-// one 8-15 %.
+// FLAGGED: a product restricted by g.fl, whose tiles are whole multiples of this kernel's.
 template <class C, bool FLAGGED>
 __global__ void __launch_bounds__(C::THREADS) dgemm_kernel(KArgs g) {
   extern __shared__ __align__(16) double smem[];
@@ -157,7 +145,8 @@ __global__ void __launch_bounds__(C::THREADS) dgemm_kernel(KArgs g) {
   const int64_t n0 = int64_t(blockIdx.x) * C::BN;
   const int64_t m0 = int64_t(blockIdx.y) * C::BM;
   if (g.lower && n0 >= m0 + C::BM) return;        // every element of the tile has column > row
-  if (FLAGGED && (*g.fl.any == 0 || !tile_flagged(g.fl, m0, C::BM, g.M, n0, C::BN, g.N))) return;
+  static_assert(!FLAGGED || (kFlagRows % C::BM == 0 && kFlagCols % C::BN == 0), "a tile is flagged as a whole");
+  if (FLAGGED && !g.fl.tile[m0 / kFlagRows * g.fl.nt + n0 / kFlagCols]) return;
   const int bz = blockIdx.z / g.splits;
   const int split = blockIdx.z % g.splits;
   const double* A = g.A + bz * g.a_bs;
@@ -239,7 +228,6 @@ __global__ void __launch_bounds__(C::THREADS) dgemm_kernel(KArgs g) {
       for (int h = 0; h < 2; ++h) {
         const int64_t col = n0 + wn * C::WN + j * 8 + 2 * t4 + h;
         if (col >= g.N) continue;
-        if (FLAGGED && !g.fl.row[row] && !g.fl.col[col]) continue;
         if (g.splits == 1) {
           double* cp = Cb + row * g.c_rs + col * g.c_cs;
           double v = g.alpha * acc[i][j][h];
@@ -265,7 +253,7 @@ __global__ void splitk_reduce_kernel(const double* ws, int splits, int batch, in
     const int64_t b = idx / MN, e = idx % MN;
     const int64_t r = e / N, c = e % N;
     if (lower && c > r) continue;
-    if (fl.any && !fl.row[r] && !fl.col[c]) continue;
+    if (fl.any && !fl.tile[r / kFlagRows * fl.nt + c / kFlagCols]) continue;
     const double* w = ws + b * splits * MN + e;
     double s = 0.0;
     for (int k = 0; k < splits; ++k) s += w[k * MN];

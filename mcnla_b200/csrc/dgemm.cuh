@@ -21,11 +21,12 @@ struct GemmBatch {
   int64_t a = 0, b = 0, c = 0;   // element strides between batch members
 };
 
-// Restricts a product to the elements whose row or whose column is flagged (device arrays, one byte each);
-// *any == 0: none is.  Element values are those of the unrestricted product.
+// Restricts a product to its flagged tiles (a device array of one byte a tile of kFlagRows x kFlagCols elements, row by
+// row, nt tiles a row); *any == 0: none is.  Element values are those of the unrestricted product.
+constexpr int kFlagRows = 128, kFlagCols = 256;
 struct GemmFlags {
-  const uint8_t* row = nullptr;
-  const uint8_t* col = nullptr;
+  const uint8_t* tile = nullptr;
+  int64_t nt = 0;
   const int* any = nullptr;
 };
 
@@ -41,7 +42,7 @@ int dgemm_heuristic_splits(const Context* c, int64_t M, int64_t N, int64_t K, in
 // (tests use it to cover the split-K path at small sizes).  lower_only: C is
 // square and only its lower triangle is needed (SYRK-like: tiles strictly
 // above the diagonal are skipped and the elements above it are unspecified).  flags: only
-// the flagged elements are computed and written.
+// the flagged tiles are computed and written.
 int dgemm(Context* ctx, int64_t M, int64_t N, int64_t K, double alpha, CMat A, CMat B, double beta, DMat C,
           GemmBatch batch = GemmBatch(), double* ws = nullptr, int force_splits = 0, bool lower_only = false,
           const GemmFlags* flags = nullptr);

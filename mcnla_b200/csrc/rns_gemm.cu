@@ -1,8 +1,8 @@
 // FP64 products through int8 tensor-core residue products (see rns.cuh).
 //
-// Four kernels: the residues of A's rows and of B's columns (K-contiguous int8 planes, one per
-// modulus), the int8 GEMMs of all moduli in one persistent launch (tcgen05 kind::i8),
-// and the CRT back to FP64; then the DMMA GEMM on what was flagged.
+// The scales of A's rows and of B's columns, which also say which tiles of C the DMMA GEMM takes; then for the other
+// tiles the residues (K-contiguous int8 planes, one per modulus), the int8 GEMMs of all moduli in one persistent
+// launch (tcgen05 kind::i8), and the CRT back to FP64; then the DMMA GEMM on the flagged tiles.
 #include "rns.cuh"
 #include "rns_math.cuh"
 #include "tma.cuh"
@@ -20,6 +20,7 @@ __constant__ rns::Tables kT = rns::make_tables();
 constexpr int kKTile = 128;                 // K of a shared-memory tile: one 128-byte swizzle row
 constexpr int64_t kMaxChunk = 131071;       // 32-bit sums of products of two signed bytes
 constexpr int kTileM = 128, kTileN = 256;    // output tile of a CTA
+static_assert(kTileM == kFlagRows && kTileN == kFlagCols, "the DMMA GEMM takes whole tiles");
 constexpr double kMaxScale = 0x1p800, kMinScale = 0x1p-800;   // squares: entries within 2^+-400
 
 __device__ __forceinline__ double pow2(int e) {   // |e| < 1023
@@ -58,38 +59,55 @@ struct Out {
   uint8_t* planes;        // [modulus][row][kp]
   int64_t rows_pad;       // rows per plane
   int64_t kp;             // bytes per row: K rounded up to kKTile, zero past K
-  double* unscale;        // per row: 2^-s
-  uint8_t* flag;          // per row: 1 when the DMMA path takes it (never cleared here)
-  int* any;
+  const uint8_t* live;    // per 1 << live_shift rows: 0 when every tile of theirs is the DMMA path's
+  int live_shift;
 };
 
-// Residues of the rows of a K-contiguous matrix, one CTA per row: the norm, then the row again (from
-// L2) into the planes.  Bound by the integer pipe: ~100 instructions an element (15 residues of a 64-bit
-// integer, two dp4a and a division by rounding each) against 8 bytes read and 15 written.
+// Per row: the scale, what undoes it, and whether the DMMA path takes the row's tiles (never cleared here).
+struct Scales {
+  int* scale;             // exponent; kFlagged
+  double* unscale;        // 2^-scale
+  uint8_t* flag;
+};
+constexpr int kFlagged = INT32_MIN;
+
+__device__ __forceinline__ void put_scale(const Scales& o, int64_t row, double norm2, double mx, int64_t K, int target) {
+  bool bad;
+  const int e = scale_of(norm2, mx, K, target, &bad);
+  o.scale[row] = bad ? kFlagged : e;
+  o.unscale[row] = pow2(-e);
+  if (bad) o.flag[row] = 1;
+}
+
 constexpr int kRowThreads = 256;
-template <bool VEC, bool IS_B>
-__global__ void __launch_bounds__(kRowThreads) k_rns_rows(const double* __restrict__ A, int64_t lda, int64_t K,
-                                                          int target, Out o) {
+template <bool VEC>
+__device__ __forceinline__ void load_quad(const double* a, int64_t q, int64_t K, double (&x)[4]) {
+  const int64_t k = 4 * q;
+  if (VEC && k + 4 <= K) {
+    const double2 p0 = *reinterpret_cast<const double2*>(a + k), p1 = *reinterpret_cast<const double2*>(a + k + 2);
+    x[0] = p0.x; x[1] = p0.y; x[2] = p1.x; x[3] = p1.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = k + j < K ? a[k + j] : 0.0;
+  }
+}
+
+// Scales of the rows of a K-contiguous matrix, one CTA per row.  A pass of its own, so that which tiles are the
+// DMMA path's is known before any row is converted: with a norm and a conversion in one kernel, a matrix with a sparse
+// row in every 64 took 1.3 times as long as by the DMMA GEMM alone.  HBM-bound.
+template <bool VEC>
+__global__ void __launch_bounds__(kRowThreads) k_rns_rowscale(const double* __restrict__ A, int64_t lda, int64_t K,
+                                                              int target, Scales o) {
   __shared__ double red_s[kRowThreads / 32], red_m[kRowThreads / 32];
-  __shared__ int scale_s;
   const int64_t row = blockIdx.x;
   const double* a = A + row * lda;
   const int tid = threadIdx.x;
   double s = 0.0, mx = 0.0;
   const int64_t quads = (K + 3) / 4;
-  auto load = [&](int64_t q, double (&x)[4]) {
-    const int64_t k = 4 * q;
-    if (VEC && k + 4 <= K) {
-      const double2 p0 = *reinterpret_cast<const double2*>(a + k), p1 = *reinterpret_cast<const double2*>(a + k + 2);
-      x[0] = p0.x; x[1] = p0.y; x[2] = p1.x; x[3] = p1.y;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) x[j] = k + j < K ? a[k + j] : 0.0;
-    }
-  };
+#pragma unroll 2
   for (int64_t q = tid; q < quads; q += kRowThreads) {
     double x[4];
-    load(q, x);
+    load_quad<VEC>(a, q, K, x);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       s = fma(x[j], x[j], s);      // NaN and infinities reach the sum
@@ -105,19 +123,26 @@ __global__ void __launch_bounds__(kRowThreads) k_rns_rows(const double* __restri
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < kRowThreads / 32; ++w) { s += red_s[w]; mx = fmax(mx, red_m[w]); }
-    bool bad;
-    const int e = scale_of(s, mx, K, target, &bad);
-    scale_s = bad ? INT32_MIN : e;
-    o.unscale[row] = pow2(-e);
-    if (bad) { o.flag[row] = 1; *o.any = 1; }
+    put_scale(o, row, s, mx, K, target);
   }
-  __syncthreads();
-  const int e = scale_s;
-  if (e == INT32_MIN) return;      // its planes' bytes are not used
+}
+
+// Residues of the rows of a K-contiguous matrix, one CTA per row.  Bound by the integer pipe: ~100 instructions an
+// element (15 residues of a 64-bit integer, two dp4a and a division by rounding each) against 8 bytes read and 15
+// written.
+template <bool VEC, bool IS_B>
+__global__ void __launch_bounds__(kRowThreads) k_rns_rows(const double* __restrict__ A, int64_t lda, int64_t K,
+                                                          const int* __restrict__ scale, Out o) {
+  const int64_t row = blockIdx.x;
+  if (o.live && !o.live[row >> o.live_shift]) return;
+  const int e = scale[row];
+  if (e == kFlagged) return;       // its planes' bytes are not used
+  const double* a = A + row * lda;
+  const int64_t quads = (K + 3) / 4;
   double s1, s2;
   split_scale(e, &s1, &s2);
   const int64_t plane = o.rows_pad * o.kp;
-  for (int64_t q = tid; q < o.kp / 4; q += kRowThreads) {
+  for (int64_t q = threadIdx.x; q < o.kp / 4; q += kRowThreads) {
     uint32_t* w = reinterpret_cast<uint32_t*>(o.planes + row * o.kp) + q;
     if (q >= quads) {
 #pragma unroll
@@ -125,7 +150,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rns_rows(const double* __restri
       continue;
     }
     double x[4];
-    load(q, x);
+    load_quad<VEC>(a, q, K, x);
     uint64_t u[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) u[j] = to_int(x[j], s1, s2);   // past K: zero, whose residues are zero
@@ -163,7 +188,7 @@ __global__ void __launch_bounds__(256) k_rns_colstats(const double* __restrict__
   }
 }
 
-__global__ void k_rns_colscale(const double* part, int64_t R, int64_t K, int chunks, int target, int* scale, Out o) {
+__global__ void k_rns_colscale(const double* part, int64_t R, int64_t K, int chunks, int target, Scales o) {
   const int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (r >= R) return;
   double s = 0.0, mx = 0.0;
@@ -171,11 +196,35 @@ __global__ void k_rns_colscale(const double* part, int64_t R, int64_t K, int chu
     s += part[2 * int64_t(c) * R + r];
     mx = fmax(mx, part[(2 * int64_t(c) + 1) * R + r]);
   }
-  bool bad;
-  const int e = scale_of(s, mx, K, target, &bad);
-  scale[r] = bad ? INT32_MIN : e;
-  o.unscale[r] = pow2(-e);
-  if (bad) { o.flag[r] = 1; *o.any = 1; }
+  put_scale(o, r, s, mx, K, target);
+}
+
+// The tiles that the DMMA path takes: those with a flagged row or column (added to what an earlier chunk of K flagged),
+// whole, since a tile costs either path the same whatever it holds.  One CTA per panel of kTileM rows; live[panel]: a
+// tile is left to the int8 path, any_live: to any panel.  lower: tiles above the diagonal count for nothing.
+__global__ void __launch_bounds__(kTileN) k_rns_tiles(const uint8_t* __restrict__ row_flag,
+                                                      const uint8_t* __restrict__ col_flag, int64_t M, int64_t N,
+                                                      int lower, uint8_t* tile, uint8_t* live, uint8_t* any_live,
+                                                      int* any) {
+  const int64_t panel = blockIdx.x, r = panel * kTileM + threadIdx.x;
+  const int nt = int((N + kTileN - 1) / kTileN);
+  const int row_bad = __syncthreads_or(threadIdx.x < kTileM && r < M && row_flag[r]);
+  bool alive = false, bad = false;
+  for (int t = 0; t < nt; ++t) {
+    const int64_t c = int64_t(t) * kTileN + threadIdx.x;
+    const int col_bad = __syncthreads_or(c < N && col_flag[c]);
+    uint8_t* p = tile + panel * nt + t;
+    const bool dmma = row_bad || col_bad || *p;
+    __syncthreads();
+    if (threadIdx.x == 0 && dmma) *p = 1;
+    if (lower && int64_t(t) * kTileN >= (panel + 1) * kTileM) continue;
+    alive |= !dmma;
+    bad |= dmma;
+  }
+  if (threadIdx.x != 0) return;
+  live[panel] = alive;
+  if (alive) *any_live = 1;
+  if (bad) *any = 1;
 }
 
 constexpr int kColTile = 32;
@@ -185,6 +234,7 @@ __global__ void __launch_bounds__(256) k_rns_cols(const double* __restrict__ B, 
   __shared__ double tile[kColTile][kKTile + 2];   // [row][k]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t r0 = int64_t(blockIdx.y) * kColTile, k0 = int64_t(blockIdx.x) * kKTile;
+  if (o.live && !o.live[r0 >> o.live_shift]) return;
   const int64_t r = r0 + lane;
   for (int k = w; k < kKTile; k += 8) tile[lane][k] = (r < R && k0 + k < K) ? B[(k0 + k) * ld + r] : 0.0;
   __syncthreads();
@@ -193,7 +243,7 @@ __global__ void __launch_bounds__(256) k_rns_cols(const double* __restrict__ B, 
     const int64_t row = r0 + i;
     if (row >= R) break;
     const int e = scale[row];
-    if (e == INT32_MIN) continue;
+    if (e == kFlagged) continue;
     double s1, s2;
     split_scale(e, &s1, &s2);
     uint64_t u[4];
@@ -218,10 +268,7 @@ struct GemmArgs {
   int64_t jobs;
   uint8_t* y;                       // [modulus][y_rows][ldy] digits
   int64_t y_rows, ldy;
-  const uint8_t* row_flag;          // rows of A / columns of B that the DMMA path takes
-  const uint8_t* col_flag;
-  const int* any;
-  int M, N;                         // valid rows and columns
+  const uint8_t* tile;              // [mt][nt]: tiles that the DMMA path takes
   int* status;
 };
 
@@ -247,17 +294,9 @@ __device__ __forceinline__ bool job_of(const GemmArgs& g, int64_t j, Job* out) {
   return !(g.lower && int64_t(out->n) * kTileN >= g.a_row0 + int64_t(out->m + 1) * kTileM);
 }
 
-// Whether every row or every column of a tile goes to the DMMA path (all threads of a warp call it).
+// Whether the DMMA path takes a tile (the same on all threads).
 __device__ __forceinline__ bool tile_unused(const GemmArgs& g, const Job& jb) {
-  if (*g.any == 0) return false;
-  const int lane = threadIdx.x & 31;
-  bool rows = true, cols = true;
-  for (int i = lane; i < kTileN; i += 32) {
-    const int r = jb.m * kTileM + i, c = jb.n * kTileN + i;
-    if (i < kTileM && r < g.M && !g.row_flag[r]) rows = false;
-    if (c < g.N && !g.col_flag[c]) cols = false;
-  }
-  return __all_sync(0xffffffffu, rows) || __all_sync(0xffffffffu, cols);
+  return g.tile[int64_t(jb.m) * g.nt + jb.n] != 0;
 }
 
 // A CTA computes 128 x 256 tiles of every modulus' product.  Warp 0: TMA into the ring of 48 KB stages; warp 1: MMA
@@ -420,12 +459,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 __global__ void __launch_bounds__(256) k_rns_crt(const uint8_t* __restrict__ y, int64_t y_rows, int64_t ldy, int64_t M,
                                                  int64_t N, const double* __restrict__ ua,
                                                  const double* __restrict__ ub, double* C, int64_t ldc, int add,
-                                                 int64_t lower_row0, const uint8_t* __restrict__ row_flag) {
+                                                 int64_t lower_row0, const uint8_t* __restrict__ tile, int nt) {
   const int64_t row = blockIdx.y;
-  if (row_flag[row]) return;
   const int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   const int64_t col = 4 * q;
-  if (col >= N || (lower_row0 >= 0 && col > lower_row0 + row)) return;
+  if (col >= N || (lower_row0 >= 0 && col > lower_row0 + row) || tile[row / kTileM * nt + col / kTileN]) return;
   const uint8_t* src = y + row * ldy + col;
   const int64_t plane = y_rows * ldy;
   rns::Crt acc[4];
@@ -450,10 +488,11 @@ __global__ void __launch_bounds__(256) k_rns_crt(const uint8_t* __restrict__ y, 
 
 // ---- host
 struct Work {   // workspace layout
-  uint8_t *pa, *pb, *y, *row_flag, *col_flag;
+  uint8_t *pa, *pb, *y, *row_flag, *col_flag, *tile, *live, *any_live;
   double *ua, *ub, *part;
   int *scale, *any;
-  int64_t a_pad, b_pad, kp, y_rows, ldy;
+  int64_t a_pad, b_pad, kp, y_rows, ldy, nt;
+  size_t block_flags, flags;   // bytes from `any` on: of a call's rows, and with the columns'
   size_t bytes;
 };
 
@@ -464,6 +503,7 @@ Work layout(const RnsPlan& p, void* ws) {
   w.kp = cdiv(p.kc, kKTile) * kKTile;
   w.a_pad = cdiv(p.mb, kTileM) * kTileM;
   w.b_pad = cdiv(p.N, kTileN) * kTileN;
+  w.nt = cdiv(p.N, kTileN);
   w.y_rows = w.a_pad;
   w.ldy = w.b_pad;
   char* base = static_cast<char*>(ws);
@@ -474,36 +514,49 @@ Work layout(const RnsPlan& p, void* ws) {
   w.y = reinterpret_cast<uint8_t*>(take(size_t(kRnsModuli) * w.y_rows * w.ldy));
   const int64_t most = std::max(p.M, p.N);
   w.part = reinterpret_cast<double*>(take(size_t(2 * cdiv(p.kc, kStatK)) * most * 8));   // of strided operands
-  w.scale = reinterpret_cast<int*>(take(size_t(most) * 4));
+  w.scale = reinterpret_cast<int*>(take(size_t(p.N + p.M) * 4));                          // B's, then A's
   w.ub = reinterpret_cast<double*>(take(size_t(p.N) * 8));
   w.ua = p.same ? w.ub : reinterpret_cast<double*>(take(size_t(p.M) * 8));
-  // one memset clears these
-  w.any = reinterpret_cast<int*>(take(up(sizeof(int)) + up(size_t(w.b_pad)) + (p.same ? 0 : up(size_t(p.M)))));
-  w.col_flag = reinterpret_cast<uint8_t*>(w.any) + up(sizeof(int));
-  w.row_flag = p.same ? w.col_flag : w.col_flag + up(size_t(w.b_pad));
+  w.live = reinterpret_cast<uint8_t*>(take(size_t(cdiv(p.M, kTileM))));
+  // cleared together, the columns' flags only where B is new
+  const size_t off0 = off;
+  w.any = reinterpret_cast<int*>(take(2 * sizeof(int)));
+  w.any_live = reinterpret_cast<uint8_t*>(w.any + 1);
+  w.tile = reinterpret_cast<uint8_t*>(take(size_t(cdiv(p.M, kTileM) * w.nt)));
+  if (!p.same) w.row_flag = reinterpret_cast<uint8_t*>(take(size_t(p.M)));
+  w.block_flags = off - off0;
+  w.col_flag = reinterpret_cast<uint8_t*>(take(size_t(w.b_pad)));
+  if (p.same) w.row_flag = w.col_flag;
+  w.flags = off - off0;
   w.bytes = off;
   return w;
 }
 
-// Scales of R rows whose k runs along the other dimension (element (r, k) at x.p[r + k x.cs]).
-int strided_scales(Context* c, CMat x, int64_t R, int64_t K, bool is_b, const Work& w, const Out& o) {
-  const int chunks = int(cdiv(K, kStatK));
-  k_rns_colstats<<<dim3(unsigned(cdiv(R, 32)), unsigned(chunks)), 256, 0, c->stream>>>(x.p, x.cs, R, K, w.part);
-  k_rns_colscale<<<unsigned(cdiv(R, 256)), 256, 0, c->stream>>>(w.part, R, K, chunks, is_b ? rns::kTB : rns::kTA,
-                                                                w.scale, o);
-  c->kernels_launched += 2;
+// Scales of R rows (element (r, k) at x.p[r x.rs + k x.cs]).
+int scales(Context* c, CMat x, int64_t R, int64_t K, bool is_b, double* part, const Scales& o) {
+  const int target = is_b ? rns::kTB : rns::kTA;
+  if (x.cs == 1) {
+    const bool vec = (reinterpret_cast<uintptr_t>(x.p) & 15) == 0 && x.rs % 2 == 0;
+    auto kern = vec ? k_rns_rowscale<true> : k_rns_rowscale<false>;
+    kern<<<unsigned(R), kRowThreads, 0, c->stream>>>(x.p, x.rs, K, target, o);
+    c->kernels_launched++;
+  } else {
+    const int chunks = int(cdiv(K, kStatK));
+    k_rns_colstats<<<dim3(unsigned(cdiv(R, 32)), unsigned(chunks)), 256, 0, c->stream>>>(x.p, x.cs, R, K, part);
+    k_rns_colscale<<<unsigned(cdiv(R, 256)), 256, 0, c->stream>>>(part, R, K, chunks, target, o);
+    c->kernels_launched += 2;
+  }
   MB_CHECK_CUDA(cudaGetLastError());
   return MCNLA_B200_OK;
 }
 
-// Residues of R rows (element (r, k) at x.p[r x.rs + k x.cs]); strided ones have their scales already, in `scale`.
-// is_b: B's, which carry the CRT's factors.
+// Residues of R rows with their scales.  is_b: B's, which carry the CRT's factors.
 int residues(Context* c, CMat x, int64_t R, int64_t K, bool is_b, const int* scale, const Out& o) {
   if (x.cs == 1) {
     const bool vec = (reinterpret_cast<uintptr_t>(x.p) & 15) == 0 && x.rs % 2 == 0;
     auto kern = vec ? (is_b ? k_rns_rows<true, true> : k_rns_rows<true, false>)
                     : (is_b ? k_rns_rows<false, true> : k_rns_rows<false, false>);
-    kern<<<unsigned(R), kRowThreads, 0, c->stream>>>(x.p, x.rs, K, is_b ? rns::kTB : rns::kTA, o);
+    kern<<<unsigned(R), kRowThreads, 0, c->stream>>>(x.p, x.rs, K, scale, o);
   } else {
     auto kern = is_b ? k_rns_cols<true> : k_rns_cols<false>;
     kern<<<dim3(unsigned(o.kp / kKTile), unsigned(cdiv(R, kColTile))), 256, 0, c->stream>>>(x.p, x.cs, R, K, scale, o);
@@ -528,6 +581,7 @@ int residues(Context* c, CMat x, int64_t R, int64_t K, bool is_b, const int* sca
 RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, int64_t max_rows) {
   RnsPlan p;
   p.M = M; p.N = N; p.K = K; p.same = same;
+  p.streamed = max_rows > 0;
   if (M < 1 || N < 1 || K < 1) return p;
   const double m = double(M), n = double(N), k = double(K), half = same ? 0.5 : 1.0;
   const double n128 = double(cdiv(N, 128)) * 128.0;
@@ -578,10 +632,8 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
   if (rows < 1 || rows > plan.M || (plan.same && rows != plan.N)) return MCNLA_B200_ERR_SHAPE;
   const Work w = layout(plan, reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~uintptr_t(1023)));
   const bool keep_b = reuse_b && plan.chunks == 1 && !plan.same;
-  // `any` and the flags collect over chunks and blocks; a kept B keeps its own flags
-  if (keep_b) MB_CHECK_CUDA(cudaMemsetAsync(w.row_flag, 0, size_t(rows), c->stream));
-  else MB_CHECK_CUDA(cudaMemsetAsync(w.any, 0, up(sizeof(int)) + up(size_t(w.b_pad)) + (plan.same ? 0 : size_t(rows)),
-                                     c->stream));
+  // the flags collect over chunks and blocks; a kept B keeps its own
+  MB_CHECK_CUDA(cudaMemsetAsync(w.any, 0, keep_b ? w.block_flags : w.flags, c->stream));
   static std::atomic<uint64_t> attr_set{0};   // the shared-memory opt-in: one bit per device
   const uint64_t bit = uint64_t(1) << (c->device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & bit)) {
@@ -591,24 +643,29 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
   for (int ch = 0; ch < plan.chunks; ++ch) {
     const int64_t k0 = ch * plan.kc, kn = std::min(plan.kc, plan.K - k0);
     const int64_t kp = cdiv(kn, kKTile) * kKTile;
-    if (!keep_b) {
-      const Out ob{w.pb, w.b_pad, kp, w.ub, w.col_flag, w.any};
-      const CMat b = cm(B.p + k0 * B.rs, B.cs, B.rs);
-      if (b.cs != 1) MB_CHECK(strided_scales(c, b, plan.N, kn, !plan.same, w, ob));
-      MB_CHECK(residues(c, b, plan.N, kn, !plan.same, w.scale, ob));
-    }
-    // A's strided scales: all rows at once (after B's residues, which share the scratch)
     const CMat ak = cm(A.p + k0 * A.cs, A.rs, A.cs);
-    const bool strided = !plan.same && A.cs != 1;
-    if (strided) MB_CHECK(strided_scales(c, ak, rows, kn, false, w, Out{nullptr, 0, kp, w.ua, w.row_flag, w.any}));
+    const CMat bk = cm(B.p + k0 * B.rs, B.cs, B.rs);
+    int* const sb = w.scale;
+    int* const sa = plan.same ? sb : w.scale + plan.N;
+    if (!keep_b) MB_CHECK(scales(c, bk, plan.N, kn, !plan.same, w.part, Scales{sb, w.ub, w.col_flag}));
+    if (!plan.same) MB_CHECK(scales(c, ak, rows, kn, false, w.part, Scales{sa, w.ua, w.row_flag}));
+    k_rns_tiles<<<unsigned(cdiv(rows, kTileM)), kTileN, 0, c->stream>>>(
+        w.row_flag, w.col_flag, rows, plan.N, plan.same ? 1 : 0, w.tile, w.live, w.any_live, w.any);
+    MB_CHECK_CUDA(cudaGetLastError());
+    c->kernels_launched++;
+    // a B that later blocks of rows will keep is converted whatever this block needs
+    if (!keep_b)
+      MB_CHECK(residues(c, bk, plan.N, kn, !plan.same, sb,
+                        Out{w.pb, w.b_pad, kp, plan.streamed ? nullptr : w.any_live, 31}));
     CUtensorMap tb;
     MB_CHECK(make_map_u8(&tb, w.pb, kRnsModuli * w.b_pad, kp, kp, kKTile, kTileN));
     for (int64_t r0 = 0; r0 < rows; r0 += plan.mb) {
       const int64_t rn = std::min(plan.mb, rows - r0);
       CUtensorMap ta;
       if (!plan.same) {
-        const Out oa{w.pa, w.a_pad, kp, w.ua + r0, w.row_flag + r0, w.any};
-        MB_CHECK(residues(c, cm(ak.p + r0 * A.rs, A.rs, A.cs), rn, kn, false, w.scale + r0, oa));
+        static_assert(kTileM == 1 << 7, "a panel's rows");
+        MB_CHECK(residues(c, cm(ak.p + r0 * A.rs, A.rs, A.cs), rn, kn, false, sa + r0,
+                          Out{w.pa, w.a_pad, kp, w.live + r0 / kTileM, 7}));
         MB_CHECK(make_map_u8(&ta, w.pa, kRnsModuli * w.a_pad, kp, kp, kKTile, kTileM));
       } else {
         MB_CHECK(make_map_u8(&ta, w.pb, kRnsModuli * w.b_pad, kp, kp, kKTile, kTileM));
@@ -625,26 +682,22 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
       g.y = w.y;
       g.y_rows = w.y_rows;
       g.ldy = w.ldy;
-      g.row_flag = w.row_flag + r0;
-      g.col_flag = w.col_flag;
-      g.any = w.any;
-      g.M = int(rn);
-      g.N = int(plan.N);
+      g.tile = w.tile + r0 / kTileM * w.nt;
       g.status = &c->scal->wait_status;
       const unsigned ctas = unsigned(std::min<int64_t>(g.jobs, c->num_sms));
       rns_gemm_kernel<<<ctas, kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
       MB_CHECK_CUDA(cudaGetLastError());
       k_rns_crt<<<dim3(unsigned(cdiv(plan.N, 1024)), unsigned(rn)), 256, 0, c->stream>>>(
           w.y, w.y_rows, w.ldy, rn, plan.N, w.ua + r0, w.ub, C.p + r0 * C.rs, C.rs, ch > 0,
-          plan.same ? r0 : -1, w.row_flag + r0);
+          plan.same ? r0 : -1, g.tile, g.nt);
       MB_CHECK_CUDA(cudaGetLastError());
       c->kernels_launched += 2;
     }
   }
   // what was flagged, over the whole K
   GemmFlags fl;
-  fl.row = w.row_flag;
-  fl.col = w.col_flag;
+  fl.tile = w.tile;
+  fl.nt = w.nt;
   fl.any = w.any;
   return dgemm(c, rows, plan.N, plan.K, 1.0, A, B, 0.0, C, GemmBatch(), dws, splits, plan.same, &fl);
 }

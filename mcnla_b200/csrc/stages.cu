@@ -1229,8 +1229,10 @@ struct RowBlocks {
 RowBlocks stream_blocks(Context* c, const Dims& d) {
   const size_t row_bytes = size_t(d.n) * sizeof(double);
   RowBlocks rb;
-  rb.rows_per = std::max<int64_t>(128, std::min<int64_t>(int64_t((size_t(1) << 30) / row_bytes), cdiv(d.m, 4)));
-  rb.first = std::min<int64_t>(rb.rows_per, std::max<int64_t>(128, int64_t((size_t(128) << 20) / row_bytes)));
+  // blocks start on whole tiles of the int8 product
+  auto aligned = [](int64_t rows) { return std::max<int64_t>(1, rows / kRnsRowAlign) * kRnsRowAlign; };
+  rb.rows_per = aligned(std::min<int64_t>(int64_t((size_t(1) << 30) / row_bytes), cdiv(d.m, 4)));
+  rb.first = std::min<int64_t>(rb.rows_per, aligned(int64_t((size_t(128) << 20) / row_bytes)));
   rb.nblocks = 1 + int(cdiv(std::max<int64_t>(0, d.m - rb.first), rb.rows_per));
   rb.splits = dgemm_heuristic_splits(c, d.m, d.L, d.n, 1);
   rb.rns = plan_rns(c, d.m, d.L, d.n, false, rb.rows_per);

@@ -74,3 +74,65 @@ def test_columns_of_one_dominating_entry(cuda, cls, rest):
     ref, itr = _kn(q, l, N, maxit, 0.0)
     assert it == itr
     assert float((qbar - ref).norm()) < 8 * maxit * 2.0 ** -53 * l ** 0.5
+
+
+def _sketch_ms(a, omega, k, p, N):
+    from mcnla_b200 import isvd
+    m, n = a.shape
+    prm = isvd.Parameters().setSize(m, n).setRank(k).setOverRank(p).setNumSketch(N).sync()
+    st = isvd.GaussianProjectionSketcher(prm, 0, 0).setOmega(omega)
+    st.initialize()
+    q = prm.createCollectionQ()
+    times = []
+    for _ in range(8):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        st(a, q)
+        e1.record()
+        torch.cuda.synchronize()
+        times.append(e0.elapsed_time(e1))
+    return q, min(times)
+
+
+@pytest.mark.parametrize("m,n", [(16384, 4096), (16321, 4095)])
+def test_spread_rows_for_the_fp64_units(cuda, m, n):
+    """A sparse row in every 64 leaves no tile to the int8 units: the sketch must not take longer than that of a matrix
+    of sparse rows alone, which the FP64 units compute, and gives what they give."""
+    k, p, N = 64, 32, 8
+    g = torch.Generator(device=cuda)
+    g.manual_seed(12)
+    a = torch.randn(m, n, generator=g, dtype=torch.float64, device=cuda)
+    omega = torch.randn(n, (k + p) * N, generator=g, dtype=torch.float64, device=cuda)
+    keep = torch.rand(n, generator=g, device=cuda) < 8.0 / n
+    a[::64] *= keep
+    q, some = _sketch_ms(a, omega, k, p, N)
+    ref = a @ omega
+    assert float(((q - ref).norm(dim=1) / (a.norm(dim=1) * omega.norm() + 1e-300)).max()) < 1e-14
+    a *= keep
+    _, every = _sketch_ms(a, omega, k, p, N)
+    assert some < 1.12 * every
+
+
+@pytest.mark.parametrize("n,layout", [(1200, "row"), (24000, "row"), (24000, "col")])
+def test_flags_over_chunks(cuda, n, layout):
+    """More columns of A than a chunk of K holds, with a NaN, an infinity and a sparse row whose entries lie in the last
+    chunk: the FP64 units' values in those rows' tiles, in the others the bound."""
+    from test_gpu_int8 import _check, _sketch
+    m, k, p, N = 1500, 100, 28, 32
+    g = torch.Generator(device=cuda)
+    g.manual_seed(n)
+    a = torch.randn(m, n, generator=g, dtype=torch.float64, device=cuda)
+    omega = torch.randn(n, (k + p) * N, generator=g, dtype=torch.float64, device=cuda)
+    a[300, n - 2] = float("nan")
+    a[700, n - 3] = float("inf")
+    a[1100] = 0
+    a[1100, n - 5] = 2.0
+    x = a.t().contiguous().t() if layout == "col" else a
+    q, _ = _sketch(x, omega, k, p, N)
+    ref = a @ omega
+    assert torch.isnan(q[300]).all() and torch.equal(q[700], ref[700])
+    assert torch.equal(q[1100], 2.0 * omega[n - 5])
+    _check(q, a, omega, [0, 127, 128, 255, 1025, 1151, 1152, 1499], [0, 255, 256, 4095])
+    ok = torch.ones(m, dtype=torch.bool, device=cuda)
+    ok[[300, 700]] = False
+    assert float(((q - ref)[ok].norm(dim=1) / (a[ok].norm(dim=1) * omega.norm())).max()) < 1e-14
