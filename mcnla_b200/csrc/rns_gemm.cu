@@ -2,7 +2,8 @@
 //
 // The scales of A's rows and of B's columns, which also say which tiles of C the DMMA GEMM takes; then for the other
 // tiles the residues (K-contiguous int8 planes, one per modulus), the int8 GEMMs of all moduli in one persistent
-// launch (tcgen05 kind::i8), and the CRT back to FP64; then the DMMA GEMM on the flagged tiles.
+// launch (tcgen05 kind::i8), and the CRT back to FP64; then the DMMA GEMM on the flagged tiles.  With a B that is not
+// drawn, the same kernel forms the products of the magnitudes first, which flag tiles too.
 #include "rns.cuh"
 #include "rns_math.cuh"
 #include "tma.cuh"
@@ -27,14 +28,28 @@ __device__ __forceinline__ double pow2(int e) {   // |e| < 1023
   return __longlong_as_double((long long)(e + 1023) << 52);
 }
 
-// The scale of a row or column from its squared 2-norm and largest |entry|: exponent s such that the 2-norm
+// The scale of a row or column from its squared 2-norm and 1-norm: exponent s such that the 2-norm
 // times 2^s is at most 2^target.  bad: the DMMA path takes it.
-__device__ __forceinline__ int scale_of(double norm2, double mx, int64_t K, int target, bool* bad) {
-  if (mx == 0.0 && norm2 == 0.0) { *bad = false; return 0; }
-  *bad = !(norm2 <= kMaxScale) || !(norm2 >= kMinScale) || norm2 * 256.0 < double(K) * mx * mx;
+__device__ __forceinline__ int scale_of(double norm2, double norm1, int64_t K, int target, bool* bad) {
+  if (norm1 == 0.0 && norm2 == 0.0) { *bad = false; return 0; }
+  *bad = !(norm2 <= kMaxScale) || !(norm2 >= kMinScale) || norm1 * norm1 * 64.0 < double(K) * norm2;
   if (*bad) return 0;
   const int e = int((__double_as_longlong(norm2) >> 52) & 0x7ff) - 1022;   // norm2 < 2^e
   return target - ((e + 1) >> 1);
+}
+
+// Magnitudes in units of a sixteenth of the root mean square, at most 127, from the upper words of the integers (as the
+// residues are; the FP64 conversions cost the residue kernels another 15 %).
+constexpr double kLevel = 16.0;
+__device__ __forceinline__ float level_of(double norm2, int e, int64_t K) {   // e: the scale's exponent
+  return float(kLevel * sqrt(double(K) / (norm2 * pow2(e) * pow2(e))) * 0x1p32);
+}
+__device__ __forceinline__ uint32_t magnitude(uint64_t u, float level) {
+  const int h = int(uint32_t(u >> 32)) - int(rns::kOffset >> 32);
+  return uint32_t(min(127, __float2int_rn(fabsf(float(h)) * level)));
+}
+__device__ __forceinline__ uint32_t pack4_magnitude(const uint64_t (&u)[4], float level) {
+  return magnitude(u[0], level) | magnitude(u[1], level) << 8 | magnitude(u[2], level) << 16 | magnitude(u[3], level) << 24;
 }
 
 // Four consecutive residue bytes of plane i; u: the elements times their scale, rounded, plus the offset.
@@ -56,11 +71,12 @@ __device__ __forceinline__ void split_scale(int s, double* s1, double* s2) {
 }
 
 struct Out {
-  uint8_t* planes;        // [modulus][row][kp]
+  uint8_t* planes;        // [modulus][row][kp], then the magnitudes
   int64_t rows_pad;       // rows per plane
   int64_t kp;             // bytes per row: K rounded up to kKTile, zero past K
   const uint8_t* live;    // per 1 << live_shift rows: 0 when every tile of theirs is the DMMA path's
   int live_shift;
+  const float* level;     // per row: of the magnitudes; null: there are none
 };
 
 // Per row: the scale, what undoes it, and whether the DMMA path takes the row's tiles (never cleared here).
@@ -68,14 +84,16 @@ struct Scales {
   int* scale;             // exponent; kFlagged
   double* unscale;        // 2^-scale
   uint8_t* flag;
+  float* level;           // of the magnitudes; 0: a zero row
 };
 constexpr int kFlagged = INT32_MIN;
 
-__device__ __forceinline__ void put_scale(const Scales& o, int64_t row, double norm2, double mx, int64_t K, int target) {
+__device__ __forceinline__ void put_scale(const Scales& o, int64_t row, double norm2, double norm1, int64_t K, int target) {
   bool bad;
-  const int e = scale_of(norm2, mx, K, target, &bad);
+  const int e = scale_of(norm2, norm1, K, target, &bad);
   o.scale[row] = bad ? kFlagged : e;
   o.unscale[row] = pow2(-e);
+  o.level[row] = bad || norm2 == 0.0 ? 0.0f : level_of(norm2, e, K);
   if (bad) o.flag[row] = 1;
 }
 
@@ -102,7 +120,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rns_rowscale(const double* __re
   const int64_t row = blockIdx.x;
   const double* a = A + row * lda;
   const int tid = threadIdx.x;
-  double s = 0.0, mx = 0.0;
+  double s = 0.0, n1 = 0.0;
   const int64_t quads = (K + 3) / 4;
 #pragma unroll 2
   for (int64_t q = tid; q < quads; q += kRowThreads) {
@@ -111,19 +129,19 @@ __global__ void __launch_bounds__(kRowThreads) k_rns_rowscale(const double* __re
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       s = fma(x[j], x[j], s);      // NaN and infinities reach the sum
-      mx = fmax(mx, fabs(x[j]));
+      n1 += fabs(x[j]);
     }
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
     s += __shfl_xor_sync(0xffffffffu, s, d);
-    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+    n1 += __shfl_xor_sync(0xffffffffu, n1, d);
   }
-  if ((tid & 31) == 0) { red_s[tid >> 5] = s; red_m[tid >> 5] = mx; }
+  if ((tid & 31) == 0) { red_s[tid >> 5] = s; red_m[tid >> 5] = n1; }
   __syncthreads();
   if (tid == 0) {
-    for (int w = 1; w < kRowThreads / 32; ++w) { s += red_s[w]; mx = fmax(mx, red_m[w]); }
-    put_scale(o, row, s, mx, K, target);
+    for (int w = 1; w < kRowThreads / 32; ++w) { s += red_s[w]; n1 += red_m[w]; }
+    put_scale(o, row, s, n1, K, target);
   }
 }
 
@@ -147,6 +165,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rns_rows(const double* __restri
     if (q >= quads) {
 #pragma unroll
       for (int i = 0; i < kRnsModuli; ++i) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(w) + i * plane) = 0u;
+      if (o.level) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(w) + kRnsModuli * plane) = 0u;
       continue;
     }
     double x[4];
@@ -157,11 +176,13 @@ __global__ void __launch_bounds__(kRowThreads) k_rns_rows(const double* __restri
 #pragma unroll
     for (int i = 0; i < kRnsModuli; ++i)
       *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(w) + i * plane) = pack4(u, IS_B ? kT.b : kT.a, i);
+    if (o.level)
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(w) + kRnsModuli * plane) = pack4_magnitude(u, o.level[row]);
   }
 }
 
 // The same for a matrix whose rows run along the other dimension (element (row r, k) at p[k ld + r]): squared
-// norms and maxima per chunk of kStatK rows of k, combined in order; then tiles through shared memory.
+// norms and 1-norms per chunk of kStatK rows of k, combined in order; then tiles through shared memory.
 constexpr int kStatK = 256;
 __global__ void __launch_bounds__(256) k_rns_colstats(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
                                                       double* part) {
@@ -169,34 +190,34 @@ __global__ void __launch_bounds__(256) k_rns_colstats(const double* __restrict__
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t r = int64_t(blockIdx.x) * 32 + lane;
   const int64_t k0 = int64_t(blockIdx.y) * kStatK, k1 = min(K, k0 + kStatK);
-  double s = 0.0, mx = 0.0;
+  double s = 0.0, n1 = 0.0;
   if (r < R) {
 #pragma unroll 4
     for (int64_t k = k0 + w; k < k1; k += 8) {
       const double x = B[k * ld + r];
       s = fma(x, x, s);
-      mx = fmax(mx, fabs(x));
+      n1 += fabs(x);
     }
   }
   ss[w][lane] = s;
-  sm[w][lane] = mx;
+  sm[w][lane] = n1;
   __syncthreads();
   if (w == 0 && r < R) {
-    for (int i = 1; i < 8; ++i) { s += ss[i][lane]; mx = fmax(mx, sm[i][lane]); }
+    for (int i = 1; i < 8; ++i) { s += ss[i][lane]; n1 += sm[i][lane]; }
     part[(2 * int64_t(blockIdx.y)) * R + r] = s;
-    part[(2 * int64_t(blockIdx.y) + 1) * R + r] = mx;
+    part[(2 * int64_t(blockIdx.y) + 1) * R + r] = n1;
   }
 }
 
 __global__ void k_rns_colscale(const double* part, int64_t R, int64_t K, int chunks, int target, Scales o) {
   const int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (r >= R) return;
-  double s = 0.0, mx = 0.0;
+  double s = 0.0, n1 = 0.0;
   for (int c = 0; c < chunks; ++c) {
     s += part[2 * int64_t(c) * R + r];
-    mx = fmax(mx, part[(2 * int64_t(c) + 1) * R + r]);
+    n1 += part[(2 * int64_t(c) + 1) * R + r];
   }
-  put_scale(o, r, s, mx, K, target);
+  put_scale(o, r, s, n1, K, target);
 }
 
 // The tiles that the DMMA path takes: those with a flagged row or column (added to what an earlier chunk of K flagged),
@@ -227,6 +248,14 @@ __global__ void __launch_bounds__(kTileN) k_rns_tiles(const uint8_t* __restrict_
   if (bad) *any = 1;
 }
 
+// The tiles in which the magnitudes' product flagged an element, to the others.
+__global__ void k_rns_low_tiles(const uint8_t* __restrict__ low, int64_t count, uint8_t* tile, int* any) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= count || !low[i]) return;
+  tile[i] = 1;
+  *any = 1;
+}
+
 constexpr int kColTile = 32;
 template <bool IS_B>
 __global__ void __launch_bounds__(256) k_rns_cols(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
@@ -253,6 +282,7 @@ __global__ void __launch_bounds__(256) k_rns_cols(const double* __restrict__ B, 
 #pragma unroll
     for (int m = 0; m < kRnsModuli; ++m)
       *reinterpret_cast<uint32_t*>(dst + m * plane) = pack4(u, IS_B ? kT.b : kT.a, m);
+    if (o.level) *reinterpret_cast<uint32_t*>(dst + kRnsModuli * plane) = pack4_magnitude(u, o.level[row]);
   }
 }
 
@@ -269,6 +299,11 @@ struct GemmArgs {
   uint8_t* y;                       // [modulus][y_rows][ldy] digits
   int64_t y_rows, ldy;
   const uint8_t* tile;              // [mt][nt]: tiles that the DMMA path takes
+  // the magnitudes' product (one job a tile) instead of the residues'
+  const float *row_level, *col_level;    // 0: a zero row or column
+  int M, N;                         // valid rows and columns
+  int low_sum;                      // below it an element is flagged
+  uint8_t* low;                     // [mt][nt]
   int* status;
 };
 
@@ -285,9 +320,10 @@ constexpr int kGemmThreads = 128 + 32 * kEpiWarps;
 // Job -> modulus and tile (false: a tile above the diagonal).  Rows of tiles run fastest, so concurrent CTAs share
 // B's tiles.
 struct Job { int p, m, n; };
+template <bool MAGNITUDES>
 __device__ __forceinline__ bool job_of(const GemmArgs& g, int64_t j, Job* out) {
   const int64_t per = int64_t(g.mt) * g.nt;
-  out->p = int(j / per);
+  out->p = MAGNITUDES ? kRnsModuli : int(j / per);
   const int64_t t = j % per;
   out->n = int(t / g.mt);
   out->m = int(t % g.mt);
@@ -304,6 +340,8 @@ __device__ __forceinline__ bool tile_unused(const GemmArgs& g, const Job& jb) {
 // accumulates in the other TMEM half.  Every wait is bounded.  What bounds it on long K is power: 2.6 POP/s at the
 // 1000 W limit on 2048 x 4096 x 20000 blocks (CTA pairs with cta_group::2, which read a third less from L2, ran
 // at the same rate; and pairs launched from several streams at once did not get past their start).
+// MAGNITUDES: the plane behind the residues' alone, and instead of digits whether an element's sum is low.
+template <bool MAGNITUDES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     rns_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, GemmArgs g) {
   extern __shared__ uint8_t smem_dyn[];
@@ -344,7 +382,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     bool ok = true;
     for (int64_t j = blockIdx.x; j < g.jobs && ok; j += gridDim.x) {
       Job jb;
-      if (!job_of(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (!job_of<MAGNITUDES>(g, j, &jb) || tile_unused(g, jb)) continue;
       if (lane == 0) {
         const int ya = int(int64_t(jb.p) * g.a_rows_pad) + g.a_row0 + jb.m * kTileM;
         const int yb = int(int64_t(jb.p) * g.b_rows_pad) + jb.n * kTileN;
@@ -377,7 +415,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     bool ok = true;
     for (int64_t j = blockIdx.x; j < g.jobs && ok; j += gridDim.x) {
       Job jb;
-      if (!job_of(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (!job_of<MAGNITUDES>(g, j, &jb) || tile_unused(g, jb)) continue;
       if (lane == 0) {
         const int b = int(done & 1);
         if (done >= 2 && !mbar_wait(&acc_empty[b], uint32_t(((done >> 1) - 1) & 1))) ok = false;
@@ -414,7 +452,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     int64_t done = 0;
     for (int64_t j = blockIdx.x; j < g.jobs; j += gridDim.x) {
       Job jb;
-      if (!job_of(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (!job_of<MAGNITUDES>(g, j, &jb) || tile_unused(g, jb)) continue;
       const int b = int(done & 1);
       // warp-uniform outcome: the TMEM loads below are .sync.aligned
       const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], uint32_t((done >> 1) & 1)));
@@ -422,6 +460,26 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (!ok) {
         if (lane == 0) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
         break;
+      }
+      if (MAGNITUDES) {
+        const int row = jb.m * kTileM + q * 32 + lane;
+        const bool row_ok = row < g.M && g.row_level[row < g.M ? row : 0] != 0.0f;
+        bool low = false;
+#pragma unroll 1
+        for (int c = 0; c < kTileN / 64; ++c) {
+          const int col = jb.n * kTileN + c0 + c * 32 + lane;
+          const unsigned cols = __ballot_sync(0xffffffffu, col < g.N && g.col_level[col < g.N ? col : 0] != 0.0f);
+          uint32_t r[32];
+          tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(b * kTileN + c0 + c * 32), r);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) low |= ((cols >> e) & 1u) && int32_t(r[e]) < g.low_sum;
+        }
+        if (__any_sync(0xffffffffu, low && row_ok) && lane == 0) g.low[int64_t(jb.m) * g.nt + jb.n] = 1;
+        fence_before();
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+        ++done;
+        continue;
       }
       uint8_t* dst = g.y + (int64_t(jb.p) * g.y_rows + int64_t(jb.m) * kTileM + q * 32 + lane) * g.ldy +
                      int64_t(jb.n) * kTileN + c0;
@@ -488,8 +546,9 @@ __global__ void __launch_bounds__(256) k_rns_crt(const uint8_t* __restrict__ y, 
 
 // ---- host
 struct Work {   // workspace layout
-  uint8_t *pa, *pb, *y, *row_flag, *col_flag, *tile, *live, *any_live;
+  uint8_t *pa, *pb, *y, *row_flag, *col_flag, *tile, *live, *any_live, *low;
   double *ua, *ub, *part;
+  float *la, *lb;
   int *scale, *any;
   int64_t a_pad, b_pad, kp, y_rows, ldy, nt;
   size_t block_flags, flags;   // bytes from `any` on: of a call's rows, and with the columns'
@@ -509,20 +568,23 @@ Work layout(const RnsPlan& p, void* ws) {
   char* base = static_cast<char*>(ws);
   size_t off = 0;
   auto take = [&](size_t b) { char* q = base + off; off += up(b); return q; };
-  w.pb = reinterpret_cast<uint8_t*>(take(size_t(kRnsModuli) * w.b_pad * w.kp));
-  w.pa = p.same ? w.pb : reinterpret_cast<uint8_t*>(take(size_t(kRnsModuli) * w.a_pad * w.kp));
+  w.pb = reinterpret_cast<uint8_t*>(take(size_t(p.planes) * w.b_pad * w.kp));
+  w.pa = p.same ? w.pb : reinterpret_cast<uint8_t*>(take(size_t(p.planes) * w.a_pad * w.kp));
   w.y = reinterpret_cast<uint8_t*>(take(size_t(kRnsModuli) * w.y_rows * w.ldy));
   const int64_t most = std::max(p.M, p.N);
   w.part = reinterpret_cast<double*>(take(size_t(2 * cdiv(p.kc, kStatK)) * most * 8));   // of strided operands
   w.scale = reinterpret_cast<int*>(take(size_t(p.N + p.M) * 4));                          // B's, then A's
   w.ub = reinterpret_cast<double*>(take(size_t(p.N) * 8));
   w.ua = p.same ? w.ub : reinterpret_cast<double*>(take(size_t(p.M) * 8));
+  w.lb = reinterpret_cast<float*>(take(size_t(p.N) * 4));
+  w.la = p.same ? w.lb : reinterpret_cast<float*>(take(size_t(p.M) * 4));
   w.live = reinterpret_cast<uint8_t*>(take(size_t(cdiv(p.M, kTileM))));
   // cleared together, the columns' flags only where B is new
   const size_t off0 = off;
   w.any = reinterpret_cast<int*>(take(2 * sizeof(int)));
   w.any_live = reinterpret_cast<uint8_t*>(w.any + 1);
   w.tile = reinterpret_cast<uint8_t*>(take(size_t(cdiv(p.M, kTileM) * w.nt)));
+  w.low = reinterpret_cast<uint8_t*>(take(size_t(cdiv(p.M, kTileM) * w.nt)));
   if (!p.same) w.row_flag = reinterpret_cast<uint8_t*>(take(size_t(p.M)));
   w.block_flags = off - off0;
   w.col_flag = reinterpret_cast<uint8_t*>(take(size_t(w.b_pad)));
@@ -569,17 +631,19 @@ int residues(Context* c, CMat x, int64_t R, int64_t K, bool is_b, const int* sca
 }  // namespace
 
 // Where the line lies: estimated microseconds of both paths.  The DMMA GEMM runs at ~31 TFLOP/s on tiles
-// of 128 columns; the int8 path costs 8.5 ps an element of A (two passes, 15 residues), 10 ps of B, 12 ps an
-// element of C (digits and CRT), 15 int8 products on 128 x 256 tiles at ~2.6 POP/s (below K = 1024 the
-// epilogue bounds a tile) and ~40 us of launches.  Measured, DMMA and int8 in us for M x K by N columns:
-//   2048 x 1024:  512: 152, 144   768: 191, 157   1536: 321, 194
-//   4096 x 4096:  128: 240, 273   192: 417, 277    768: 994, 375   1536: 1844, 544
-//   16384 x 1024: 128: 236, 337   192: 399, 351    512: 662, 408   1536: 1739, 760
-//   16384 x 256: 1536: 516, 586   700 x 8192: 384: 208, 220   512: 251, 229
-//   100000 x 20000: 4096: 490800, 122000
+// of 128 columns; the int8 path costs 8.5 ps an element of A (15 residues), 10 ps of B, 12 ps an element of C (digits and
+// CRT), waves of 128 x 256 tiles of 15 int8 products at 0.48 us a k-tile (below K = 1024 the epilogue bounds a tile) and
+// ~40 us of launches.  Measured, DMMA and int8 (with the magnitudes) in us for M x K by N columns:
+//   2048 x 1024:  768: 194, 178   1536: 325, 208     700 x 8192: 512: 257, 272   768: 419, 295
+//   4096 x 4096:  192: 422, 319    768: 997, 428    1536: 1850, 646
+//   8192 x 2048:  192: 382, 321    256: 391, 321     512: 718, 376
+//   16384 x 1024: 192: 406, 354    512: 665, 459    1536: 1744, 802
 // A Gramian's triangle halves the products of both.
-RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, int64_t max_rows) {
+RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, RnsKind kind, int64_t max_rows) {
   RnsPlan p;
+  const bool same = kind == RnsKind::Gramian;
+  const int most_planes = same ? kRnsModuli : kRnsModuli + 1;
+  p.planes = kind == RnsKind::Given ? kRnsModuli + 1 : kRnsModuli;
   p.M = M; p.N = N; p.K = K; p.same = same;
   p.streamed = max_rows > 0;
   if (M < 1 || N < 1 || K < 1) return p;
@@ -590,13 +654,13 @@ RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, i
   const double computed = same ? 0.5 * (tiles + 2.0 * double(cdiv(N, kTileM))) : tiles;
   const double dmma = half * 2.0 * m * n128 * k / 31e6;
   const double int8 = 40.0 + (same ? 0.0 : 8.5e-6 * m * k) + 10e-6 * n * k + half * 12e-6 * m * n +
-                      computed * double(kTileM) * kTileN * 2.0 * kRnsModuli * std::max(k, 1024.0) / 2.6e9;
+                      std::ceil(kRnsModuli * computed / double(c ? c->num_sms : 148)) * 0.48 * std::max(k, 1024.0) / kKTile;
   if (int8 >= dmma) return p;
   if (c && (!c->int8 || c->smem_optin < kGemmSmem)) return p;
   // B's planes within ~1.3 GB (a Gramian's, beside the integrator's state, 0.5 GB): K in chunks of equal size
   const int64_t b_pad = cdiv(N, kTileN) * kTileN;
   const int64_t b_most = int64_t(same ? 512 : 1300) << 20;
-  const int64_t most = std::min<int64_t>(kMaxChunk, std::max<int64_t>(4096, b_most / (kRnsModuli * b_pad)));
+  const int64_t most = std::min<int64_t>(kMaxChunk, std::max<int64_t>(4096, b_most / (most_planes * b_pad)));
   p.chunks = int(cdiv(K, most));
   p.kc = p.chunks == 1 ? K : cdiv(cdiv(K, p.chunks), kKTile) * kKTile;
   p.chunks = int(cdiv(K, p.kc));
@@ -605,7 +669,7 @@ RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, i
   const int64_t kp = cdiv(p.kc, kKTile) * kKTile;
   const int64_t rows = max_rows > 0 ? std::min(max_rows, M) : M;
   const int64_t cap = std::min<int64_t>(int64_t(700) << 20, std::max<int64_t>(int64_t(320) << 20, 16 * M * N));
-  const int64_t row_bytes = kRnsModuli * ((same ? 0 : kp) + b_pad);
+  const int64_t row_bytes = p.planes * (same ? 0 : kp) + kRnsModuli * b_pad;
   const int64_t panels = cdiv(rows, kTileM), most_panels = std::max<int64_t>(1, cap / row_bytes / kTileM);
   const int64_t sms = c ? c->num_sms : 148, per_panel = kRnsModuli * cdiv(N, kTileN);
   double best = 0.0;
@@ -617,7 +681,7 @@ RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, bool same, i
     }
   }
   // a plane's row index is a 32-bit tensor coordinate, a grid dimension at most 65535
-  if (kRnsModuli * b_pad > INT32_MAX / 2 || cdiv(N, kColTile) > 65535 || p.mb > 65535 || cdiv(K, kStatK) > 65535)
+  if (p.planes * b_pad > INT32_MAX / 2 || cdiv(N, kColTile) > 65535 || p.mb > 65535 || cdiv(K, kStatK) > 65535)
     return p;
   p.bytes = layout(p, nullptr).bytes + 1024;
   p.use = true;
@@ -631,13 +695,15 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
   if ((A.cs != 1 && A.rs != 1) || (B.cs != 1 && B.rs != 1)) return MCNLA_B200_ERR_LAYOUT;
   if (rows < 1 || rows > plan.M || (plan.same && rows != plan.N)) return MCNLA_B200_ERR_SHAPE;
   const Work w = layout(plan, reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~uintptr_t(1023)));
+  const bool magnitudes = plan.planes > kRnsModuli;
   const bool keep_b = reuse_b && plan.chunks == 1 && !plan.same;
   // the flags collect over chunks and blocks; a kept B keeps its own
   MB_CHECK_CUDA(cudaMemsetAsync(w.any, 0, keep_b ? w.block_flags : w.flags, c->stream));
   static std::atomic<uint64_t> attr_set{0};   // the shared-memory opt-in: one bit per device
   const uint64_t bit = uint64_t(1) << (c->device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & bit)) {
-    MB_CHECK_CUDA(cudaFuncSetAttribute(rns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGemmSmem)));
+    for (auto kern : {rns_gemm_kernel<false>, rns_gemm_kernel<true>})
+      MB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGemmSmem)));
     attr_set.fetch_or(bit, std::memory_order_acq_rel);
   }
   for (int ch = 0; ch < plan.chunks; ++ch) {
@@ -647,8 +713,8 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
     const CMat bk = cm(B.p + k0 * B.rs, B.cs, B.rs);
     int* const sb = w.scale;
     int* const sa = plan.same ? sb : w.scale + plan.N;
-    if (!keep_b) MB_CHECK(scales(c, bk, plan.N, kn, !plan.same, w.part, Scales{sb, w.ub, w.col_flag}));
-    if (!plan.same) MB_CHECK(scales(c, ak, rows, kn, false, w.part, Scales{sa, w.ua, w.row_flag}));
+    if (!keep_b) MB_CHECK(scales(c, bk, plan.N, kn, !plan.same, w.part, Scales{sb, w.ub, w.col_flag, w.lb}));
+    if (!plan.same) MB_CHECK(scales(c, ak, rows, kn, false, w.part, Scales{sa, w.ua, w.row_flag, w.la}));
     k_rns_tiles<<<unsigned(cdiv(rows, kTileM)), kTileN, 0, c->stream>>>(
         w.row_flag, w.col_flag, rows, plan.N, plan.same ? 1 : 0, w.tile, w.live, w.any_live, w.any);
     MB_CHECK_CUDA(cudaGetLastError());
@@ -656,19 +722,19 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
     // a B that later blocks of rows will keep is converted whatever this block needs
     if (!keep_b)
       MB_CHECK(residues(c, bk, plan.N, kn, !plan.same, sb,
-                        Out{w.pb, w.b_pad, kp, plan.streamed ? nullptr : w.any_live, 31}));
+                        Out{w.pb, w.b_pad, kp, plan.streamed ? nullptr : w.any_live, 31, magnitudes ? w.lb : nullptr}));
     CUtensorMap tb;
-    MB_CHECK(make_map_u8(&tb, w.pb, kRnsModuli * w.b_pad, kp, kp, kKTile, kTileN));
+    MB_CHECK(make_map_u8(&tb, w.pb, plan.planes * w.b_pad, kp, kp, kKTile, kTileN));
     for (int64_t r0 = 0; r0 < rows; r0 += plan.mb) {
       const int64_t rn = std::min(plan.mb, rows - r0);
       CUtensorMap ta;
       if (!plan.same) {
         static_assert(kTileM == 1 << 7, "a panel's rows");
         MB_CHECK(residues(c, cm(ak.p + r0 * A.rs, A.rs, A.cs), rn, kn, false, sa + r0,
-                          Out{w.pa, w.a_pad, kp, w.live + r0 / kTileM, 7}));
-        MB_CHECK(make_map_u8(&ta, w.pa, kRnsModuli * w.a_pad, kp, kp, kKTile, kTileM));
+                          Out{w.pa, w.a_pad, kp, w.live + r0 / kTileM, 7, magnitudes ? w.la + r0 : nullptr}));
+        MB_CHECK(make_map_u8(&ta, w.pa, plan.planes * w.a_pad, kp, kp, kKTile, kTileM));
       } else {
-        MB_CHECK(make_map_u8(&ta, w.pb, kRnsModuli * w.b_pad, kp, kp, kKTile, kTileM));
+        MB_CHECK(make_map_u8(&ta, w.pb, plan.planes * w.b_pad, kp, kp, kKTile, kTileM));
       }
       GemmArgs g;
       g.a_rows_pad = plan.same ? w.b_pad : w.a_pad;
@@ -684,8 +750,26 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
       g.ldy = w.ldy;
       g.tile = w.tile + r0 / kTileM * w.nt;
       g.status = &c->scal->wait_status;
+      g.row_level = w.la + r0;
+      g.col_level = w.lb;
+      g.M = int(rn);
+      g.N = int(plan.N);
+      g.low_sum = int(double(kn) * kLevel * kLevel / 16.0);
+      g.low = w.low + r0 / kTileM * w.nt;
+      if (magnitudes) {
+        const int64_t tiles = int64_t(g.mt) * g.nt;
+        GemmArgs gm = g;
+        gm.jobs = tiles;
+        rns_gemm_kernel<true><<<unsigned(std::min<int64_t>(tiles, c->num_sms)), kGemmThreads, kGemmSmem, c->stream>>>(
+            ta, tb, gm);
+        MB_CHECK_CUDA(cudaGetLastError());
+        k_rns_low_tiles<<<unsigned(cdiv(tiles, 256)), 256, 0, c->stream>>>(g.low, tiles, w.tile + r0 / kTileM * w.nt,
+                                                                          w.any);
+        MB_CHECK_CUDA(cudaGetLastError());
+        c->kernels_launched += 2;
+      }
       const unsigned ctas = unsigned(std::min<int64_t>(g.jobs, c->num_sms));
-      rns_gemm_kernel<<<ctas, kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
+      rns_gemm_kernel<false><<<ctas, kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
       MB_CHECK_CUDA(cudaGetLastError());
       k_rns_crt<<<dim3(unsigned(cdiv(plan.N, 1024)), unsigned(rn)), 256, 0, c->stream>>>(
           w.y, w.y_rows, w.ldy, rn, plan.N, w.ua + r0, w.ub, C.p + r0 * C.rs, C.rs, ch > 0,

@@ -57,11 +57,11 @@ int64_t problem_bytes(const mcnla_b200_problem& p) {
   // the int8 products' workspaces past the 64 MB below: an FP64 sketch's (a mixed solve is counted with it too, and
   // leaves it unused), and a KN Gramian's beside its state
   const int64_t small = int64_t(64) << 20;
-  stage = std::max(stage, int64_t(mb::plan_rns(nullptr, m, L, n, false).bytes) - small);
+  stage = std::max(stage, int64_t(mb::plan_rns(nullptr, m, L, n, mb::RnsKind::Drawn).bytes) - small);
   if (p.integrator == MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO) {
     const mb::SlicePlan sp = mb::plan_slices(nullptr, L, L, int(l));
     stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + int64_t(sp.a_bytes + sp.w_bytes) +
-                                int64_t(mb::plan_rns(nullptr, L, L, m, true).bytes) - small);
+                                int64_t(mb::plan_rns(nullptr, L, L, m, mb::RnsKind::Gramian).bytes) - small);
   }
   stage = std::max(stage, 4 * l * n * 8 + n * l * 8);                           // formers
   if (mixed) stage = std::max(stage, 3 * l * round8(m) * 2 + 16 * l * n * 8);   // precision former

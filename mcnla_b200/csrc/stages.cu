@@ -97,15 +97,15 @@ int with_int8_fallback(Context* c, F stage) {
 // ---------------------------------------------------------------------------
 // Sketcher
 // ---------------------------------------------------------------------------
-int run_sketch(Context* c, const Dims& d, const double* A, int layout, int64_t lda, double* omega, int exponent,
+int run_sketch(Context* c, const Dims& d, const double* A, int layout, int64_t lda, double* omega, bool drawn, int exponent,
                double* Q, bool timed_generation) {
   if (layout != MCNLA_B200_ROW_MAJOR && layout != MCNLA_B200_COL_MAJOR) return MCNLA_B200_ERR_ARG;
   if (layout == MCNLA_B200_ROW_MAJOR ? lda < d.n : lda < d.m) return MCNLA_B200_ERR_SHAPE;
   if (exponent < 0) return MCNLA_B200_ERR_ARG;
   const CMat Am = layout == MCNLA_B200_ROW_MAJOR ? crow(A, lda) : ccol(A, lda);
   // large products run on the int8 tensor cores (rns.cuh)
-  const RnsPlan fwd = plan_rns(c, d.m, d.L, d.n, false);
-  const RnsPlan back = exponent > 0 ? plan_rns(c, d.n, d.L, d.m, false) : RnsPlan();
+  const RnsPlan fwd = plan_rns(c, d.m, d.L, d.n, drawn && exponent == 0 ? RnsKind::Drawn : RnsKind::Given);
+  const RnsPlan back = exponent > 0 ? plan_rns(c, d.n, d.L, d.m, RnsKind::Given) : RnsPlan();
   const size_t wsr = std::max(fwd.bytes, back.bytes);
   Plan pl;
   pl.add(gemm_ws(c, {{d.m, d.L, d.n, 1}, {d.n, d.L, d.m, 1}}) / 8 + 1);
@@ -526,7 +526,7 @@ size_t gkn_ws_bytes(const Context* c, const Dims& d) {
 
 // The int8 plan of Bs = Qs' Qs.
 RnsPlan gkn_bs_plan(const Context* c, const Dims& d) {
-  return c->mixed_gramian ? RnsPlan() : plan_rns(c, d.L, d.L, d.m, true);
+  return c->mixed_gramian ? RnsPlan() : plan_rns(c, d.L, d.L, d.m, RnsKind::Gramian);
 }
 
 // The int8 plan of the loop's Bs Bc.
@@ -1198,7 +1198,7 @@ int run_isvd(Context* c, const Dims& d, int integrator, int former, const double
   } else {
     omega = const_cast<double*>(omega_in);   // read only: the sketch runs without power iterations
   }
-  MB_CHECK(with_int8_fallback(c, [&] { return run_sketch(c, d, A, layout, lda, omega, 0, Q, false); }));
+  MB_CHECK(with_int8_fallback(c, [&] { return run_sketch(c, d, A, layout, lda, omega, !omega_in, 0, Q, false); }));
   MB_CHECK(run_orthogonalize(c, d, Q));
   MB_CHECK(run_integrate(c, d, integrator, Q, maxit, tol, Qbar, iters));
   MB_CHECK(run_form(c, d, former, A, layout, lda, Qbar, S, U, V));
@@ -1235,7 +1235,7 @@ RowBlocks stream_blocks(Context* c, const Dims& d) {
   rb.first = std::min<int64_t>(rb.rows_per, aligned(int64_t((size_t(128) << 20) / row_bytes)));
   rb.nblocks = 1 + int(cdiv(std::max<int64_t>(0, d.m - rb.first), rb.rows_per));
   rb.splits = dgemm_heuristic_splits(c, d.m, d.L, d.n, 1);
-  rb.rns = plan_rns(c, d.m, d.L, d.n, false, rb.rows_per);
+  rb.rns = plan_rns(c, d.m, d.L, d.n, RnsKind::Given, rb.rows_per);
   return rb;
 }
 
@@ -1412,7 +1412,7 @@ size_t stage_bytes_upper(Context* c, const Dims& d) {
                       gemm_ws(c, {{L, L, m, 1}, {L, l, m, 1}, {m, l, L, 1}, {l, 2 * l, L, 1}}));
   b = std::max(b, 3 * size_t(l) * n * 8 + size_t(n) * l * 8 + gemm_ws(c, {{l, n, m, 1}, {n, l, m, 1}, {l, l, n, 1}}));
   // the int8 products: the sketch alone, Bs beside the Gramian integrator's state
-  b = std::max(b, plan_rns(c, m, L, n, false).bytes + gemm_ws(c, {{m, L, n, 1}}));
+  b = std::max(b, plan_rns(c, m, L, n, RnsKind::Given).bytes + gemm_ws(c, {{m, L, n, 1}}));
   b = std::max(b, gkn_bs_plan(c, d).bytes + gkn_state_bytes(c, d) + gkn_ws_bytes(c, d));
   return b + (64 << 20);
 }
@@ -1636,7 +1636,7 @@ int gitem_phase_a(Context* c, GItem& it, SolveScratch& s) {
     int64_t lda = 0;
     MB_CHECK(problem_a64(c, p, s, &A, &lda));
     MB_CHECK(launch_gaussian(c, p.seed, int64_t(d.n) * d.L, it.omega));
-    MB_CHECK(with_int8_fallback(c, [&] { return run_sketch(c, d, A, p.a_layout, lda, it.omega, 0, it.Q, false); }));
+    MB_CHECK(with_int8_fallback(c, [&] { return run_sketch(c, d, A, p.a_layout, lda, it.omega, true, 0, it.Q, false); }));
   } else {
     const uint16_t* part[3];
     int64_t ld16 = 0;
@@ -1984,7 +1984,7 @@ int mcnla_b200_sketch(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, cons
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  return mb::with_int8_fallback(ctx, [&] { return mb::run_sketch(ctx, d, A, a_layout, lda, omega, exponent, Q, false); });
+  return mb::with_int8_fallback(ctx, [&] { return mb::run_sketch(ctx, d, A, a_layout, lda, omega, false, exponent, Q, false); });
 }
 
 int mcnla_b200_gaussian(mcnla_b200_ctx* ctx, uint64_t seed, int64_t count, double* out) {

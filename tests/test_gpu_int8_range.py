@@ -136,3 +136,36 @@ def test_flags_over_chunks(cuda, n, layout):
     ok = torch.ones(m, dtype=torch.bool, device=cuda)
     ok[[300, 700]] = False
     assert float(((q - ref)[ok].norm(dim=1) / (a[ok].norm(dim=1) * omega.norm())).max()) < 1e-14
+
+
+@pytest.mark.parametrize("m,n", [(2048, 4096), (2176, 4001)])
+def test_omega_small_where_a_is_large(cuda, m, n):
+    """Sums whose large factors do not meet: an Omega that is zero where A is large, a share of A's rows with few entries,
+    and a power iteration on rows of two scales.  The error stays within what a running FP64 sum loses by
+    elements, sqrt(K) 2^-53 |A| |B| (rounding errors of K terms, uncorrelated)."""
+    import numpy as np
+    from test_gpu_int8 import _sketch
+    k, p, N = 64, 32, 16
+    g = torch.Generator(device=cuda)
+    g.manual_seed(n)
+    a = torch.randn(m, n, generator=g, dtype=torch.float64, device=cuda)
+    omega = torch.randn(n, (k + p) * N, generator=g, dtype=torch.float64, device=cuda)
+    a[:, :n // 2] *= 1e10
+    omega[:n // 2] = 0
+    a[1000:1100] *= torch.rand(100, n, generator=g, device=cuda) < 0.01
+    q, _ = _sketch(a, omega.clone(), k, p, N)
+    rows = [0, 1, 127, 128, 1000, 1050, 1099, m - 1]
+    cols = list(range(0, (k + p) * N, 37))
+    al, bl = a[rows].cpu().numpy().astype(np.longdouble), omega[:, cols].cpu().numpy().astype(np.longdouble)
+    err = np.abs(q[rows][:, cols].cpu().numpy() - al @ bl)
+    assert (err <= 2.0 ** -53 * n ** 0.5 * (np.abs(al) @ np.abs(bl))).all()
+    # A' Q with Q = A Omega: columns of A that live on the small rows alone
+    a = torch.randn(m, n, generator=g, dtype=torch.float64, device=cuda)
+    a[:m // 2, n // 2:] = 0
+    a[m // 2:, :n // 2] = 0
+    a[m // 2:] *= 1e-8
+    omega = torch.randn(n, (k + p) * N, generator=g, dtype=torch.float64, device=cuda)
+    q, _ = _sketch(a, omega.clone(), k, p, N, exponent=1)
+    ref = a @ (a.T @ (a @ omega))
+    low = q[m // 2:]
+    assert float((low - ref[m // 2:]).norm() / ref[m // 2:].norm()) < 1e-13
