@@ -58,7 +58,6 @@ struct DevScalars {
   int resume_it;      // persistent integrator: iteration it handed back to the host (-1: none)
   int eig_needed;     // SVD former: 1 when the second Gram matrix is not close to the identity
   int kn_ns_failed;   // 1: the Newton-Schulz KN step with its matrices in global memory failed
-  int slice_few;      // fixed matrices (a bit each) that the int8 slices are not for (slice.cuh)
   int wait_status;    // a bounded wait of the int8 GEMM ran out: kept (ctx_reset_scalars) until it is reported
 };
 

@@ -10,13 +10,15 @@
 // element, less than its FP64 form).
 //
 // Error: the integers' rounding, about 2^-56 (max|a_i| |b_j| + |a_i| max|b_j|), and what is left out (d > kSlices),
-// about 2^-64 sqrt(K) max|a_i| max|b_j|: for any row and column at most about the 2^-55 |a_i| |b_j| of a running FP64
-// sum, and for rows and columns without dominating entries below it by the square root of K.  (Without the order
-// d = kSlices, 2^-56 sqrt(K) max|a_i| max|b_j| was left out: 4e-15 |a_i| |b_j| where one entry dominates at K = 16384.)
-// A sum over few large terms loses less than that bound in FP64, so where a row of A has few entries near its largest
-// (2-norm^2 below K / 256 times the largest entry^2, the residue products' rule), or NaN or infinities, slice_a says
-// so and the caller keeps the DMMA GEMM.  Any finite magnitude of a row or column is taken; NaN or an infinity in a
-// column of B makes that column of C NaN.
+// about 2^-64 sqrt(K) max|a_i| max|b_j|: for any row and column at most about 2^-55 |a_i| |b_j|, and for rows and columns
+// without dominating entries below that by the square root of K.  (Without the order d = kSlices, 2^-56 sqrt(K) max|a_i|
+// max|b_j| was left out: 4e-15 |a_i| |b_j| where one entry dominates at K = 16384, and 12 iterations on such bases were
+// off by 6e-13 in the Frobenius norm, where they are by 3e-14 now and with the DMMA GEMM.)  That is normwise by rows and
+// columns, as the bases themselves are known (an orthogonalizer's sums leave 1e-16 of a row's norm in its every entry),
+// so small entries beside large ones have no rule of their own; one that kept rows with dominating entries on the
+// DMMA GEMM, as the residue products do, took every Bs with directions the sketches do not share (rows near the unit
+// vectors), for the same results.
+// Any finite magnitude of a row or column is taken; NaN or an infinity in it makes its results NaN.
 #pragma once
 #include "common.cuh"
 
@@ -38,10 +40,8 @@ struct SlicePlan {
 
 // The plan, or use = false where the DMMA GEMM is the faster one.  c may be null (an estimate).
 SlicePlan plan_slices(const Context* c, int64_t M, int64_t K, int l);
-// Cuts A (unit stride along K or along M) into aw (plan.a_bytes), and sets `bit` in the device scalar slice_few when a
-// row is not for the slices.  slice_bits reads that scalar and waits for it.
-int slice_a(Context* c, const SlicePlan& p, CMat A, void* aw, int bit);
-int slice_bits(Context* c, int* bits);
+// Cuts A (unit stride along K or along M) into aw (plan.a_bytes).
+int slice_a(Context* c, const SlicePlan& p, CMat A, void* aw);
 // C := alpha A B (B with unit stride along its columns' direction l, C row-major), with A's slices in aw; ww:
 // plan.w_bytes of scratch.  Honours the context's iteration guard; nothing but launches.
 int slice_mul(Context* c, const SlicePlan& p, const void* aw, CMat B, double alpha, DMat C, void* ww);

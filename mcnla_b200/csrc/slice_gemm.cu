@@ -75,13 +75,8 @@ __device__ __forceinline__ void store4(const unsigned long long (&u)[4], uint8_t
   }
 }
 
-// Whether a row has too few entries near its largest for fixed-point digits (see slice.cuh), from the sums over its
-// scaled entries.
-__device__ __forceinline__ bool few_large(double norm2, double mx, int64_t K) { return norm2 * 256.0 < double(K) * mx * mx; }
-
-// Rows with K contiguous, one CTA a row.  *few |= bit: a row that is not for the slices.
-__global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A, int64_t lda, int64_t K, Sliced o,
-                                                    int* few, int bit) {
+// Rows with K contiguous, one CTA a row.
+__global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A, int64_t lda, int64_t K, Sliced o) {
   __shared__ double red[8];
   const int64_t row = blockIdx.x;
   const double* a = A + row * lda;
@@ -104,33 +99,19 @@ __global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A
   const int h = e / 2;
   const double s1 = pow2(h), s2 = pow2(e - h);
   const bool ok = un != kNotFinite;
-  double ss = 0.0;
   for (int64_t q = threadIdx.x; q < o.kt * (kKTile / 4); q += 256) {
     unsigned long long u[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int64_t k = 4 * q + j;
-      const double y = ok && k < K ? a[k] * s1 * s2 : 0.0;
-      ss = fma(y, y, ss);
-      u[j] = digits(y);
+      u[j] = digits(ok && k < K ? a[k] * s1 * s2 : 0.0);
     }
     store4(u, o.at(row, 4 * q), o.plane());
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ss = 0.0;
-    for (int w = 0; w < 8; ++w) ss += red[w];
-    if (!ok || few_large(ss, mx * s1 * s2, K)) atomicOr(few, bit);
   }
 }
 
 // Rows along the other dimension (element (r, k) at p[k ld + r]): the maxima of chunks of kStatK, then tiles
-// through shared memory; each CTA of the second kernel combines its rows' maxima itself and leaves the rows' sums of
-// scaled squares over its k-tile (and, the first one, their scaled maxima) to the third.
+// through shared memory; each CTA of the second kernel combines its rows' maxima itself.
 __global__ void __launch_bounds__(256) k_slice_max(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
                                                    double* part) {
   __shared__ double sm[8][33];
@@ -156,8 +137,7 @@ __global__ void __launch_bounds__(256) k_slice_max(const double* __restrict__ B,
 }
 
 __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B, int64_t ld, int64_t R, int64_t K,
-                                                    const double* __restrict__ part, int chunks, Sliced o,
-                                                    double* sums, double* peak) {
+                                                    const double* __restrict__ part, int chunks, Sliced o) {
   __shared__ double tile[32][kKTile + 2];
   __shared__ double sm[8][33];
   __shared__ int se[32];
@@ -174,13 +154,9 @@ __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B
   if (w == 0) {
     for (int i = 1; i < 8; ++i) mx = fmax(mx, sm[i][lane]);
     int un;
-    const int e = scale_of(mx, &un), h = e / 2;
-    se[lane] = e;
+    se[lane] = scale_of(mx, &un);
     sok[lane] = un != kNotFinite;
-    if (r < R && blockIdx.x == 0) {
-      o.unscale[r] = un;
-      peak[r] = mx * pow2(h) * pow2(e - h);
-    }
+    if (r < R && blockIdx.x == 0) o.unscale[r] = un;
   }
   __syncthreads();
   for (int i = w; i < 32; i += 8) {
@@ -188,28 +164,10 @@ __global__ void __launch_bounds__(256) k_slice_cols(const double* __restrict__ B
     const int e = se[i], h = e / 2;
     const double s1 = pow2(h), s2 = pow2(e - h);
     unsigned long long u[4];
-    double ss = 0.0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const double y = sok[i] ? tile[i][4 * lane + j] * s1 * s2 : 0.0;
-      ss = fma(y, y, ss);
-      u[j] = digits(y);
-    }
+    for (int j = 0; j < 4; ++j) u[j] = digits(sok[i] ? tile[i][4 * lane + j] * s1 * s2 : 0.0);
     store4(u, o.at(r0 + i, k0 + 4 * lane), o.plane());
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-    if (lane == 0) sums[int64_t(blockIdx.x) * R + r0 + i] = ss;
   }
-}
-
-__global__ void __launch_bounds__(256) k_slice_few_large(const double* __restrict__ sums, const double* __restrict__ peak,
-                                                         int64_t R, int64_t K, int64_t kt, Sliced o, int* few, int bit) {
-  const int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (r >= R) return;
-  double ss = 0.0;
-#pragma unroll 8
-  for (int64_t t = 0; t < kt; ++t) ss += sums[t * R + r];
-  if (o.unscale[r] == kNotFinite || few_large(ss, peak[r], K)) atomicOr(few, bit);
 }
 
 // The l columns of B (element (k, j) at p[k ld + j]) in one launch: four columns a cluster, K cut over its CTAs, which
@@ -461,7 +419,7 @@ __global__ void k_slice_sum(const double* __restrict__ P, int parts, int64_t M, 
 
 size_t up(size_t b) { return (b + 1023) & ~size_t(1023); }
 
-struct ALayout { Sliced o; double *part, *sums, *peak; int64_t rows; size_t bytes; };
+struct ALayout { Sliced o; double* part; int64_t rows; size_t bytes; };
 ALayout a_layout(const SlicePlan& p, void* w) {
   ALayout a;
   a.o.kt = cdiv(p.K, kKTile);
@@ -474,10 +432,6 @@ ALayout a_layout(const SlicePlan& p, void* w) {
   off += up(size_t(p.M) * 4);
   a.part = reinterpret_cast<double*>(base + off);
   off += up(size_t(cdiv(p.K, kStatK)) * p.M * 8);
-  a.sums = reinterpret_cast<double*>(base + off);
-  off += up(size_t(a.o.kt) * p.M * 8);
-  a.peak = reinterpret_cast<double*>(base + off);
-  off += up(size_t(p.M) * 8);
   a.bytes = off + 1024;
   return a;
 }
@@ -553,32 +507,22 @@ SlicePlan plan_slices(const Context* c, int64_t M, int64_t K, int l) {
   return p;
 }
 
-int slice_a(Context* c, const SlicePlan& p, CMat A, void* aw, int bit) {
+int slice_a(Context* c, const SlicePlan& p, CMat A, void* aw) {
   if (!p.use || !aw) return MCNLA_B200_ERR_ARG;
-  int* few = &c->scal->slice_few;
   const ALayout a = a_layout(p, aw);
   if (A.cs == 1) {
-    k_slice_rows<<<unsigned(p.M), 256, 0, c->stream>>>(A.p, A.rs, p.K, a.o, few, bit);
+    k_slice_rows<<<unsigned(p.M), 256, 0, c->stream>>>(A.p, A.rs, p.K, a.o);
     c->kernels_launched++;
   } else if (A.rs == 1) {
     const int chunks = int(cdiv(p.K, kStatK));
     k_slice_max<<<dim3(unsigned(cdiv(p.M, 32)), unsigned(chunks)), 256, 0, c->stream>>>(A.p, A.cs, p.M, p.K, a.part);
     k_slice_cols<<<dim3(unsigned(a.o.kt), unsigned(cdiv(p.M, 32))), 256, 0, c->stream>>>(A.p, A.cs, p.M, p.K, a.part,
-                                                                                       chunks, a.o, a.sums, a.peak);
-    k_slice_few_large<<<unsigned(cdiv(p.M, 256)), 256, 0, c->stream>>>(a.sums, a.peak, p.M, p.K, a.o.kt, a.o, few, bit);
-    c->kernels_launched += 3;
+                                                                                       chunks, a.o);
+    c->kernels_launched += 2;
   } else {
     return MCNLA_B200_ERR_LAYOUT;
   }
   MB_CHECK_CUDA(cudaGetLastError());
-  return MCNLA_B200_OK;
-}
-
-int slice_bits(Context* c, int* bits) {
-  MB_CHECK_CUDA(cudaMemcpyAsync(&c->scal_host->slice_few, &c->scal->slice_few, sizeof(int), cudaMemcpyDeviceToHost,
-                                c->stream));
-  MB_CHECK_CUDA(cudaStreamSynchronize(c->stream));
-  *bits = c->scal_host->slice_few;
   return MCNLA_B200_OK;
 }
 

@@ -310,13 +310,8 @@ struct QsProducts {
     ws = gemm_ws;
   }
   int prepare(Context* c) {
-    if (!rows.use && !cols.use) return MCNLA_B200_OK;
-    if (rows.use) MB_CHECK(slice_a(c, rows, crow(Qs, L), rows8, 1));
-    if (cols.use) MB_CHECK(slice_a(c, cols, cm(Qs, 1, L), cols8, 2));
-    int few = 0;
-    MB_CHECK(slice_bits(c, &few));
-    if (few & 1) rows.use = false;
-    if (few & 2) cols.use = false;
+    if (rows.use) MB_CHECK(slice_a(c, rows, crow(Qs, L), rows8));
+    if (cols.use) MB_CHECK(slice_a(c, cols, cm(Qs, 1, L), cols8));
     return MCNLA_B200_OK;
   }
   // C (m x l) := alpha Qs B
@@ -628,19 +623,14 @@ GknJob gkn_job(const Context* c, const Dims& d, const GknBufs& b, int it0, int m
 }
 
 // Bs := Qs' Qs; Bc := Bs(:, 0:l); F~ := I; E~ := 0   (:112-133)
-int gkn_prepare(Context* c, const Dims& d, const double* Qs, GknBufs& b, double* ws, const RnsPlan& plan,
+int gkn_prepare(Context* c, const Dims& d, const double* Qs, const GknBufs& b, double* ws, const RnsPlan& plan,
                 void* wr) {
   const int l = d.l;
   const int64_t L = d.L, l3 = 3 * l;
   MB_CHECK(gramian_bs(c, d, Qs, b.Bs, b.EB[0] + l, l3, ws, b.bs16, plan, wr));
   MB_CHECK(launch_fill(c, L, l, 0.0, b.EB[0], l3));
   MB_CHECK(launch_set_identity(c, l, b.FF[0], l));
-  if (b.slices.use) {
-    int few = 0;
-    MB_CHECK(slice_a(c, b.slices, crow(b.Bs, L), b.bs8, 1));
-    MB_CHECK(slice_bits(c, &few));
-    if (few) b.slices.use = false;
-  }
+  if (b.slices.use) MB_CHECK(slice_a(c, b.slices, crow(b.Bs, L), b.bs8));
   const int64_t ldL = (L + 7) & ~int64_t(7);
   const size_t bpart = size_t(L) * ldL;
   if (b.bf16_bgc)
