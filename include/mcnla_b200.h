@@ -336,7 +336,8 @@ MCNLA_B200_API int mcnla_b200_isvd_mixed(mcnla_b200_ctx* ctx, const mcnla_b200_p
  *   formers.  Other problems run whole solves on the workers.
  * A itself is the caller's and is not counted.  Every solve is deterministic:
  * a problem gives the same bits alone, in a batch of the pool and in a served
- * mix; in a grouped batch it gives the same bits in any batch and agrees with
+ * mix (where a large FP64 product's int8 workspace does not fit on the device,
+ * its stage runs again on the FP64 units: the same to rounding); in a grouped batch it gives the same bits in any batch and agrees with
  * the single solve to rounding with the same iteration count (the grouped
  * kernel sums its products in its own fixed order).
  * Precisions: FP64 runs the plain path (an FP32 A is converted to FP64 on the

@@ -10,7 +10,9 @@
 // workspaces they hold (and grow them again on their next solve), so large
 // requests do not leave every worker holding their size; workspaces that
 // block nothing are kept.  Results do not depend on what else is in flight:
-// every kernel reduces in a fixed order.
+// every kernel reduces in a fixed order, and which units a product runs on
+// follows from the problem (only where an int8 workspace does not fit on the
+// device does its stage run again on the FP64 units).
 #include "common.cuh"
 #include "rns.cuh"
 #include "slice.cuh"
@@ -62,6 +64,13 @@ int64_t problem_bytes(const mcnla_b200_problem& p) {
     const mb::SlicePlan sp = mb::plan_slices(nullptr, L, L, int(l));
     stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + int64_t(sp.a_bytes + sp.w_bytes) +
                                 int64_t(mb::plan_rns(nullptr, L, L, m, mb::RnsKind::Gramian).bytes) - small);
+  }
+  if ((p.integrator == MCNLA_B200_KOLMOGOROV_NAGUMO || p.integrator == MCNLA_B200_ROW_BLOCK_KOLMOGOROV_NAGUMO) &&
+      mb::use_qs_slices(p.max_iteration)) {
+    // the loops' int8 slices of Qs, in both layouts, beside their state
+    const mb::SlicePlan rows = mb::plan_slices(nullptr, m, L, int(l)), cols = mb::plan_slices(nullptr, L, m, int(l));
+    stage = std::max(stage, 2 * (m + L) * 2 * l * 8 + int64_t(rows.a_bytes + cols.a_bytes +
+                                                              std::max(rows.w_bytes, cols.w_bytes)));
   }
   stage = std::max(stage, 4 * l * n * 8 + n * l * 8);                           // formers
   if (mixed) stage = std::max(stage, 3 * l * round8(m) * 2 + 16 * l * n * 8);   // precision former

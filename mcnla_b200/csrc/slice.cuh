@@ -40,6 +40,9 @@ struct SlicePlan {
 
 // The plan, or use = false where the DMMA GEMM is the faster one.  c may be null (an estimate).
 SlicePlan plan_slices(const Context* c, int64_t M, int64_t K, int l);
+// Whether a KN loop with Qs and Qs' cuts Qs at all: by the problem alone, so that a solve gives the same bits in a
+// server's worker as alone.
+inline bool use_qs_slices(int maxit) { return maxit >= 8; }
 // Cuts A (unit stride along K or along M) into aw (plan.a_bytes).
 int slice_a(Context* c, const SlicePlan& p, CMat A, void* aw);
 // C := alpha A B (B with unit stride along its columns' direction l, C row-major), with A's slices in aw; ww:

@@ -285,8 +285,7 @@ int kn_loop(Context* c, int maxit, Body body, int* iters) {
 }
 
 // The products of an iteration loop with Qs and Qs', Qs cut into int8 slices once in each layout
-// (slice.cuh).  14 bytes an element of Qs next to its 8, so not in the server's workers (their memory is admitted
-// by an estimate without them), and not for a handful of iterations.
+// (slice.cuh): 14 bytes an element of Qs next to its 8, and not for a handful of iterations (use_qs_slices).
 struct QsProducts {
   SlicePlan rows, cols;            // Qs B (K = L), Qs' X (K = m)
   double *rows8 = nullptr, *cols8 = nullptr, *work = nullptr;
@@ -296,7 +295,7 @@ struct QsProducts {
   double* ws = nullptr;
 
   QsProducts(const Context* c, const Dims& d, int maxit, const double* q) : Qs(q), m(d.m), L(d.L), l(d.l) {
-    if (c->coop_cta_limit > 0 || maxit < 8) return;
+    if (!use_qs_slices(maxit)) return;
     rows = plan_slices(c, m, L, l);
     cols = plan_slices(c, L, m, l);
   }

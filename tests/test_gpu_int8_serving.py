@@ -1,0 +1,25 @@
+"""Problems whose products run on the int8 tensor cores, served: the same bits as alone."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("integrator", ["kn", "rb_kn"])
+def test_loops_with_slices_served_as_alone(cuda, integrator):
+    """From 8e6 elements of Qs on the loops multiply with its int8 slices; a worker's share of the SMs must not change
+    that, nor the bits."""
+    from mcnla_b200 import isvd, synthetic
+    m, n, k, p, N = 8200, 900, 48, 16, 16
+    a = torch.as_tensor(synthetic.lowrank_np(m, n, [1.0 / j for j in range(1, 121)], seed=3, noise=1e-4), device=cuda)
+    reqs = [isvd.Request(a, k, p, N, seed=5 + i, integrator=integrator, former="svd", tol=1e-6, maxit=32)
+            for i in range(3)]
+    with isvd.Server(workers=2) as server:
+        for r in reqs:
+            server.submit(r)
+        for r in reqs:
+            server.wait(r)
+    for i, r in enumerate(reqs):
+        s, u, v, it = isvd.solve(a, k, p, N, seed=5 + i, integrator=integrator, former="svd", tol=1e-6, maxit=32)
+        assert it == r.result.iteration
+        assert torch.equal(s, r.s) and torch.equal(u, r.u) and torch.equal(v, r.v)
