@@ -151,7 +151,9 @@ MCNLA_B200_API int mcnla_b200_last_times(mcnla_b200_ctx* ctx, double* times, int
 /* Pre-allocates the workspaces a pipeline with these parameters, integrator
  * and former will use, like StageWrapper::initialize()
  * (include/mcnla/isvd/core/stage_wrapper.hpp:37-46).  Optional: stages grow
- * the workspace on first use otherwise.                                      */
+ * the workspace on first use otherwise.  integrator -1: any but the int8
+ * slices of Qs of the plain and the row-block KN loops (14 bytes an element),
+ * which are pre-allocated for those integrators only; former: -1 for any.    */
 MCNLA_B200_API int mcnla_b200_initialize(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, int integrator, int former);
 
 /* ---- sketcher ------------------------------------------------------------

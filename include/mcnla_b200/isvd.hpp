@@ -150,10 +150,11 @@ class Parameters {
 template <class Derived>
 class StageWrapper {
  public:
+  static constexpr int kIntegrator = -1;   // an integrator's enumerator
   explicit StageWrapper(const Parameters& p) : parameters_(p) {}
   void initialize() {
     if (!parameters_.isSynchronized()) throw Error(MCNLA_B200_ERR_ARG, "initialize: parameters not synchronized");
-    check(mcnla_b200_initialize(parameters_.ctx(), &parameters_.c(), -1, -1), "initialize");
+    check(mcnla_b200_initialize(parameters_.ctx(), &parameters_.c(), Derived::kIntegrator, -1), "initialize");
     initialized_ = true;
     computed_ = false;
   }
@@ -234,6 +235,7 @@ class IntegratorStage : public StageWrapper<IntegratorStage<Kind>> {
   using Base = StageWrapper<IntegratorStage<Kind>>;
 
  public:
+  static constexpr int kIntegrator = Kind;
   IntegratorStage(const Parameters& p, int max_iteration = 256,
                   double tolerance = (Kind >= MCNLA_B200_ROW_BLOCK_WEN_YIN ? 1e-3 : 1e-4))
       : Base(p), max_iteration_(max_iteration), tolerance_(tolerance) {}

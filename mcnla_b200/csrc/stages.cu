@@ -299,6 +299,7 @@ struct QsProducts {
     rows = plan_slices(c, m, L, l);
     cols = plan_slices(c, L, m, l);
   }
+  size_t bytes() const { return rows.a_bytes + cols.a_bytes + std::max(rows.w_bytes, cols.w_bytes); }
   void plan(Plan& pl) const {
     pl.add(rows.a_bytes, 1); pl.add(cols.a_bytes, 1); pl.add(std::max(rows.w_bytes, cols.w_bytes), 1);
   }
@@ -1393,13 +1394,18 @@ size_t pipeline_bytes(const Dims& d) {
 }
 
 // Workspace bytes each stage will ask for (for mcnla_b200_initialize).
-size_t stage_bytes_upper(Context* c, const Dims& d) {
+size_t stage_bytes_upper(Context* c, const Dims& d, int integrator) {
   const int64_t m = d.m, n = d.n, L = d.L, l = d.l;
   size_t b = 0;
-  b = std::max(b, size_t(m) * L * 8 + 5 * size_t(l) * l * d.N * 8 + gemm_ws(c, {{l, l, m, d.N}, {m, l, l, d.N}}));
+  b = std::max(b, std::max(size_t(m) * L * 8, syev_work_bytes(int(l), d.N)) + 5 * size_t(l) * l * d.N * 8 +
+                      gemm_ws(c, {{l, l, m, d.N}, {m, l, l, d.N}}));
   b = std::max(b, size_t(L) * L * 8 + 8 * size_t(L) * 3 * l * 8 + 4 * size_t(m) * 2 * l * 8 +
                       gemm_ws(c, {{L, L, m, 1}, {L, l, m, 1}, {m, l, L, 1}, {l, 2 * l, L, 1}}));
-  b = std::max(b, 3 * size_t(l) * n * 8 + size_t(n) * l * 8 + gemm_ws(c, {{l, n, m, 1}, {n, l, m, 1}, {l, l, n, 1}}));
+  if (integrator == MCNLA_B200_KOLMOGOROV_NAGUMO || integrator == MCNLA_B200_ROW_BLOCK_KOLMOGOROV_NAGUMO)
+    b = std::max(b, 2 * size_t(m + L) * 2 * l * 8 + QsProducts(c, d, 256, nullptr).bytes() +
+                        gemm_ws(c, {{L, l, m, 1}, {m, l, L, 1}, {l, 2 * l, L, 1}, {l, l, m, 1}, {m, l, 2 * l, 1}}));
+  b = std::max(b, 3 * size_t(l) * n * 8 + size_t(n) * l * 8 + syev_work_bytes(int(l), 1) +
+                      gemm_ws(c, {{l, n, m, 1}, {n, l, m, 1}, {l, l, n, 1}}));
   // the int8 products: the sketch alone, Bs beside the Gramian integrator's state
   b = std::max(b, plan_rns(c, m, L, n, RnsKind::Given).bytes + gemm_ws(c, {{m, L, n, 1}}));
   b = std::max(b, gkn_bs_plan(c, d).bytes + gkn_state_bytes(c, d) + gkn_ws_bytes(c, d));
@@ -1860,7 +1866,8 @@ int batched_solve(int device, mcnla_b200_problem* problems, int count, int worke
   // ---- waves within the budget (besides the workers' own workspaces and scratch)
   size_t worker_bytes = 0;
   for (auto& it : items) {
-    worker_bytes = std::max(worker_bytes, problem_scratch_bytes(*it.p) + size_t(it.d.m) * it.d.L * 8 +
+    worker_bytes = std::max(worker_bytes, problem_scratch_bytes(*it.p) +
+                                              std::max(size_t(it.d.m) * it.d.L * 8, syev_work_bytes(it.d.l, it.d.N)) +
                                               gkn_ws_bytes(ctx[0], it.d) + gkn_bs_plan(ctx[0], it.d).bytes +
                                               (size_t(64) << 20));
   }
@@ -1964,7 +1971,7 @@ int mcnla_b200_initialize(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, 
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  return mb::with_int8_fallback(ctx, [&] { return mb::ctx_reserve(ctx, mb::stage_bytes_upper(ctx, d)); });
+  return mb::with_int8_fallback(ctx, [&] { return mb::ctx_reserve(ctx, mb::stage_bytes_upper(ctx, d, integrator)); });
 }
 
 int mcnla_b200_sketch(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, const double* A, int a_layout,

@@ -263,10 +263,12 @@ class _Stage:
         self.initialized_ = True
         self.computed_ = False
 
+    _kind = -1     # an integrator's enumerator
+
     def _initializeImpl(self):
         ctx = context(self.parameters_.device)
         p = self.parameters_.c_params()
-        _lib.check(ctx.lib.mcnla_b200_initialize(ctx.bind(), ctypes.byref(p), -1, -1), "initialize")
+        _lib.check(ctx.lib.mcnla_b200_initialize(ctx.bind(), ctypes.byref(p), self._kind, -1), "initialize")
 
     def __call__(self, *args):
         if not self.parameters_.isSynchronized():

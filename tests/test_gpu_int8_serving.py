@@ -1,4 +1,4 @@
-"""Problems whose products run on the int8 tensor cores, served: the same bits as alone."""
+"""Problems whose products run on the int8 tensor cores, served (the same bits as alone), and their workspaces."""
 import pytest
 import torch
 
@@ -23,3 +23,21 @@ def test_loops_with_slices_served_as_alone(cuda, integrator):
         s, u, v, it = isvd.solve(a, k, p, N, seed=5 + i, integrator=integrator, former="svd", tol=1e-6, maxit=32)
         assert it == r.result.iteration
         assert torch.equal(s, r.s) and torch.equal(u, r.u) and torch.equal(v, r.v)
+
+
+@pytest.mark.parametrize("name", ["KolmogorovNagumoIntegrator", "RowBlockKolmogorovNagumoIntegrator"])
+def test_initialize_allocates_what_the_loop_uses(cuda, name):
+    from mcnla_b200 import isvd
+    m, l, N = 60000, 64, 16 if name.startswith("K") else 20
+    g = torch.Generator(device=cuda)
+    g.manual_seed(2)
+    q = torch.randn(m, l * N, generator=g, dtype=torch.float64, device=cuda) / m ** 0.5
+    prm = isvd.Parameters().setSize(m, 1000).setRank(l).setOverRank(0).setNumSketch(N).sync()
+    st = getattr(isvd, name)(prm, 16, 1e-6)
+    st.initialize()
+    qbar = prm.createMatrixQbar()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    st(q, qbar)
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < 64 << 20      # the code of a kernel's first launch, not 14 m L bytes
