@@ -385,7 +385,9 @@ typedef struct mcnla_b200_problem {
 
 typedef struct mcnla_b200_server mcnla_b200_server;
 
-/* Device bytes a problem needs while in flight (workspaces and sketches).   */
+/* Device bytes a problem needs while in flight (workspaces and sketches), an
+ * upper estimate: a mixed problem is admitted with less where an FP64 sketch's
+ * workspace is its largest term.                                             */
 MCNLA_B200_API int64_t mcnla_b200_problem_bytes(const mcnla_b200_problem* problem);
 /* `workers` host threads, each with its own context and stream.  Admission
  * keeps the workers' device memory within budget_bytes: an idle worker counts

@@ -14,6 +14,7 @@
 // follows from the problem (only where an int8 workspace does not fit on the
 // device does its stage run again on the FP64 units).
 #include "common.cuh"
+#include "kernels.cuh"
 #include "rns.cuh"
 #include "slice.cuh"
 #include "solve.cuh"
@@ -49,17 +50,21 @@ constexpr int64_t kKeepBytes = int64_t(64) << 20;
 
 }  // namespace
 
-int64_t problem_bytes(const mcnla_b200_problem& p) {
+// admit: what the problem is admitted with; else an upper estimate, which counts the int8 sketch with a mixed
+// problem too.
+int64_t problem_bytes(const mcnla_b200_problem& p, bool admit) {
   const int64_t m = p.params.nrow, n = p.params.ncol, l = p.params.rank + p.params.over_rank;
   const int64_t L = l * p.params.num_sketch;
   const bool mixed = p.precision == MCNLA_B200_PRECISION_MIXED || p.precision == MCNLA_B200_PRECISION_MIXED3;
   int64_t bytes = (m * L + m * l) * 8 + (mixed ? L * round8(n) * 2 : n * L * 8);  // Q, Qbar, Omega
-  int64_t stage = m * L * 8 + 5 * l * l * p.params.num_sketch * 8;              // orthogonalizer
+  // orthogonalizer: a copy of Q or the eigensolver's rotation logs in one buffer, and l x l matrices
+  int64_t stage = std::max<int64_t>(m * L * 8, int64_t(mb::syev_work_bytes(int(l), p.params.num_sketch))) +
+                  5 * l * l * p.params.num_sketch * 8;
   stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + 4 * m * 2 * l * 8);   // integrators
-  // the int8 products' workspaces past the 64 MB below: an FP64 sketch's (a mixed solve is counted with it too, and
-  // leaves it unused), and a KN Gramian's beside its state
+  // the int8 products' workspaces past the 64 MB below: an FP64 sketch's, and a KN Gramian's beside its state
   const int64_t small = int64_t(64) << 20;
-  stage = std::max(stage, int64_t(mb::plan_rns(nullptr, m, L, n, mb::RnsKind::Drawn).bytes) - small);
+  if (!mixed || !admit)
+    stage = std::max(stage, int64_t(mb::plan_rns(nullptr, m, L, n, mb::RnsKind::Drawn).bytes) - small);
   if (p.integrator == MCNLA_B200_ROW_BLOCK_GRAMIAN_KOLMOGOROV_NAGUMO) {
     const mb::SlicePlan sp = mb::plan_slices(nullptr, L, L, int(l));
     stage = std::max(stage, L * L * 8 + 8 * L * 3 * l * 8 + int64_t(sp.a_bytes + sp.w_bytes) +
@@ -72,7 +77,7 @@ int64_t problem_bytes(const mcnla_b200_problem& p) {
     stage = std::max(stage, 2 * (m + L) * 2 * l * 8 + int64_t(rows.a_bytes + cols.a_bytes +
                                                               std::max(rows.w_bytes, cols.w_bytes)));
   }
-  stage = std::max(stage, 4 * l * n * 8 + n * l * 8);                           // formers
+  stage = std::max(stage, 4 * l * n * 8 + n * l * 8 + int64_t(mb::syev_work_bytes(int(l), 1)));   // formers
   if (mixed) stage = std::max(stage, 3 * l * round8(m) * 2 + 16 * l * n * 8);   // precision former
   bytes += stage + small;                                                       // + split-K partials, small terms
   bytes += int64_t(mb::problem_scratch_bytes(p));                               // FP64 copy or BF16 parts of A, A'
@@ -212,7 +217,7 @@ void mcnla_b200_server::worker(int me) {
 
 extern "C" {
 
-int64_t mcnla_b200_problem_bytes(const mcnla_b200_problem* p) { return p ? mb::problem_bytes(*p) : -1; }
+int64_t mcnla_b200_problem_bytes(const mcnla_b200_problem* p) { return p ? mb::problem_bytes(*p, false) : -1; }
 
 int mcnla_b200_server_create(mcnla_b200_server** out, int device, int workers, int64_t budget_bytes) {
   if (!out || workers < 1 || workers > 256 || budget_bytes <= 0) return MCNLA_B200_ERR_ARG;
@@ -240,7 +245,7 @@ int mcnla_b200_server_submit(mcnla_b200_server* s, const mcnla_b200_problem* pro
     j.p.status = -1;
     j.p.seconds = 0;
     j.p.latency = 0;
-    j.bytes = mb::problem_bytes(*problem);
+    j.bytes = mb::problem_bytes(*problem, true);
     j.submitted = mb::Clock::now();
     s->jobs.emplace(t, j);
     s->queue.push_back(t);

@@ -41,3 +41,17 @@ def test_initialize_allocates_what_the_loop_uses(cuda, name):
     st(q, qbar)
     torch.cuda.synchronize()
     assert before - torch.cuda.mem_get_info()[0] < 64 << 20      # the code of a kernel's first launch, not 14 m L bytes
+
+
+def test_mixed_request_is_admitted_without_the_int8_sketch(cuda):
+    """A mixed solve sketches on BF16 parts: it is admitted with less than the upper estimate, whose largest term is the
+    workspace of an FP64 sketch."""
+    from mcnla_b200 import isvd, synthetic
+    m, n, k, p, N = 8192, 2048, 32, 16, 8
+    a = torch.as_tensor(synthetic.lowrank_np(m, n, [1.0 / j for j in range(1, 81)], seed=3, noise=1e-4), device=cuda)
+    req = isvd.Request(a, k, p, N, seed=5, integrator="rb_gramian_kn", former="svd", tol=1e-5, mixed=3)
+    with isvd.Server(workers=1) as server:
+        server.wait(server.submit(req))
+        peak = server.stats()["peak_bytes"]
+    assert req.result.status == 0
+    assert peak < req.bytes() - (100 << 20)
