@@ -103,6 +103,8 @@ struct Context {
   // large products on the int8 tensor cores (rns.cuh, slice.cuh); off while a stage whose int8 workspace did not
   // fit on the device runs again without
   bool int8 = true;
+  // kernels with bounded waits of their own were launched since the scalars were last read (ctx_finish_waits)
+  bool waits_pending = false;
   // precision form: the Gramian integrators form Bs = Qs' Qs from BF16 parts of Qs
   bool mixed_gramian = false;
   // row-block decomposition over several GPUs: the stages sum their row-dependent
@@ -154,6 +156,10 @@ int ctx_toc(Context* c);
 int ctx_collect_times(Context* c);
 
 int ctx_sync_scalars(Context* c);   // copies DevScalars to the pinned mirror and waits
+// At the end of an entry point: reads the scalars where an int8 product's wait has not been looked at yet, and returns its
+// status, so that the call that ran out of time says so and not a later one.  (Nothing under stream capture, where
+// nothing has run; the next call that reads them reports it.)
+int ctx_finish_waits(Context* c);
 int ctx_reset_scalars(Context* c);  // zeroes DevScalars (stream-ordered), except a wait_status not yet reported
 
 // Sums `count` doubles at the device pointer buf over the ranks of the context's

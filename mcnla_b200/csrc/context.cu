@@ -107,11 +107,21 @@ int ctx_collect_times(Context* c) {
 int ctx_sync_scalars(Context* c) {
   MB_CHECK_CUDA(cudaMemcpyAsync(c->scal_host, c->scal, sizeof(DevScalars), cudaMemcpyDeviceToHost, c->stream));
   MB_CHECK_CUDA(cudaStreamSynchronize(c->stream));
+  c->waits_pending = false;
   if (c->scal_host->wait_status) {
     if (!c->scal_host->status) c->scal_host->status = c->scal_host->wait_status;
     MB_CHECK_CUDA(cudaMemsetAsync(&c->scal->wait_status, 0, sizeof(int), c->stream));
   }
   return MCNLA_B200_OK;
+}
+
+int ctx_finish_waits(Context* c) {
+  if (!c->waits_pending) return MCNLA_B200_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  MB_CHECK_CUDA(cudaStreamIsCapturing(c->stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) return MCNLA_B200_OK;
+  MB_CHECK(ctx_sync_scalars(c));
+  return c->scal_host->wait_status;
 }
 
 int ctx_reset_scalars(Context* c) {

@@ -778,6 +778,7 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
       c->kernels_launched += 2;
     }
   }
+  c->waits_pending = true;
   // what was flagged, over the whole K
   GemmFlags fl;
   fl.tile = w.tile;

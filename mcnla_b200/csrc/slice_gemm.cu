@@ -555,6 +555,7 @@ int slice_mul(Context* c, const SlicePlan& p, const void* aw, CMat B, double alp
   k_slice_sum<<<blocks, 256, 0, c->stream>>>(b.sums, p.splits, p.M, p.l, alpha, C.p, C.rs, c->guard_stop, c->guard_it);
   MB_CHECK_CUDA(cudaGetLastError());
   c->kernels_launched += 3;
+  c->waits_pending = true;
   return MCNLA_B200_OK;
 }
 

@@ -1192,7 +1192,7 @@ int run_isvd(Context* c, const Dims& d, int integrator, int former, const double
   MB_CHECK(run_orthogonalize(c, d, Q));
   MB_CHECK(run_integrate(c, d, integrator, Q, maxit, tol, Qbar, iters));
   MB_CHECK(run_form(c, d, former, A, layout, lda, Qbar, S, U, V));
-  return MCNLA_B200_OK;
+  return ctx_finish_waits(c);
 }
 
 // Host-buffer solve with A streamed in: the row-major host A is copied to the
@@ -1980,7 +1980,9 @@ int mcnla_b200_sketch(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, cons
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  return mb::with_int8_fallback(ctx, [&] { return mb::run_sketch(ctx, d, A, a_layout, lda, omega, false, exponent, Q, false); });
+  MB_CHECK(mb::with_int8_fallback(
+      ctx, [&] { return mb::run_sketch(ctx, d, A, a_layout, lda, omega, false, exponent, Q, false); }));
+  return mb::ctx_finish_waits(ctx);
 }
 
 int mcnla_b200_gaussian(mcnla_b200_ctx* ctx, uint64_t seed, int64_t count, double* out) {
@@ -2003,7 +2005,8 @@ int mcnla_b200_integrate(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, i
   Dims d;
   MB_CHECK(mb::get_dims(params, d));
   MB_CHECK_CUDA(cudaSetDevice(ctx->device));
-  return mb::run_integrate(ctx, d, kind, Q, max_iteration, tolerance, Qbar, iteration);
+  MB_CHECK(mb::run_integrate(ctx, d, kind, Q, max_iteration, tolerance, Qbar, iteration));
+  return mb::ctx_finish_waits(ctx);
 }
 
 int mcnla_b200_form(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, int kind, const double* A, int a_layout,
@@ -2073,6 +2076,7 @@ int mcnla_b200_isvd_host(mcnla_b200_ctx* ctx, const mcnla_b200_params* params, i
     MB_CHECK_CUDA(cudaMemcpyAsync(U_host, U, size_t(d.m) * d.k * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (V_host)
     MB_CHECK_CUDA(cudaMemcpyAsync(V_host, V, size_t(d.n) * d.k * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  MB_CHECK(mb::ctx_finish_waits(ctx));
   MB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
   return MCNLA_B200_OK;
 }
@@ -2112,6 +2116,7 @@ int mcnla_b200_isvd_stream(mcnla_b200_ctx* ctx, const mcnla_b200_params* params,
     MB_CHECK_CUDA(cudaMemcpyAsync(U_host, U, size_t(d.m) * d.k * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (V_host)
     MB_CHECK_CUDA(cudaMemcpyAsync(V_host, V, size_t(d.n) * d.k * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  MB_CHECK(mb::ctx_finish_waits(ctx));
   MB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
   return MCNLA_B200_OK;
 }
