@@ -195,12 +195,13 @@ struct HotLoop {
 
 //
 // CUDA graph: the bodies of one chunk depend on the iteration only through
-// its parity (double buffers) and the guard index, so after the first chunk
-// is launched (directly: it also tunes every product shape) the next full
-// chunk is captured once, while the device works on the first (captured after
-// the first chunk's end it left the device idle for 0.2 - 0.3 ms a solve),
-// with guard indices relative to the chunk start, and every later full chunk
-// replays that graph.  Relative indices work because the KN step records the
+// its parity (double buffers) and the guard index, so after the first two
+// chunks (launched directly; the first also tunes every product shape) the next
+// full chunk is captured once, while the device works on the second, with guard
+// indices relative to the chunk start, and every later full chunk replays that
+// graph.  (Captured between two chunks it left the device idle for 0.2 - 0.3 ms
+// a solve; behind the first one it was work for nothing in loops that end
+// there: an integration of 0.34 ms took 0.65.)  Relative indices work because the KN step records the
 // converged iteration as the guard index it was given: the host adds the
 // chunk start.  A capture that fails (an operation the graph cannot hold) is
 // abandoned and the loop continues with direct launches.
@@ -266,8 +267,8 @@ int kn_loop(Context* c, int maxit, Body body, int* iters) {
     }
     const int start = launched;
     launched = end;
-    // graph replays for full chunks after the first, when at least two remain
-    if (use_graph && !graph.exec && maxit - launched >= 2 * chunk) {
+    // graph replays for full chunks after the second, when at least two remain
+    if (use_graph && !graph.exec && start > 0 && maxit - launched >= 2 * chunk) {
       if (capture_chunk(c, launched, chunk, body, graph, &graph_kernels) != MCNLA_B200_OK) use_graph = false;
     }
     MB_CHECK(ctx_sync_scalars(c));
