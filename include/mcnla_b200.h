@@ -125,7 +125,7 @@ MCNLA_B200_API int64_t mcnla_b200_graph_replays(const mcnla_b200_ctx* ctx);
 MCNLA_B200_API int mcnla_b200_set_autotune(mcnla_b200_ctx* ctx, int on);
 /* CUDA-graph iteration loops (on by default): the Kolmogorov-Nagumo
  * integrators that launch their products per iteration (kolmogorov_nagumo_
- * integrator.hpp:109-183 and the row-block forms) run the first two chunks of 8
+ * integrator.hpp:109-183 and the row-block forms) run the first chunk of 8
  * iterations as ordinary launches, capture the next chunk once as a CUDA
  * graph and replay it for every later full chunk; results are bit-identical
  * either way.  Off: every iteration is launched.                             */

@@ -155,7 +155,10 @@ int ctx_tic(Context* c);
 int ctx_toc(Context* c);
 int ctx_collect_times(Context* c);
 
-int ctx_sync_scalars(Context* c);   // copies DevScalars to the pinned mirror and waits
+// Copies DevScalars to the pinned mirror (stream-ordered); waits for the copy; both.
+int ctx_queue_scalars(Context* c);
+int ctx_wait_scalars(Context* c);
+int ctx_sync_scalars(Context* c);
 // At the end of an entry point: reads the scalars where an int8 product's wait has not been looked at yet, and returns its
 // status, so that the call that ran out of time says so and not a later one.  (Nothing under stream capture, where
 // nothing has run; the next call that reads them reports it.)

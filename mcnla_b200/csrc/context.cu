@@ -104,8 +104,17 @@ int ctx_collect_times(Context* c) {
   return MCNLA_B200_OK;
 }
 
-int ctx_sync_scalars(Context* c) {
+int ctx_queue_scalars(Context* c) {
   MB_CHECK_CUDA(cudaMemcpyAsync(c->scal_host, c->scal, sizeof(DevScalars), cudaMemcpyDeviceToHost, c->stream));
+  return MCNLA_B200_OK;
+}
+
+int ctx_sync_scalars(Context* c) {
+  MB_CHECK(ctx_queue_scalars(c));
+  return ctx_wait_scalars(c);
+}
+
+int ctx_wait_scalars(Context* c) {
   MB_CHECK_CUDA(cudaStreamSynchronize(c->stream));
   c->waits_pending = false;
   if (c->scal_host->wait_status) {

@@ -195,16 +195,18 @@ struct HotLoop {
 
 //
 // CUDA graph: the bodies of one chunk depend on the iteration only through
-// its parity (double buffers) and the guard index, so after the first two
-// chunks (launched directly; the first also tunes every product shape) the next
-// full chunk is captured once, while the device works on the second, with guard
-// indices relative to the chunk start, and every later full chunk replays that
-// graph.  (Captured between two chunks it left the device idle for 0.2 - 0.3 ms
-// a solve; behind the first one it was work for nothing in loops that end
-// there: an integration of 0.34 ms took 0.65.)  Relative indices work because the KN step records the
+// its parity (double buffers) and the guard index, so after the first chunk
+// is launched (directly: it also tunes every product shape) the next full
+// chunk is captured once, while the device works on all but its first two iterations (captured after
+// the first chunk's end it left the device idle for 0.2 - 0.3 ms a solve),
+// with guard indices relative to the chunk start, and every later full chunk
+// replays that graph.  Relative indices work because the KN step records the
 // converged iteration as the guard index it was given: the host adds the
-// chunk start.  A capture that fails (an operation the graph cannot hold) is
-// abandoned and the loop continues with direct launches.
+// chunk start.  Nothing is captured when the first two iterations ended the
+// loop, and a capture is given up as soon as the first chunk is seen to have
+// (finished behind its back, it made an integration of 0.34 ms take 0.65).  A
+// capture that fails (an operation the graph cannot hold) is abandoned and the
+// loop continues with direct launches.
 struct LoopGraph {
   cudaGraphExec_t exec = nullptr;
   cudaStream_t cap = nullptr;
@@ -214,15 +216,16 @@ struct LoopGraph {
   }
 };
 
-template <class Body>
-int capture_chunk(Context* c, int it0, int chunk, Body& body, LoopGraph& g, int64_t* kernels) {
+// ended(): the loop is over, and the capture for nothing.
+template <class Body, class Ended>
+int capture_chunk(Context* c, int it0, int chunk, Body& body, Ended ended, LoopGraph& g, int64_t* kernels) {
   if (cudaStreamCreateWithFlags(&g.cap, cudaStreamNonBlocking) != cudaSuccess) return MCNLA_B200_ERR_CUDA;
   struct Swap { Context* c; cudaStream_t s; ~Swap() { c->stream = s; } } swap{c, c->stream};
   const int64_t k0 = c->kernels_launched;
   if (cudaStreamBeginCapture(g.cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return MCNLA_B200_ERR_CUDA;
   c->stream = g.cap;
   int st = MCNLA_B200_OK;
-  for (int r = 0; r < chunk && st == MCNLA_B200_OK; ++r) {
+  for (int r = 0; r < chunk && st == MCNLA_B200_OK && !ended(); ++r) {
     c->guard_it = r;
     st = body(it0 + r);
   }
@@ -232,7 +235,7 @@ int capture_chunk(Context* c, int it0, int chunk, Body& body, LoopGraph& g, int6
   *kernels = c->kernels_launched - k0;
   c->kernels_launched = k0;            // nothing ran yet: replays count themselves
   if (st == MCNLA_B200_OK && (ec != cudaSuccess || !graph)) st = MCNLA_B200_ERR_CUDA;
-  if (st == MCNLA_B200_OK && cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) {
+  if (st == MCNLA_B200_OK && !ended() && cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) {
     g.exec = nullptr;
     st = MCNLA_B200_ERR_CUDA;
   }
@@ -255,6 +258,11 @@ int kn_loop(Context* c, int maxit, Body body, int* iters) {
   while (launched < maxit) {
     const int end = std::min(maxit, launched + chunk);
     const bool relative = use_graph && graph.exec && end - launched == chunk;
+    // graph replays for full chunks after the first, when at least two remain
+    const bool capture = use_graph && !graph.exec && maxit - end >= 2 * chunk;
+    // the outcome arrives in the pinned mirror: -1 until then (no iteration)
+    volatile int* arrived = &c->scal_host->stop_it;
+    *arrived = -1;
     if (relative) {
       MB_CHECK_CUDA(cudaGraphLaunch(graph.exec, c->stream));
       c->kernels_launched += graph_kernels;
@@ -263,15 +271,20 @@ int kn_loop(Context* c, int maxit, Body body, int* iters) {
       for (int it = launched; it < end; ++it) {
         c->guard_it = it;
         MB_CHECK(body(it));
+        // whether the first iterations ended the loop, for the capture
+        if (capture && it == launched + 1) MB_CHECK(ctx_queue_scalars(c));
       }
     }
     const int start = launched;
     launched = end;
-    // graph replays for full chunks after the second, when at least two remain
-    if (use_graph && !graph.exec && start > 0 && maxit - launched >= 2 * chunk) {
-      if (capture_chunk(c, launched, chunk, body, graph, &graph_kernels) != MCNLA_B200_OK) use_graph = false;
+    MB_CHECK(ctx_queue_scalars(c));
+    if (capture) {
+      auto ended = [&] { return *arrived >= 0 && *arrived < launched; };
+      while (*arrived < 0 && cudaStreamQuery(c->stream) == cudaErrorNotReady) {}
+      if (!ended() && capture_chunk(c, launched, chunk, body, ended, graph, &graph_kernels) != MCNLA_B200_OK)
+        use_graph = false;
     }
-    MB_CHECK(ctx_sync_scalars(c));
+    MB_CHECK(ctx_wait_scalars(c));
     if (c->scal_host->status) return c->scal_host->status;
     const int stop = c->scal_host->stop_it;
     if (relative) {
