@@ -299,7 +299,7 @@ struct GemmArgs {
   uint8_t* y;                       // [modulus][y_rows][ldy] digits
   int64_t y_rows, ldy;
   const uint8_t* tile;              // [mt][nt]: tiles that the DMMA path takes
-  // the magnitudes' product (one job a tile) instead of the residues'
+  // the magnitudes' product
   const float *row_level, *col_level;    // 0: a zero row or column
   int M, N;                         // valid rows and columns
   int low_sum;                      // below it an element is flagged
@@ -320,10 +320,12 @@ constexpr int kGemmThreads = 128 + 32 * kEpiWarps;
 // Job -> modulus and tile (false: a tile above the diagonal).  Rows of tiles run fastest, so concurrent CTAs share
 // B's tiles.
 struct Job { int p, m, n; };
-template <bool MAGNITUDES>
+// The planes of a launch: the residues', the magnitudes' behind them, or all.
+enum : int { kResidues = 0, kMagnitudes = 1, kAllPlanes = 2 };
+template <int PLANES>
 __device__ __forceinline__ bool job_of(const GemmArgs& g, int64_t j, Job* out) {
   const int64_t per = int64_t(g.mt) * g.nt;
-  out->p = MAGNITUDES ? kRnsModuli : int(j / per);
+  out->p = PLANES == kMagnitudes ? kRnsModuli : int(j / per);
   const int64_t t = j % per;
   out->n = int(t / g.mt);
   out->m = int(t % g.mt);
@@ -335,13 +337,13 @@ __device__ __forceinline__ bool tile_unused(const GemmArgs& g, const Job& jb) {
   return g.tile[int64_t(jb.m) * g.nt + jb.n] != 0;
 }
 
-// A CTA computes 128 x 256 tiles of every modulus' product.  Warp 0: TMA into the ring of 48 KB stages; warp 1: MMA
+// A CTA computes 128 x 256 tiles of every plane's product.  Warp 0: TMA into the ring of 48 KB stages; warp 1: MMA
 // issue (M = 128, N = 256, K = 32); warps 4-11: the finished accumulator to CRT digits while the next tile
 // accumulates in the other TMEM half.  Every wait is bounded.  What bounds it on long K is power: 2.6 POP/s at the
 // 1000 W limit on 2048 x 4096 x 20000 blocks (CTA pairs with cta_group::2, which read a third less from L2, ran
 // at the same rate; and pairs launched from several streams at once did not get past their start).
-// MAGNITUDES: the plane behind the residues' alone, and instead of digits whether an element's sum is low.
-template <bool MAGNITUDES>
+// The magnitudes' plane gives instead of digits whether an element's sum is low.
+template <int PLANES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     rns_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, GemmArgs g) {
   extern __shared__ uint8_t smem_dyn[];
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     bool ok = true;
     for (int64_t j = blockIdx.x; j < g.jobs && ok; j += gridDim.x) {
       Job jb;
-      if (!job_of<MAGNITUDES>(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (!job_of<PLANES>(g, j, &jb) || tile_unused(g, jb)) continue;
       if (lane == 0) {
         const int ya = int(int64_t(jb.p) * g.a_rows_pad) + g.a_row0 + jb.m * kTileM;
         const int yb = int(int64_t(jb.p) * g.b_rows_pad) + jb.n * kTileN;
@@ -415,7 +417,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     bool ok = true;
     for (int64_t j = blockIdx.x; j < g.jobs && ok; j += gridDim.x) {
       Job jb;
-      if (!job_of<MAGNITUDES>(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (!job_of<PLANES>(g, j, &jb) || tile_unused(g, jb)) continue;
       if (lane == 0) {
         const int b = int(done & 1);
         if (done >= 2 && !mbar_wait(&acc_empty[b], uint32_t(((done >> 1) - 1) & 1))) ok = false;
@@ -452,7 +454,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     int64_t done = 0;
     for (int64_t j = blockIdx.x; j < g.jobs; j += gridDim.x) {
       Job jb;
-      if (!job_of<MAGNITUDES>(g, j, &jb) || tile_unused(g, jb)) continue;
+      if (!job_of<PLANES>(g, j, &jb) || tile_unused(g, jb)) continue;
       const int b = int(done & 1);
       // warp-uniform outcome: the TMEM loads below are .sync.aligned
       const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], uint32_t((done >> 1) & 1)));
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (lane == 0) atomicExch(g.status, MCNLA_B200_ERR_DEVICE_TIMEOUT);
         break;
       }
-      if (MAGNITUDES) {
+      if (PLANES == kMagnitudes || (PLANES == kAllPlanes && jb.p == kRnsModuli)) {
         const int row = jb.m * kTileM + q * 32 + lane;
         const bool row_ok = row < g.M && g.row_level[row < g.M ? row : 0] != 0.0f;
         bool low = false;
@@ -671,7 +673,7 @@ RnsPlan plan_rns(const Context* c, int64_t M, int64_t N, int64_t K, RnsKind kind
   const int64_t cap = std::min<int64_t>(int64_t(700) << 20, std::max<int64_t>(int64_t(320) << 20, 16 * M * N));
   const int64_t row_bytes = p.planes * (same ? 0 : kp) + kRnsModuli * b_pad;
   const int64_t panels = cdiv(rows, kTileM), most_panels = std::max<int64_t>(1, cap / row_bytes / kTileM);
-  const int64_t sms = c ? c->num_sms : 148, per_panel = kRnsModuli * cdiv(N, kTileN);
+  const int64_t sms = c ? c->num_sms : 148, per_panel = p.planes * cdiv(N, kTileN);
   double best = 0.0;
   for (int64_t q = 1; q <= std::min(panels, most_panels); ++q) {
     const double us = double(cdiv(panels, q)) * (double(cdiv(q * per_panel, sms)) * 0.48 * double(kp / kKTile) + 10.0);
@@ -702,7 +704,7 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
   static std::atomic<uint64_t> attr_set{0};   // the shared-memory opt-in: one bit per device
   const uint64_t bit = uint64_t(1) << (c->device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & bit)) {
-    for (auto kern : {rns_gemm_kernel<false>, rns_gemm_kernel<true>})
+    for (auto kern : {rns_gemm_kernel<kResidues>, rns_gemm_kernel<kMagnitudes>, rns_gemm_kernel<kAllPlanes>})
       MB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGemmSmem)));
     attr_set.fetch_or(bit, std::memory_order_acq_rel);
   }
@@ -744,7 +746,6 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
       g.nt = int(cdiv(plan.N, kTileN));
       g.kt = int(kp / kKTile);
       g.lower = plan.same ? 1 : 0;
-      g.jobs = int64_t(kRnsModuli) * g.mt * g.nt;
       g.y = w.y;
       g.y_rows = w.y_rows;
       g.ldy = w.ldy;
@@ -756,26 +757,35 @@ int rns_gemm(Context* c, const RnsPlan& plan, int64_t rows, CMat A, CMat B, DMat
       g.N = int(plan.N);
       g.low_sum = int(double(kn) * kLevel * kLevel / 16.0);
       g.low = w.low + r0 / kTileM * w.nt;
-      if (magnitudes) {
-        const int64_t tiles = int64_t(g.mt) * g.nt;
-        GemmArgs gm = g;
-        gm.jobs = tiles;
-        rns_gemm_kernel<true><<<unsigned(std::min<int64_t>(tiles, c->num_sms)), kGemmThreads, kGemmSmem, c->stream>>>(
-            ta, tb, gm);
+      const int64_t tiles = int64_t(g.mt) * g.nt;
+      auto gemm = [&](auto kern, int64_t jobs) -> int {
+        g.jobs = jobs;
+        kern<<<unsigned(std::min<int64_t>(jobs, c->num_sms)), kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
         MB_CHECK_CUDA(cudaGetLastError());
+        c->kernels_launched++;
+        return MCNLA_B200_OK;
+      };
+      if (!magnitudes) {
+        MB_CHECK(gemm(rns_gemm_kernel<kResidues>, kRnsModuli * tiles));
+      } else {
+        // in a launch of their own first, so that the residues' skips the tiles they flag, where that costs at most a
+        // twenty-fifth of the waves; else in the same launch
+        const int64_t apart = cdiv(tiles, c->num_sms) + cdiv(kRnsModuli * tiles, c->num_sms);
+        const int64_t together = cdiv((kRnsModuli + 1) * tiles, c->num_sms);
+        const bool first = 25 * (apart - together) <= together;
+        if (first) MB_CHECK(gemm(rns_gemm_kernel<kMagnitudes>, tiles));
+        else MB_CHECK(gemm(rns_gemm_kernel<kAllPlanes>, (kRnsModuli + 1) * tiles));
         k_rns_low_tiles<<<unsigned(cdiv(tiles, 256)), 256, 0, c->stream>>>(g.low, tiles, w.tile + r0 / kTileM * w.nt,
                                                                           w.any);
         MB_CHECK_CUDA(cudaGetLastError());
-        c->kernels_launched += 2;
+        c->kernels_launched++;
+        if (first) MB_CHECK(gemm(rns_gemm_kernel<kResidues>, kRnsModuli * tiles));
       }
-      const unsigned ctas = unsigned(std::min<int64_t>(g.jobs, c->num_sms));
-      rns_gemm_kernel<false><<<ctas, kGemmThreads, kGemmSmem, c->stream>>>(ta, tb, g);
-      MB_CHECK_CUDA(cudaGetLastError());
       k_rns_crt<<<dim3(unsigned(cdiv(plan.N, 1024)), unsigned(rn)), 256, 0, c->stream>>>(
           w.y, w.y_rows, w.ldy, rn, plan.N, w.ua + r0, w.ub, C.p + r0 * C.rs, C.rs, ch > 0,
           plan.same ? r0 : -1, g.tile, g.nt);
       MB_CHECK_CUDA(cudaGetLastError());
-      c->kernels_launched += 2;
+      c->kernels_launched++;
     }
   }
   c->waits_pending = true;

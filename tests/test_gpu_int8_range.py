@@ -138,14 +138,13 @@ def test_flags_over_chunks(cuda, n, layout):
     assert float(((q - ref)[ok].norm(dim=1) / (a[ok].norm(dim=1) * omega.norm())).max()) < 1e-14
 
 
-@pytest.mark.parametrize("m,n", [(2048, 4096), (2176, 4001)])
-def test_omega_small_where_a_is_large(cuda, m, n):
+@pytest.mark.parametrize("m,n,k,p,N", [(2048, 4096, 64, 32, 16), (2176, 4001, 64, 32, 16), (4480, 4096, 16, 8, 8)])
+def test_omega_small_where_a_is_large(cuda, m, n, k, p, N):
     """Sums whose large factors do not meet: an Omega that is zero where A is large, a share of A's rows with few entries,
     and a power iteration on rows of two scales.  The error stays within what a running FP64 sum loses by
     elements, sqrt(K) 2^-53 |A| |B| (rounding errors of K terms, uncorrelated)."""
     import numpy as np
     from test_gpu_int8 import _sketch
-    k, p, N = 64, 32, 16
     g = torch.Generator(device=cuda)
     g.manual_seed(n)
     a = torch.randn(m, n, generator=g, dtype=torch.float64, device=cuda)
