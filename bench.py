@@ -230,6 +230,52 @@ def fp64_peak_tflops():
     return 2 * n ** 3 / best / 1e12
 
 
+def int8_peak_tops():
+    """cuBLAS int8 GEMM throughput on this GPU (the denominator of the products that run on
+    the int8 tensor cores).  Best of 5 at 8192^3, after warm-up; None where torch has none."""
+    import torch
+    n = 8192
+    try:
+        a = torch.randint(-128, 127, (n, n), dtype=torch.int8, device="cuda")
+        b = torch.randint(-128, 127, (n, n), dtype=torch.int8, device="cuda").t()
+        torch._int_mm(a, b)
+        torch.cuda.synchronize()
+        best = float("inf")
+        for _ in range(5):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            torch._int_mm(a, b)
+            e1.record()
+            e1.synchronize()
+            best = min(best, e0.elapsed_time(e1) / 1e3)
+        del a, b
+        return 2 * n ** 3 / best / 1e12
+    except (RuntimeError, AttributeError):
+        return None
+
+
+RNS_MODULI = 15
+
+
+def sketch_roofline(m, n, L, seconds, int8, peak64, peak_int8, traffic=None):
+    """The roofline record of the sketch Y = A Omega, from the path that ran: the DMMA GEMM
+    against the FP64 peak, or RNS_MODULI int8 products (their conversion, the magnitudes' and
+    the CRT in the time) against the int8 peak."""
+    achieved = 2.0 * m * n * L / seconds / 1e12
+    fp64 = {"achieved": round(achieved, 3), "peak": round(peak64, 3), "unit": "TFLOP/s",
+            "frac": round(achieved / peak64, 4), "peak_source": "cuBLAS DGEMM 8192^3 measured in this run"}
+    if not int8:
+        return dict({"bound": "tensor", "kernel": "dgemm_kernel (sketch Y = A Omega, FP64 DMMA)",
+                     "traffic": traffic, "algorithmic": "2*m*n*N*l flops per launch"}, **fp64)
+    tops = RNS_MODULI * achieved
+    return {"bound": "tensor",
+            "kernel": "rns_gemm_kernel with its residues and CRT (sketch Y = A Omega, FP64 by int8 residues)",
+            "achieved": round(tops, 1), "peak": round(peak_int8, 1) if peak_int8 else None, "unit": "TOP/s (int8)",
+            "frac": round(tops / peak_int8, 4) if peak_int8 else None, "traffic": traffic,
+            "peak_source": "cuBLAS int8 GEMM 8192^3 measured in this run",
+            "algorithmic": "%d x 2*m*n*N*l int8 operations" % RNS_MODULI, "as_fp64": fp64}
+
+
 def stage_rooflines(m, n, k, l, N, integrator, former, stages, peak_tflops, hbm_gbs):
     """Per-stage roofline of the FP64 solve: algorithmic flops and HBM bytes of each
     stage (the minimum any implementation must do), the stage's roofline time
@@ -510,7 +556,10 @@ def run_b200(args, world, rank, local):
     q = prm.createCollectionQ()
     sketch_t = []
     for _ in range(3):
+        before = isvd.context().kernels_launched()
         sk(a, q)
+        # Omega's, the DMMA GEMM's and its reduction: more are the int8 path's
+        sketch_int8 = isvd.context().kernels_launched() - before > 3
         sketch_t.append(sk.times()[1])      # "projection" part: the sketch GEMM alone
     sketch_s = sum(sketch_t) / len(sketch_t)
     orth = isvd.RowBlockGramianOrthogonalizer(prm)
@@ -547,8 +596,6 @@ def run_b200(args, world, rank, local):
             variants[name] = {"s": round(it_.time(), 5), "iterations": it_.iteration(),
                               "s_per_iteration": round(it_.time() / max(1, it_.iteration()), 7)}
     peak64 = fp64_peak_tflops()
-    flops = 2.0 * m * n * L
-    achieved = flops / sketch_s / 1e12
     traffic = None
     if SKETCH_TRAFFIC_PER_ROW is not None:
         traffic = SKETCH_TRAFFIC_PER_ROW * m
@@ -625,16 +672,7 @@ def run_b200(args, world, rank, local):
 
     stage_roof = stage_rooflines(m, n, k, l, N, args.integrator, args.former, stages, peak64,
                                  _measured_peak("hbm_gbs"))
-    # the sketch runs on the int8 tensor cores (15 residue products and the CRT): against the FP64 peak frac is the
-    # speed-up over the FP64 pipe, and int8_tops the rate of the pipe that does the work
-    roofline = {"bound": "tensor",
-                "kernel": "rns_gemm_kernel with its residues and CRT (sketch Y = A Omega, FP64 by int8 residues)",
-                "int8_tops": round(15 * achieved, 1),
-                "achieved": round(achieved, 3), "peak": round(peak64, 3), "unit": "TFLOP/s",
-                "frac": round(achieved / peak64, 4), "traffic": traffic,
-                "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 has no tcgen05 kind; the "
-                               "measured-peaks file holds bf16 and HBM only)",
-                "algorithmic": "2*m*n*N*l flops per launch"}
+    roofline = sketch_roofline(m, n, L, sketch_s, sketch_int8, peak64, int8_peak_tops() if sketch_int8 else None, traffic)
 
     # ---- end to end through the host-buffer C-ABI call (copies inside the timed region)
     e2e = None
