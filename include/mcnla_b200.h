@@ -25,7 +25,9 @@
  *     mcnla_b200_status_string() for the meanings.
  *   - Work is enqueued on the context's stream.  Functions that must read a
  *     device result to decide what to do next (the integrators' convergence
- *     tests) synchronize that stream; all others return without waiting.
+ *     tests) or to know their status (products on the tensor cores' int8 and
+ *     BF16 units, whose kernels wait with a limit) synchronize that stream; all
+ *     others return without waiting.
  */
 #ifndef MCNLA_B200_H_
 #define MCNLA_B200_H_

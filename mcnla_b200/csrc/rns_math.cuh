@@ -17,7 +17,7 @@ constexpr u128 product() {
   for (int i = 0; i < kNum; ++i) p *= unsigned(kMod[i]);
   return p;
 }
-constexpr u128 kP = product();   // 2^117.6
+constexpr u128 kP = product();   // 2^117.78
 static_assert(kP > (u128(1) << 117) && kP < (u128(1) << 118), "the scales below assume P between 2^117 and 2^118");
 // A row of A is scaled to a 2-norm of at most 2^kTA, a column of B to 2^kTB: |sum| < 2^(kTA + kTB)
 // (rounding to integers adds at most sqrt(K) / 2 < 2^8 to a norm), below P / 4 > 2^115

@@ -15,7 +15,7 @@
 // Measured against one kernel doing both with two barriers a round on a square (V in global memory for n > 112):
 // us a call, before and now: n = 12 (8 matrices) 93, 70; 20 (16) 182, 151; 32 (16) 335, 268; 64 (64) 1208, 878;
 // 80 (32) 2241, 1315; 96 (8) 3379, 1549; 128 (16) 8435, 3120; 160 (16) 16771, 5773.  At n = 160 the rotations'
-// kernel is at 80 % of the shared-memory pipe (every entry read and written once a round).
+// kernel is at 86 % of the shared-memory pipe (every entry read and written once a round).
 #include "kernels.cuh"
 #include "small.cuh"
 
