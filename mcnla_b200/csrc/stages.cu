@@ -1880,8 +1880,11 @@ int batched_solve(int device, mcnla_b200_problem* problems, int count, int worke
   // ---- waves within the budget (besides the workers' own workspaces and scratch)
   size_t worker_bytes = 0;
   for (auto& it : items) {
+    // the sketch, then the orthogonalizer, in the same workspace
+    const size_t sketch = problem_mixed(*it.p) ? 0 : plan_rns(ctx[0], it.d.m, it.d.L, it.d.n, RnsKind::Drawn).bytes;
     worker_bytes = std::max(worker_bytes, problem_scratch_bytes(*it.p) +
-                                              std::max(size_t(it.d.m) * it.d.L * 8, syev_work_bytes(it.d.l, it.d.N)) +
+                                              std::max({size_t(it.d.m) * it.d.L * 8, syev_work_bytes(it.d.l, it.d.N),
+                                                        sketch}) +
                                               gkn_ws_bytes(ctx[0], it.d) + gkn_bs_plan(ctx[0], it.d).bytes +
                                               (size_t(64) << 20));
   }
