@@ -280,7 +280,11 @@ int kn_loop(Context* c, int maxit, Body body, int* iters) {
     MB_CHECK(ctx_queue_scalars(c));
     if (capture) {
       auto ended = [&] { return *arrived >= 0 && *arrived < launched; };
-      while (*arrived < 0 && cudaStreamQuery(c->stream) == cudaErrorNotReady) {}
+      // (the stream is asked now and then, for a device that will not answer any more)
+      for (int polls = 1; *arrived < 0; ++polls) {
+        if (polls % 1024 == 0 && cudaStreamQuery(c->stream) != cudaErrorNotReady) break;
+        std::this_thread::yield();
+      }
       if (!ended() && capture_chunk(c, launched, chunk, body, ended, graph, &graph_kernels) != MCNLA_B200_OK)
         use_graph = false;
     }

@@ -168,3 +168,15 @@ def test_omega_small_where_a_is_large(cuda, m, n, k, p, N):
     ref = a @ (a.T @ (a @ omega))
     low = q[m // 2:]
     assert float((low - ref[m // 2:]).norm() / ref[m // 2:].norm()) < 1e-13
+
+
+def test_gramian_over_chunks(cuda):
+    """Bs = Qs' Qs with more rows than a chunk of K holds: the same Qbar as the row-block form, which makes no Gramian."""
+    m, l, N = 40001, 64, 16
+    g = torch.Generator(device=cuda)
+    g.manual_seed(21)
+    base = torch.linalg.qr(torch.randn(m, l, generator=g, dtype=torch.float64, device=cuda))[0]
+    q = _orth(base[None] + 0.3 / m ** 0.5 * torch.randn(N, m, l, generator=g, dtype=torch.float64, device=cuda))
+    a, ita = _integrate("RowBlockGramianKolmogorovNagumoIntegrator", q, l, N, 64, 1e-6)
+    b, itb = _integrate("RowBlockKolmogorovNagumoIntegrator", q, l, N, 64, 1e-6)
+    assert ita == itb and float((a - b).abs().max()) < 1e-12
